@@ -72,6 +72,12 @@ __global__ void k_gather(const int* __restrict__ idx, int n, const int* __restri
                        __int_as_float(Z[i]));
 }
 
+__global__ void k_zbin_starts(const int* __restrict__ off, long long off_stride, int nz, int* __restrict__ out) {
+  const int* o = off + blockIdx.y * off_stride;
+  const int z = blockIdx.x * blockDim.x + threadIdx.x;
+  if (z <= nz) out[(long long)blockIdx.y * (nz + 1) + z] = o[(long long)z * kBins2];
+}
+
 // ---- exclusive scan of int counts (nbins) into offsets (nbins + 1) ----
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
@@ -650,19 +656,22 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_conv(PotArgs a) {
 // ---------------------------------------------------------------------------
 // Separable conventional potential.  Each Gaussian of an element's expansion
 // v(r) ~= sum_j w_j exp(-alpha_j r^2) factorises over r^2 = rho^2 + dz_m^2, so
-// an atom's sub-plane sum at a pixel is
-//   sum_{m valid} wsub v(rho^2 + dz_m^2) ~= sum_j exp(-alpha_j rho^2) T_K[j],
+// an atom's sub-plane sum at a pixel is a function of rho^2 alone,
+//   G(rho^2) = sum_{m valid} wsub v(rho^2 + dz_m^2) ~= sum_j exp(-alpha_j rho^2) T_K[j],
 //   T_K[j] = wsub sum_{k < K} w_j exp(-alpha_j dz_(k)^2),
 // where the valid sub-planes (r^2 < 5 in the reference's FP32 rounding) are the
 // K with the smallest dz^2: for a fixed pixel the decision is monotone in dz^2.
-// k_atom_tables forms the T rows once per atom and slice; the pixel kernel
-// finds K with a five-step search over the atom's ascending thresholds (the
-// reference's own FP32 test, sub-plane by sub-plane) and takes kGaussJ
-// exponentials per (pixel, atom) instead of four per (pixel, atom, sub-plane).
-// Inside the 0.25 A clamp, where v is constant and the expansion does not
-// hold, the pixel sums vatom over its K sub-planes directly.
+// k_atom_tables expands G once per atom and slice into the piecewise
+// polynomials of ms_atoms.cuh; a pixel takes its bin from the bits of s, counts
+// the bin's thresholds passed (the reference's own FP32 test, sub-plane by
+// sub-plane) and evaluates five coefficients: about 35 instructions per
+// (pixel, atom) and no exponential, against about 95 (12 ex2 and a gathered
+// row of T_K among them) for the sum over the Gaussians at every pixel.
+// Inside the 0.25 A clamp v is constant: the clamped planes are the nearest
+// ones, and the others keep their Gaussians, summed directly (one pixel in a
+// hundred).
 // ---------------------------------------------------------------------------
-constexpr int kTabAtoms = 16;  // atoms per CTA of the table kernel, 16 threads each
+constexpr int kTabThreads = 128;  // threads per CTA of the table kernel
 
 // The cut-off test fadd(dxy, q) < 5 (round to nearest even) holds exactly when
 // the real sum dxy + q < 5 - 2^-22 (the midpoint below 5 rounds up to the even
@@ -673,100 +682,279 @@ __device__ __forceinline__ float cutoff_threshold(float q) {
   return __double2float_ru(4.999999761581421 - (double)q);
 }
 
-__global__ void __launch_bounds__(256) k_atom_tables(PotArgs a) {
-  __shared__ float s_d2[kTabAtoms][20];
-  __shared__ float s_qv[kTabAtoms][20];
-  __shared__ float s_e[kTabAtoms][20][kGaussJ];
-  __shared__ int s_n[kTabAtoms];
-  if (a.kt > a.kb || a.kt < 0 || a.kb >= a.nz) return;  // (no z-bin in the window)
-  // (this instance's index and tables; a itself stays in parameter space,
-  // where a.zsub is read)
+// Bin of s >= 0 (negative below 1/16), and the centre of s's bin.
+__device__ __forceinline__ int rad_bin(float s) { return (__float_as_int(s) >> 19) - kRadBin0; }
+__device__ __forceinline__ float rad_centre(float s) {
+  return __int_as_float((__float_as_int(s) & 0x7FF80000) | 0x00040000);
+}
+
+// exp(-alpha_j s) of every element's Gaussians at the bins' centres (FP64,
+// rounded once; once per parameterisation).
+__global__ void k_gauss_bins(const float* __restrict__ gauss, float* __restrict__ gbin) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kRadBins * kGaussJ) return;
+  const int b = i / kGaussJ, j = i - b * kGaussJ;
+  const float m = rad_centre(__int_as_float((b + kRadBin0) << 19));
+  gbin[(size_t)blockIdx.y * kRadBins * kGaussJ + i] =
+      (float)exp2(-(double)gauss[blockIdx.y * 2 * kGaussJ + j] * (double)m);
+}
+
+// The tables of the slices' atoms, LPA lanes of a warp per atom.  SEGS: with
+// the bins and segments (the forward; the position adjoint reads the rows T
+// only).  Bound: issue, about 730 warp instructions an atom at 16 lanes, half
+// of them the segments' moments (their exponentials come from gbin), and for
+// few atoms the chain of dependent steps: 32 lanes halve the loops over
+// planes, bins and segments at 1.4 times the instructions (see
+// launch_atom_tables).
+template <bool SEGS, int LPA>
+__global__ void __launch_bounds__(kTabThreads) k_atom_tables(const __grid_constant__ SepArgs q) {
+  constexpr int NA = kTabThreads / LPA;  // atoms per CTA and round
+  __shared__ float s_d2[NA][20];
+  __shared__ float s_qv[NA][20];
+  __shared__ float s_asc[NA][20];
+  __shared__ int s_tb[NA][20];
+  __shared__ __align__(16) float s_T[NA][20][kGaussJ];
+  __shared__ int s_range[SEGS ? NA : 1][2];
+  __shared__ unsigned short s_seg[SEGS ? NA : 1][SEGS ? kRadSegs : 1];
+  constexpr float kLn2 = 0.6931471805599453f;
+  // (the planes are read from parameter space)
+  const PotArgs& a = q.p;
+  const SlicePlanes& pl = q.pl[blockIdx.z];
+  if (pl.kt > pl.kb || pl.kt < 0 || pl.kb >= a.nz) return;  // (no z-bin in the window)
+  // this instance's index and tables
   const float4* atoms = a.atoms + blockIdx.y * a.b_atoms;
   const int* off = a.off + blockIdx.y * a.b_off;
-  float* tabs = a.tab + blockIdx.y * a.b_tab;
-  const int a0 = off[a.kt * kBins2], na = off[(a.kb + 1) * kBins2] - a0;
-  const int la = threadIdx.x >> 4, j = threadIdx.x & 15;
-  for (int base = blockIdx.x * kTabAtoms; base < na; base += gridDim.x * kTabAtoms) {
+  float* tabs = a.tab + blockIdx.y * a.b_tab + blockIdx.z * q.s_tab;
+  const int a0 = off[pl.kt * kBins2], na = off[(pl.kb + 1) * kBins2] - a0;
+  const int la = threadIdx.x / LPA, j = threadIdx.x % LPA;
+  for (int base = blockIdx.x * NA; base < na; base += gridDim.x * NA) {
     const bool valid = base + la < na;
     float* tab = tabs + (size_t)(base + la) * kTabStride;
     float4 at = make_float4(0.f, 0.f, 0.f, 0.f);
     if (valid) {
       at = atoms[a0 + base + la];
-      // dz_m^2 as the cut-off rounds it (16 lanes, two planes for the first 4)
-      for (int m = j; m < 20; m += 16) {
-        const float dz = fsub_x(a.zsub[m], at.z);
+      // dz_m^2 as the cut-off rounds it
+      for (int m = j; m < 20; m += LPA) {
+        const float dz = fsub_x(pl.zsub[m], at.z);
         s_d2[la][m] = fmul_x(dz, dz);
       }
     }
-    __syncthreads();
-    const float* g = a.gauss + (valid ? __float_as_int(at.w) - 1 : 0) * 2 * kGaussJ;
+    __syncwarp();
+    const int zi = valid ? __float_as_int(at.w) - 1 : 0;
+    const float* g = a.gauss + zi * 2 * kGaussJ;
+    int n = 0;
+    float dz0 = 1e30f;
     if (valid) {
       // each lane places its sub-planes by rank (ascending dz^2, ties by m);
       // the planes with dz^2 < 5 are the first n of that order
-      int cnt = 0;
-      for (int m = 0; m < 20; ++m) cnt += s_d2[la][m] < 5.0f;
-      if (j == 0) s_n[la] = cnt;
-      for (int m = j; m < 20; m += 16) {
+#pragma unroll 4
+      for (int m = 0; m < 20; ++m) {
+        n += s_d2[la][m] < 5.0f;
+        dz0 = fminf(dz0, s_d2[la][m]);
+      }
+      for (int m = j; m < 20; m += LPA) {
         const float d = s_d2[la][m];
         if (!(d < 5.0f)) continue;
         int r = 0;
+#pragma unroll 4
         for (int k = 0; k < 20; ++k) {
           const float e = s_d2[la][k];
           r += (e < d) || (e == d && k < m);
         }
-        const float dzv = fsub_x(a.zsub[m], at.z) + a.zsub_lo[m];
+        const float dzv = fsub_x(pl.zsub[m], at.z) + pl.zsub_lo[m];
         const float qv = dzv * dzv;
-        tab[kTabQ + r] = cutoff_threshold(d);
-        tab[kTabQV + r] = qv;
+        const float t = cutoff_threshold(d);
         s_qv[la][r] = qv;
+        tab[kTabQV + r] = qv;
+        // thresholds ascending; the bin each falls into (the same rounded sum
+        // as a pixel's s, which is monotone in rho^2), -1 below the bins
+        s_asc[la][n - 1 - r] = t;
+        tab[kTabAsc + n - 1 - r] = t;
+        const float st = fadd_x(t, dz0);
+        s_tb[la][n - 1 - r] = (t > 0.0f && st >= 0.0625f) ? rad_bin(st) : -1;
       }
-      for (int k = cnt + j; k < 32; k += 16) tab[kTabQ + k] = -1e30f;
+      for (int k = n + j; k < 24; k += LPA) tab[kTabAsc + k] = 1e30f;
     }
-    __syncthreads();
+    __syncwarp();
+    const int b0 = max(rad_bin(dz0), 0);
     if (valid) {
-      // w_j exp(-alpha_j dzv_k^2) for every (sub-plane, Gaussian), independent
-      const int nk = s_n[la];
-      for (int q = j; q < nk * kGaussJ; q += 16) {
-        const int k = q / kGaussJ, jj = q - k * kGaussJ;
-        s_e[la][k][jj] = g[kGaussJ + jj] * exp2f(-g[jj] * s_qv[la][k]);
+      if (j == 0)
+        *reinterpret_cast<float4*>(tab + kTabHead) =
+            make_float4(n > 0 ? dz0 : 1e30f, n > 0 ? s_qv[la][0] : 1e30f, __int_as_float(b0), __int_as_float(n));
+      // w_j exp(-alpha_j (dzv_k^2 - dzv_0^2)) for every (sub-plane, Gaussian)
+      for (int i = j; i < n * kGaussJ; i += LPA) {
+        const int k = i / kGaussJ, jj = i - k * kGaussJ;
+        s_T[la][k][jj] = g[kGaussJ + jj] * exp2f(-g[jj] * (s_qv[la][k] - s_qv[la][0]));
       }
     }
-    __syncthreads();
+    __syncwarp();
     if (valid && j < kGaussJ) {
       // running sums over the sub-planes in ascending dz^2 (FP64, rounded once)
-      const int nk = s_n[la];
       double sum = 0.0;
-      for (int k = 0; k < nk; ++k) {
-        sum += (double)s_e[la][k][j];
-        tab[kTabT + k * kGaussJ + j] = (float)((double)a.wsub * sum);
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) {
+        sum += (double)s_T[la][k][j];
+        const float t = (float)((double)a.wsub * sum);
+        s_T[la][k][j] = t;
+        tab[kTabT + k * kGaussJ + j] = t;
       }
     }
-    __syncthreads();
+    __syncwarp();
+    if constexpr (SEGS) {
+      // bins: the thresholds below each, the next ones, and which (bin,
+      // thresholds passed) each segment is
+      if (valid && n > 0) {
+        if (j < 2) {  // bins -1 and 100, and the zero segment
+          *reinterpret_cast<float4*>(tab + kTabBin + 4 * (j ? kRadBins + 1 : 0)) =
+              make_float4(1e30f, 1e30f, 1e30f, __int_as_float(kRadSegs + (j ? 0 : kRadMore)));
+          if (j) tab[kTabC4 + kRadSegs] = 0.0f;
+          else *reinterpret_cast<float4*>(tab + kTabSeg + 4 * kRadSegs) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (int b = b0 + j; b < kRadBins; b += LPA) {
+          int c = 0;  // thresholds below the bin (s_tb ascends)
+#pragma unroll
+          for (int st = 16; st >= 1; st >>= 1)
+            if (c + st <= n && s_tb[la][c + st - 1] < b) c += st;
+          int e = c;  // ... and through it
+          while (e < n && s_tb[la][e] <= b) ++e;
+          auto asc = [&](int k) { return k < n ? s_asc[la][k] : 1e30f; };
+          *reinterpret_cast<float4*>(tab + kTabBin + 4 * (b + 1)) =
+              make_float4(asc(c), asc(c + 1), asc(c + 2), __int_as_float(b - b0 + c + (e - c > 3 ? kRadMore : 0)));
+          // (segments below the first bin's and past the last bin's counts do not exist)
+          if (b == b0) s_range[la][0] = c;
+          if (b == kRadBins - 1) s_range[la][1] = b - b0 + min(e, n - 1) + 1;
+          for (; c <= min(e, n - 1); ++c) s_seg[la][b - b0 + c] = (unsigned short)(b | c << 8);
+        }
+      }
+      __syncwarp();
+      if (valid && n > 0) {
+        // (Gaussians in pairs on the packed FP32x2 pipe)
+        f2p al[kGaussJ / 2];
+#pragma unroll
+        for (int i = 0; i < kGaussJ / 2; ++i) al[i] = pk2(-kLn2 * g[2 * i], -kLn2 * g[2 * i + 1]);
+        const float* gb = a.gbin + (size_t)zi * kRadBins * kGaussJ;
+        // (unrolled: the next segments' gbin rows load while these are summed)
+#pragma unroll 2
+        for (int sg = s_range[la][0] + j; sg < s_range[la][1]; sg += LPA) {
+          const int bc = s_seg[la][sg], b = bc & 255, c = bc >> 8;
+          const ulonglong2* T = reinterpret_cast<const ulonglong2*>(s_T[la][n - 1 - c]);
+          const ulonglong2* E = reinterpret_cast<const ulonglong2*>(gb + b * kGaussJ);
+          // moments sum_j T_K[j] exp(-alpha_j s_c) (-alpha_j)^i, i = 0..5
+          f2p mp[6];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) mp[k] = 0ull;
+#pragma unroll
+          for (int i = 0; i < kGaussJ / 4; ++i) {
+            const ulonglong2 e = __ldg(E + i), t = T[i];
+            f2p xa = mul2(t.x, e.x), xb = mul2(t.y, e.y);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+              mp[k] = add2(mp[k], add2(xa, xb));
+              if (k < 4) {
+                xa = mul2(xa, al[2 * i]);
+                xb = mul2(xb, al[2 * i + 1]);
+              }
+            }
+            mp[5] = fma2(xa, al[2 * i], fma2(xb, al[2 * i + 1], mp[5]));
+          }
+          float mo[6];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) {
+            float lo, hi;
+            up2(mp[k], lo, hi);
+            mo[k] = lo + hi;
+          }
+          // half the bin's width: 2^e / 32; Taylor to degree five, the last
+          // term economised over the bin (tau^5 ~ 5/4 h^2 tau^3 - 5/16 h^4 tau)
+          const float h = __int_as_float(((b + kRadBin0) << 19) & 0x7F800000) * 0.03125f, h2 = h * h;
+          const float c5 = mo[5] * (1.0f / 120.0f);
+          *reinterpret_cast<float4*>(tab + kTabSeg + 4 * sg) =
+              make_float4(mo[0], fmaf(-0.3125f * h2 * h2, c5, mo[1]), 0.5f * mo[2],
+                          fmaf(1.25f * h2, c5, mo[3] * (1.0f / 6.0f)));
+          tab[kTabC4 + sg] = mo[4] * (1.0f / 24.0f);
+        }
+      }
+      __syncwarp();
+    }
   }
 }
 
+// A pixel inside the clamp region (s < 1/16): of the n planes, K pass the
+// cut-off and the nearest Kc of them are clamped, at v(0.25 A) each; the others
+// are sum_j exp(-alpha_j s) (T_K - T_Kc)[j].
+__device__ __noinline__ float clamp_value(const float* __restrict__ tab, const float* __restrict__ g,
+                                          const float* __restrict__ coef, float wsub, int n, float dxy, float dxyv,
+                                          float qv0) {
+  int c = 0;
+  while (c < n && dxy >= __ldg(tab + kTabAsc + c)) ++c;
+  const int K = n - c;
+  int Kc = 0;
+  while (Kc < K && dxyv + __ldg(tab + kTabQV + Kc) < 0.0625f) ++Kc;
+  float e = 0.0f;
+  if (K > Kc) {
+    for (int j = 0; j < kGaussJ; ++j) {
+      const float t = __ldg(tab + kTabT + (K - 1) * kGaussJ + j) -
+                      (Kc > 0 ? __ldg(tab + kTabT + (Kc - 1) * kGaussJ + j) : 0.0f);
+      e = fmaf(ex2_fast(-__ldg(g + j) * (dxyv + qv0)), t, e);
+    }
+  }
+  return Kc > 0 ? fmaf(wsub * (float)Kc, vatom_f(coef, 0.0f), e) : e;
+}
+
 // Each thread sums RY pixels of one column (rows y, y + 4, ...): a warp covers
-// an 8 x 4RY patch, and the per-atom work of a warp (staged atom, element,
-// table row base, loop) is shared by RY pixels per lane.  Each warp walks
-// only the staged atoms that can reach its own patch.
+// an 8 x 4RY patch, and the per-atom work of a warp (staged atom, table row,
+// loop) is shared by RY pixels per lane.  Each warp walks only the staged
+// atoms that can reach its own patch.
+//
+// Bound: issue and the ALU pipe (bin, segment and threshold arithmetic on
+// integers and predicates), with the gathers of bins and coefficients in L1.
+// Hence every lane takes the same straight path: bins below and above the
+// range map to a zero segment, positions of two pixels share packed FP32x2
+// instructions, and the rare rest (clamp region, bins with many thresholds) is
+// one branch per atom.  Per slice of the 50k-atom carbon slab (0.1 atoms/A^3,
+// 2 A slices) in a stack build, tables included: 1024^2 at 0.049 A 49 -> 28.6 us,
+// 4096^2 at 0.012 A 547 -> 276 us (against the sum over 12 Gaussians at every
+// pixel).  CTAs of four warps: eight warps waited longer at the staging
+// barriers (30.2 us); tables staged in shared memory cost occupancy and more
+// L2 traffic (34.8 us).
+constexpr int kSepChunk = 128;  // candidates staged at a time
+
+// Exact-position residual of fadd(off, fmul(i, ps)): off + i ps minus that
+// rounded value (error of the product by FMA, of the sum by two-sum).
+__device__ __forceinline__ float position_residual(float off, float i, float ps, float pos) {
+  const float p = fmul_x(i, ps), e = __fmaf_rn(i, ps, -p);
+  const float bb = fsub_x(pos, off);
+  return fadd_x(fadd_x(fsub_x(off, fsub_x(pos, bb)), fsub_x(p, bb)), e);
+}
+
+constexpr int kSepThreads = 128;
+constexpr int kSepSegs = 2 * kSepThreads;  // CSR segments at a time
+
+// CTAs per SM the registers are sized for.
+template <int RY>
+__host__ __device__ constexpr int sep_ctas() { return RY >= 8 ? 6 : RY >= 4 ? 8 : 10; }
+
 template <int TX, int TY, int RY>
-__global__ void __launch_bounds__(kPotThreads, RY >= 4 ? 5 : 6) k_potential_sep(PotArgs a) {
-  static_assert(TX * TY == kPotThreads * RY && TX % 8 == 0 && TY % (4 * RY) == 0, "tile of 8 x 4RY warp patches");
-  __shared__ float4 s_at[kConvChunk];
-  __shared__ __align__(16) float s_t[kConvChunk][32];
-  __shared__ __align__(16) float s_al[kConvChunk][kGaussJ];
-  __shared__ int s_l[kConvChunk];
-  __shared__ int s_wcnt[kPotThreads / 32];
-  __shared__ int s_start[kMaxSeg];
-  __shared__ int s_pref[kMaxSeg + 1];
+__global__ void __launch_bounds__(kSepThreads, sep_ctas<RY>()) k_potential_sep(const __grid_constant__ SepArgs q) {
+  static_assert(TX * TY == kSepThreads * RY && TX % 8 == 0 && TY % (4 * RY) == 0, "tile of 8 x 4RY warp patches");
+  static_assert(RY % 2 == 0 && kSepChunk == kSepThreads, "pixels in pairs, a thread per candidate");
+  __shared__ float4 s_at[kSepChunk];
+  __shared__ float4 s_h[kSepChunk];
+  __shared__ int s_l[kSepChunk];
+  __shared__ int s_wcnt[kSepChunk / 32];
+  __shared__ int s_start[kSepSegs];
+  __shared__ int s_pref[kSepSegs + 1];
   __shared__ int s_warp[33];
 
-  constexpr int PX = TX / 8;  // patches across
-  // (this instance's index, tables and output)
-  const float4* atoms = a.atoms + blockIdx.z * a.b_atoms;
-  const int* off = a.off + blockIdx.z * a.b_off;
-  const float* tabs = a.tab + blockIdx.z * a.b_tab;
-  float* V = a.V + blockIdx.z * a.b_V;
+  constexpr int PX = TX / 8, RP = RY / 2;  // patches across, pixel pairs per thread
+  // this slice's window, this instance's index, tables and output
+  const PotArgs& a = q.p;
+  const int sl = blockIdx.z / q.nb, inst = blockIdx.z - sl * q.nb;
+  const int kt = q.pl[sl].kt, kb = q.pl[sl].kb;
+  const float4* atoms = a.atoms + inst * a.b_atoms;
+  const int* off = a.off + inst * a.b_off;
+  const float* tabs = a.tab + inst * a.b_tab + sl * q.s_tab;
+  float* V = a.V + inst * a.b_V + sl * q.s_V;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
   const int wx0 = x0 + (w % PX) * 8, wy0 = y0 + (w / PX) * 4 * RY;  // this warp's patch
@@ -774,14 +962,16 @@ __global__ void __launch_bounds__(kPotThreads, RY >= 4 ? 5 : 6) k_potential_sep(
   const float px = fadd_x(a.xoff, fmul_x((float)x, a.ps));
   // values at the exact positions, decisions at the reference's FP32 ones (as
   // in k_potential_conv)
-  const float px_lo = (float)(((double)a.xoff + (double)x * (double)a.ps) - (double)px);
-  float py[RY], py_lo[RY], acc[RY];
+  const float px_lo = position_residual(a.xoff, (float)x, a.ps, px);
+  f2p py[RP], py_lo[RP];
+  float acc[RY];
 #pragma unroll
-  for (int r = 0; r < RY; ++r) {
-    const int y = wy0 + (lane >> 3) + 4 * r;
-    py[r] = fadd_x(a.yoff, fmul_x((float)y, a.ps));
-    py_lo[r] = (float)(((double)a.yoff + (double)y * (double)a.ps) - (double)py[r]);
-    acc[r] = 0.0f;
+  for (int h = 0; h < RP; ++h) {
+    const float ya = (float)(wy0 + (lane >> 3) + 8 * h), yb = ya + 4.0f;
+    const float pa = fadd_x(a.yoff, fmul_x(ya, a.ps)), pb = fadd_x(a.yoff, fmul_x(yb, a.ps));
+    py[h] = pk2(pa, pb);
+    py_lo[h] = pk2(position_residual(a.yoff, ya, a.ps, pa), position_residual(a.yoff, yb, a.ps, pb));
+    acc[2 * h] = acc[2 * h + 1] = 0.0f;
   }
   const float tx_lo = fadd_x(a.xoff, fmul_x((float)x0, a.ps));
   const float tx_hi = fadd_x(a.xoff, fmul_x((float)(x0 + TX - 1), a.ps));
@@ -790,20 +980,20 @@ __global__ void __launch_bounds__(kPotThreads, RY >= 4 ? 5 : 6) k_potential_sep(
   const float wx_lo = fadd_x(a.xoff, fmul_x((float)wx0, a.ps)), wx_hi = fadd_x(a.xoff, fmul_x((float)(wx0 + 7), a.ps));
   const float wy_lo = fadd_x(a.yoff, fmul_x((float)wy0, a.ps));
   const float wy_hi = fadd_x(a.yoff, fmul_x((float)(wy0 + 4 * RY - 1), a.ps));
-  const float xlo = a.xoff + x0 * a.ps - 2.2361f, xhi = a.xoff + (x0 + TX - 1) * a.ps + 2.2361f;
-  const float ylo = a.yoff + y0 * a.ps - 2.2361f, yhi = a.yoff + (y0 + TY - 1) * a.ps + 2.2361f;
-  const int bxl = max((int)floorf(xlo / a.bw_x) - 1, 0);
-  const int bxh = min((int)floorf(xhi / a.bw_x) + 1, kBins - 1);
-  const int byl = max((int)floorf(ylo / a.bw_y) - 1, 0);
-  const int byh = min((int)floorf(yhi / a.bw_y) + 1, kBins - 1);
+  // candidate bins of the tile (conservative: sqrt(5) plus one bin, which
+  // covers the approximate quotient)
+  const int bxl = max((int)floorf(__fdividef(tx_lo - 2.2361f, a.bw_x)) - 1, 0);
+  const int bxh = min((int)floorf(__fdividef(tx_hi + 2.2361f, a.bw_x)) + 1, kBins - 1);
+  const int byl = max((int)floorf(__fdividef(ty_lo - 2.2361f, a.bw_y)) - 1, 0);
+  const int byh = min((int)floorf(__fdividef(ty_hi + 2.2361f, a.bw_y)) + 1, kBins - 1);
   const int nyb = byh - byl + 1;
-  const bool window = a.kt <= a.kb && a.kt >= 0 && a.kb < a.nz;
-  const int a0 = window ? off[a.kt * kBins2] : 0;
+  const bool window = kt <= kb && kt >= 0 && kb < a.nz;
+  const int a0 = window ? off[kt * kBins2] : 0;
 
   if (bxl <= bxh && byl <= byh && window) {
-    const int kstep = max(kMaxSeg / nyb, 1);
-    for (int kg = a.kt; kg <= a.kb; kg += kstep) {
-      const int kend = min(kg + kstep - 1, a.kb);
+    const int kstep = max(kSepSegs / nyb, 1);
+    for (int kg = kt; kg <= kb; kg += kstep) {
+      const int kend = min(kg + kstep - 1, kb);
       const int nseg = (kend - kg + 1) * nyb;
       int len0 = 0, len1 = 0, st0 = 0, st1 = 0;
       // thread t holds the adjacent segments 2t and 2t + 1, so that the scan of
@@ -819,20 +1009,36 @@ __global__ void __launch_bounds__(kPotThreads, RY >= 4 ? 5 : 6) k_potential_sep(
         st1 = off[b + bxl];
         len1 = off[b + bxh + 1] - st1;
       }
-      int total;
-      const int ex = block_exclusive_scan(len0 + len1, s_warp, &total);
+      int total, ex;
+      if (nseg <= 64) {
+        // one warp holds them all
+        ex = 0;
+        if (w == 0) {
+          int incl = len0 + len1;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          ex = incl - len0 - len1;
+          if (lane == 31) s_pref[nseg] = incl;
+        }
+      } else {
+        ex = block_exclusive_scan(len0 + len1, s_warp, &total);
+        if (threadIdx.x == 0) s_pref[nseg] = total;
+      }
       if (s0 < nseg) { s_start[s0] = st0; s_pref[s0] = ex; }
       if (s1 < nseg) { s_start[s1] = st1; s_pref[s1] = ex + len0; }
-      if (threadIdx.x == 0) s_pref[nseg] = total;
       __syncthreads();
+      total = s_pref[nseg];
 
-      for (int base = 0; base < total; base += kConvChunk) {
-        const int nload = min(kConvChunk, total - base);
+      for (int base = 0; base < total; base += kSepChunk) {
+        const int nload = min(kSepChunk, total - base);
         // candidates kept when the nearest sub-plane can pass the cut-off
         // within sqrt(5) A of the tile's pixel rectangle (margin far above
         // FP32 rounding); kept atoms stay in CSR order
         bool keep = false;
-        float4 at = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 at = make_float4(0.f, 0.f, 0.f, 0.f), hd = at;
         int li = 0;
         if (threadIdx.x < nload) {
           const int gidx = base + threadIdx.x;
@@ -844,30 +1050,25 @@ __global__ void __launch_bounds__(kPotThreads, RY >= 4 ? 5 : 6) k_potential_sep(
           const int l = s_start[lo] + (gidx - s_pref[lo]);
           at = atoms[l];
           li = l - a0;
-          const float t0 = tabs[(size_t)li * kTabStride + kTabQ];
+          hd = __ldg(reinterpret_cast<const float4*>(tabs + (size_t)li * kTabStride + kTabHead));
           const float ddx = fmaxf(0.0f, fmaxf(tx_lo - at.x, at.x - tx_hi));
           const float ddy = fmaxf(0.0f, fmaxf(ty_lo - at.y, at.y - ty_hi));
-          keep = ddx * ddx + ddy * ddy < t0 + 0.0005f;
+          keep = ddx * ddx + ddy * ddy + hd.x < 5.0005f;
         }
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
         if (lane == 0) s_wcnt[w] = __popc(bal);
         __syncthreads();
         int pos = 0, cnt = 0;
-        for (int ww = 0; ww < kConvChunk / 32; ++ww) {
+#pragma unroll
+        for (int ww = 0; ww < kSepChunk / 32; ++ww) {
           if (ww < w) pos += s_wcnt[ww];
           cnt += s_wcnt[ww];
         }
         if (keep) {
           pos += __popc(bal & ((1u << lane) - 1u));
           s_at[pos] = at;
+          s_h[pos] = hd;
           s_l[pos] = li;
-        }
-        __syncthreads();
-        for (int q = threadIdx.x; q < cnt * 32; q += kPotThreads)
-          s_t[q >> 5][q & 31] = tabs[(size_t)s_l[q >> 5] * kTabStride + kTabQ + (q & 31)];
-        for (int q = threadIdx.x; q < cnt * kGaussJ; q += kPotThreads) {
-          const int i = q / kGaussJ, jj = q - i * kGaussJ;
-          s_al[i][jj] = -a.gauss[(__float_as_int(s_at[i].w) - 1) * 2 * kGaussJ + jj];
         }
         __syncthreads();
         // each warp walks the staged atoms that can reach its own patch
@@ -877,63 +1078,81 @@ __global__ void __launch_bounds__(kPotThreads, RY >= 4 ? 5 : 6) k_potential_sep(
             const float4 ar = s_at[c0 + lane];
             const float ddx = fmaxf(0.0f, fmaxf(wx_lo - ar.x, ar.x - wx_hi));
             const float ddy = fmaxf(0.0f, fmaxf(wy_lo - ar.y, ar.y - wy_hi));
-            reach = ddx * ddx + ddy * ddy < s_t[c0 + lane][0] + 0.0005f;
+            reach = ddx * ddx + ddy * ddy + s_h[c0 + lane].x < 5.0005f;
           }
           unsigned mask = __ballot_sync(0xffffffffu, reach);
           while (mask) {
             const int i = c0 + __ffs(mask) - 1;
             mask &= mask - 1u;
             const float4 at = s_at[i];
-            const float* t = s_t[i];
+            const float4 hd = s_h[i];
             const float* tab = tabs + (size_t)s_l[i] * kTabStride;
-            const float4* A = reinterpret_cast<const float4*>(&s_al[i][0]);
+            // (bins by the bits of s: the key of bin -1 folded into the base)
+            const float4* bins = reinterpret_cast<const float4*>(tab + kTabBin) - (kRadBin0 - 1);
             const float dx = fsub_x(px, at.x);
             const float dx2 = fmul_x(dx, dx);
             const float dxv = dx + px_lo;
+            const float xv = fmaf(dxv, dxv, hd.y);
+            const f2p dx2p = pk2(dx2, dx2), xvp = pk2(xv, xv), nay = pk2(-at.y, -at.y), h0 = pk2(hd.x, hd.x);
+            float dxy[RY], tau[RY];
+            int sg[RY], more = 0;
+#pragma unroll
+            for (int h = 0; h < RP; ++h) {
+              const f2p dy = add2(py[h], nay);
+              const f2p d2 = add2(dx2p, mul2(dy, dy));
+              const f2p s2 = add2(d2, h0);
+              const f2p dyv = add2(dy, py_lo[h]);
+              const f2p sv = fma2(dyv, dyv, xvp);
+              float s[2], v[2];
+              up2(d2, dxy[2 * h], dxy[2 * h + 1]);
+              up2(s2, s[0], s[1]);
+              up2(sv, v[0], v[1]);
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                const int r = 2 * h + k;
+                // bin -1 (clamp region) .. 100 (out of reach)
+                const float sc = fminf(fmaxf(s[k], 0.061f), 5.0f);
+                tau[r] = v[k] - rad_centre(sc);
+                const float4 e = __ldg(bins + (__float_as_int(sc) >> 19));
+                sg[r] = __float_as_int(e.w) + (dxy[r] >= e.x) + (dxy[r] >= e.y) + (dxy[r] >= e.z);
+                more |= sg[r];
+              }
+            }
+            if (more & kRadMore) {
+#pragma unroll
+              for (int r = 0; r < RY; ++r) {
+                if (!(sg[r] & kRadMore)) continue;
+                sg[r] -= kRadMore;
+                const float s = fadd_x(dxy[r], hd.x);
+                if (s < 0.0625f) {
+                  float pa, pb, la, lb;
+                  up2(py[r / 2], pa, pb);
+                  up2(py_lo[r / 2], la, lb);
+                  const float dyv = fsub_x(r % 2 ? pb : pa, at.y) + (r % 2 ? lb : la);
+                  const int zi = __float_as_int(at.w) - 1;
+                  acc[r] += clamp_value(tab, a.gauss + zi * 2 * kGaussJ, a.coef + zi * kCoefPerZ, a.wsub,
+                                        __float_as_int(hd.w), dxy[r], fmaf(dxv, dxv, dyv * dyv), hd.y);
+                } else {
+                  // more than three thresholds in the bin (the cut-off's rim)
+                  int c = sg[r] - (rad_bin(s) - __float_as_int(hd.z));
+                  while (dxy[r] >= __ldg(tab + kTabAsc + c)) ++c, ++sg[r];
+                }
+              }
+            }
 #pragma unroll
             for (int r = 0; r < RY; ++r) {
-              const float dy = fsub_x(py[r], at.y);
-              const float dxy = fadd_x(dx2, fmul_x(dy, dy));
-              // K = the sub-planes with r^2 = dxy + dz^2 < 5 (the reference's test)
-              int K = 0;
-#pragma unroll
-              for (int st = 16; st >= 1; st >>= 1)
-                if (dxy < t[K + st - 1]) K += st;
-              if (K == 0) continue;
-              const float dyv = dy + py_lo[r];
-              const float dxyv = fmaf(dxv, dxv, dyv * dyv);
-              if (dxy < t[0] - 4.9373f) {
-                // a sub-plane can reach the 0.25 A clamp (dxy + dz^2 < 0.0627;
-                // the clamp itself is decided on the exact r^2 inside vatom_f):
-                // the direct sum
-                const float* c = a.coef + (__float_as_int(at.w) - 1) * kCoefPerZ;
-                float v = 0.0f;
-                for (int k = 0; k < K; ++k) v += vatom_f(c, dxyv + __ldg(tab + kTabQV + k));
-                acc[r] += a.wsub * v;
-              } else {
-                // sum_j exp(-alpha_j rho^2) T_K[j]: per pair of Gaussians one
-                // packed multiply, two ex2, one packed fused multiply-add
-                const ulonglong2* T = reinterpret_cast<const ulonglong2*>(tab + kTabT + (K - 1) * kGaussJ);
-                const ulonglong2* A2 = reinterpret_cast<const ulonglong2*>(A);
-                const f2p rr = pk2(dxyv, dxyv);
-                f2p s2 = pk2(0.0f, 0.0f);
-#pragma unroll
-                for (int g = 0; g < kGaussJ / 4; ++g) {
-                  const ulonglong2 al = A2[g];
-                  const ulonglong2 tt = __ldg(T + g);
-                  s2 = fma2(ex2_pair(mul2(al.x, rr)), tt.x, s2);
-                  s2 = fma2(ex2_pair(mul2(al.y, rr)), tt.y, s2);
-                }
-                float e0, e1;
-                up2(s2, e0, e1);
-                acc[r] += e0 + e1;
-              }
+              const float4 c = __ldg(reinterpret_cast<const float4*>(tab + kTabSeg) + sg[r]);
+              float v = fmaf(__ldg(tab + kTabC4 + sg[r]), tau[r], c.w);
+              v = fmaf(v, tau[r], c.z);
+              v = fmaf(v, tau[r], c.y);
+              acc[r] += fmaf(v, tau[r], c.x);
             }
           }
         }
         // (no barrier here: the next round writes the staged arrays only after
         // its first barrier, which every warp reaches after this loop)
       }
+      if (kend < kb) __syncthreads();  // (the next group's segments overwrite these)
     }
   }
   if (x < a.nx) {
@@ -1059,13 +1278,16 @@ __device__ __forceinline__ float vatom_deriv_f(const float* __restrict__ c, floa
 //   dL/dX = 2 sum_p G(p) (px - X) sum_j alpha_j exp(-alpha_j rho^2) T_K[j],
 // likewise for Y (the cut-off decisions are not differentiated, as in the
 // per-sub-plane adjoint).  Pixels with a sub-plane inside the 0.25 A clamp
-// take the per-sub-plane derivative.  blockIdx.x: the atom of the window (its
+// take the per-sub-plane derivative.  (The forward's piecewise polynomials do
+// not serve here: their rounding, 1e-7, is the same over a whole ring of
+// pixels and the sum over the ring does not average it out: dL/dxy went from
+// 1.7e-6 to 8.7e-6 off FP64 with derivative segments.)  blockIdx.x: the atom of the window (its
 // table row), blockIdx.y: one of gridDim.y interleaved row sets of its
 // +-2.3 A pixel square; FP64 block sums, added atomically in input order.
 __global__ void __launch_bounds__(kPotThreads) k_potential_sep_adjoint(PotArgs a, const float* __restrict__ G,
                                                                        const int* __restrict__ perm, int a0,
                                                                        double* __restrict__ dxy) {
-  __shared__ float s_t[32];
+  __shared__ float s_asc[32];
   __shared__ float s_qv[20];
   __shared__ __align__(16) float s_al[kGaussJ];
   __shared__ double s_red[2][kPotThreads / 32];
@@ -1073,8 +1295,10 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_sep_adjoint(PotArgs a
   const int l = a0 + blockIdx.x;
   const float4 at = a.atoms[l];
   const float* tab = a.tab + (size_t)blockIdx.x * kTabStride;
-  const float* c = a.coef + (__float_as_int(at.w) - 1) * kCoefPerZ;
-  if (threadIdx.x < 32) s_t[threadIdx.x] = tab[kTabQ + threadIdx.x];
+  const float* cz = a.coef + (__float_as_int(at.w) - 1) * kCoefPerZ;
+  const float4 hd = __ldg(reinterpret_cast<const float4*>(tab + kTabHead));
+  const int n = __float_as_int(hd.w);
+  if (threadIdx.x < 32) s_asc[threadIdx.x] = threadIdx.x < 24 ? tab[kTabAsc + threadIdx.x] : 1e30f;
   if (threadIdx.x < 20) s_qv[threadIdx.x] = tab[kTabQV + threadIdx.x];
   if (threadIdx.x < kGaussJ) s_al[threadIdx.x] = a.gauss[(__float_as_int(at.w) - 1) * 2 * kGaussJ + threadIdx.x];
   __syncthreads();
@@ -1084,7 +1308,6 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_sep_adjoint(PotArgs a
   const int yh = min((int)ceilf((at.y + 2.3f - a.yoff) / a.ps), a.ny - 1);
   const int wx = xh - xl + 1, wy = yh - yl + 1;
   const int ns = gridDim.y, js = blockIdx.y;
-  const float t0 = s_t[0];
   float gx = 0.0f, gy = 0.0f;
   if (wx > 0 && wy > js) {
     const int npx = wx * ((wy - js + ns - 1) / ns);
@@ -1094,31 +1317,33 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_sep_adjoint(PotArgs a
       const float py = fadd_x(a.yoff, fmul_x((float)y, a.ps));
       const float dx = fsub_x(px, at.x), dy = fsub_x(py, at.y);
       const float dxy2 = fadd_x(fmul_x(dx, dx), fmul_x(dy, dy));
-      int K = 0;
+      int c = 0;  // thresholds passed: K = n - c planes remain
 #pragma unroll
       for (int st = 16; st >= 1; st >>= 1)
-        if (dxy2 < s_t[K + st - 1]) K += st;
-      if (K == 0) continue;
+        if (dxy2 >= s_asc[c + st - 1]) c += st;
+      const int K = n - c;
+      if (K <= 0) continue;
       const float dxv = dx + (float)(((double)a.xoff + (double)x * (double)a.ps) - (double)px);
       const float dyv = dy + (float)(((double)a.yoff + (double)y * (double)a.ps) - (double)py);
       const float dxyv = fmaf(dxv, dxv, dyv * dyv);
       const float gp = G[(long long)y * a.nx + x];
       float D;  // d/d(rho^2) of the atom's value at this pixel
-      if (dxy2 < t0 - 4.9373f) {
+      if (dxy2 + hd.x < 0.0627f) {
         D = 0.0f;
-        for (int k = 0; k < K; ++k) D += vatom_deriv_f(c, dxyv + s_qv[k]);
+        for (int k = 0; k < K; ++k) D += vatom_deriv_f(cz, dxyv + s_qv[k]);
         D *= a.wsub;
       } else {
         const float4* T = reinterpret_cast<const float4*>(tab + kTabT + (K - 1) * kGaussJ);
+        const float sv = dxyv + hd.y;  // (the rows T are relative to the nearest plane)
         float e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
         for (int g = 0; g < kGaussJ / 4; ++g) {
           const float4 al = *reinterpret_cast<const float4*>(&s_al[4 * g]);
           const float4 tt = __ldg(T + g);
-          e0 = fmaf(al.x * ex2_fast(-al.x * dxyv), tt.x, e0);
-          e1 = fmaf(al.y * ex2_fast(-al.y * dxyv), tt.y, e1);
-          e0 = fmaf(al.z * ex2_fast(-al.z * dxyv), tt.z, e0);
-          e1 = fmaf(al.w * ex2_fast(-al.w * dxyv), tt.w, e1);
+          e0 = fmaf(al.x * ex2_fast(-al.x * sv), tt.x, e0);
+          e1 = fmaf(al.y * ex2_fast(-al.y * sv), tt.y, e1);
+          e0 = fmaf(al.z * ex2_fast(-al.z * sv), tt.z, e0);
+          e1 = fmaf(al.w * ex2_fast(-al.w * sv), tt.w, e1);
         }
         D = -kLn2 * (e0 + e1);  // (s_al holds alpha_j log2(e))
       }
@@ -1159,13 +1384,22 @@ cudaError_t launch_potential_adjoint(const PotArgs& a, const float* G, const int
   const int na = a1 - a0;
   const int ns = std::min(16, std::max(1, (8 * 148 + na - 1) / na));
   if (separable) {
-    if (!a.tab || !a.gauss) return cudaErrorInvalidValue;
     // the slice's per-atom tables (a0 is the window's first atom, as there)
-    k_atom_tables<<<148 * 8, 256, 0, s>>>(a);
+    if (cudaError_t e = launch_atom_tables(sep_args(a, na), s, false)) return e;
     k_potential_sep_adjoint<<<dim3(na, ns), kPotThreads, 0, s>>>(a, G, perm, a0, dxy);
     return cudaGetLastError();
   }
   k_potential_conv_adjoint<<<dim3(na, ns), kPotThreads, 0, s>>>(a, G, perm, a0, dxy);
+  return cudaGetLastError();
+}
+
+cudaError_t zbin_starts(const int* off, long long off_stride, int nz, int nb, int* out, cudaStream_t s) {
+  k_zbin_starts<<<dim3((nz + 256) / 256, nb), 256, 0, s>>>(off, off_stride, nz, out);
+  return cudaGetLastError();
+}
+
+cudaError_t build_gauss_bins(const float* gauss, float* gbin, cudaStream_t s) {
+  k_gauss_bins<<<dim3((kRadBins * kGaussJ + 255) / 256, 103), 256, 0, s>>>(gauss, gbin);
   return cudaGetLastError();
 }
 
@@ -1196,45 +1430,59 @@ cudaError_t build_atom_index(const int* dZ, const float* dx, const float* dy, co
 int potential_tiles() { return 3; }
 int potential_tiles_separable() { return 4; }
 
-cudaError_t launch_atom_tables(const PotArgs& a, cudaStream_t s, int nbatch) {
-  if (!a.tab || !a.gauss || nbatch < 1 || nbatch > 65535) return cudaErrorInvalidValue;
-  // the window's atoms (read on the device) in 16-atom rounds
-  k_atom_tables<<<dim3(nbatch > 1 ? 296 : 148 * 8, nbatch), 256, 0, s>>>(a);
+template <bool SEGS, int LPA>
+static void run_atom_tables(const SepArgs& a, cudaStream_t s) {
+  constexpr int NA = kTabThreads / LPA;
+  const int ctas = (int)std::min<long long>(((long long)a.rows + NA - 1) / NA, 65535);
+  k_atom_tables<SEGS, LPA><<<dim3(ctas, a.nb, a.ns), kTabThreads, 0, s>>>(a);
+}
+
+// Lanes per atom: 32 while every atom's warp is resident at once (a launch of
+// few atoms is one pass through the chain of dependent steps), else 16.
+cudaError_t launch_atom_tables(const SepArgs& a, cudaStream_t s, bool segments) {
+  if (!a.p.tab || !a.p.gauss || !a.p.gbin || a.rows < 1 || a.nb < 1 || a.nb > 65535 || a.ns < 1 || a.ns > kSepGroup)
+    return cudaErrorInvalidValue;
+  const bool few = (long long)a.rows * a.nb * a.ns <= 148 * 16;
+  if (segments)
+    few ? run_atom_tables<true, 32>(a, s) : run_atom_tables<true, 16>(a, s);
+  else
+    few ? run_atom_tables<false, 32>(a, s) : run_atom_tables<false, 16>(a, s);
   return cudaGetLastError();
 }
 
-cudaError_t launch_potential_from_tables(const PotArgs& a, cudaStream_t s, int tile, int nbatch) {
-  if (!a.tab || !a.gauss || nbatch < 1 || nbatch > 65535) return cudaErrorInvalidValue;
-  // tiles of two or four pixels per thread: 16 x 32, 32 x 16, 16 x 64, 32 x 32
-  const int nb = nbatch;
+template <int TX, int TY, int RY>
+static cudaError_t run_potential_sep(const SepArgs& a, cudaStream_t s) {
+  k_potential_sep<TX, TY, RY>
+      <<<dim3((a.p.nx + TX - 1) / TX, (a.p.ny + TY - 1) / TY, a.nb * a.ns), kSepThreads, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+// Tile of a launch: four pixels per thread (a warp's per-atom work shared by
+// four rows), eight for pixels of at most 0.02 A (a patch of 0.16 x 0.32 A is
+// still small against the atoms' reach: 4096^2 at 0.012 A 276 us against 290;
+// at 0.049 A 30.6 against 28.5), two where four would leave SMs without a CTA
+// (64^2, two slices: 7.6 us a slice against 8.0).
+static int separable_tile(const SepArgs& a) {
+  const long long ctas = (long long)((a.p.nx + 31) / 32) * ((a.p.ny + 15) / 16) * a.nb * a.ns;
+  if (ctas < 148) return 0;
+  return a.p.ps <= 0.02f ? 3 : 2;
+}
+
+cudaError_t launch_potential_from_tables(const SepArgs& a, cudaStream_t s, int tile) {
+  const int nz = a.nb * a.ns;
+  if (!a.p.tab || !a.p.gauss || a.nb < 1 || a.ns < 1 || a.ns > kSepGroup || nz > 65535) return cudaErrorInvalidValue;
+  if (tile < 0) tile = separable_tile(a);
   switch (tile) {
-    case 0: k_potential_sep<16, 32, 2><<<dim3((a.nx + 15) / 16, (a.ny + 31) / 32, nb), kPotThreads, 0, s>>>(a); break;
-    case 1: k_potential_sep<32, 16, 2><<<dim3((a.nx + 31) / 32, (a.ny + 15) / 16, nb), kPotThreads, 0, s>>>(a); break;
-    case 2: k_potential_sep<16, 64, 4><<<dim3((a.nx + 15) / 16, (a.ny + 63) / 64, nb), kPotThreads, 0, s>>>(a); break;
-    case 3: k_potential_sep<32, 32, 4><<<dim3((a.nx + 31) / 32, (a.ny + 31) / 32, nb), kPotThreads, 0, s>>>(a); break;
+    case 0: return run_potential_sep<16, 16, 2>(a, s);
+    case 1: return run_potential_sep<16, 32, 4>(a, s);
+    case 2: return run_potential_sep<32, 16, 4>(a, s);
+    case 3: return run_potential_sep<32, 32, 8>(a, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
-cudaError_t launch_potential(const PotArgs& a, int kind, cudaStream_t s, int tile, bool separable, int nbatch) {
+cudaError_t launch_potential(const PotArgs& a, int kind, cudaStream_t s, int tile) {
   dim3 grid((a.nx + kTX - 1) / kTX, (a.ny + kTY - 1) / kTY);
-  if (kind == POT_CONVENTIONAL && separable) {
-    if (!a.tab || !a.gauss || nbatch < 1 || nbatch > 65535) return cudaErrorInvalidValue;
-    // the window's atoms (read on the device) in 16-atom rounds
-    k_atom_tables<<<dim3(nbatch > 1 ? 296 : 148 * 8, nbatch), 256, 0, s>>>(a);
-    // tiles of two or four pixels per thread: 16 x 32, 32 x 16, 16 x 64, 32 x 32
-    const int nb = nbatch;
-    switch (tile) {
-      case 0: k_potential_sep<16, 32, 2><<<dim3((a.nx + 15) / 16, (a.ny + 31) / 32, nb), kPotThreads, 0, s>>>(a); break;
-      case 1: k_potential_sep<32, 16, 2><<<dim3((a.nx + 31) / 32, (a.ny + 15) / 16, nb), kPotThreads, 0, s>>>(a); break;
-      case 2: k_potential_sep<16, 64, 4><<<dim3((a.nx + 15) / 16, (a.ny + 63) / 64, nb), kPotThreads, 0, s>>>(a); break;
-      case 3: k_potential_sep<32, 32, 4><<<dim3((a.nx + 31) / 32, (a.ny + 31) / 32, nb), kPotThreads, 0, s>>>(a); break;
-      default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-  }
-  if (nbatch != 1) return cudaErrorInvalidValue;
   if (kind == POT_CONVENTIONAL) {
     switch (tile) {
       case 0: k_potential_conv<32, 8><<<grid, kPotThreads, 0, s>>>(a); break;

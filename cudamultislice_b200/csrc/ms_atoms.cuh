@@ -28,6 +28,12 @@ struct BinScratch {
 };
 
 size_t bin_scratch_blocks(int nbins);
+// First sorted atom of every z-bin (and the atom count) of nb indices whose
+// offsets lie off_stride apart: out[k * (nz + 1) + z].
+cudaError_t zbin_starts(const int* off, long long off_stride, int nz, int nb, int* out, cudaStream_t s);
+// The Gaussians of every element at the radial bins' centres (PotArgs::gbin)
+// from the expansions (PotArgs::gauss).
+cudaError_t build_gauss_bins(const float* gauss, float* gbin, cudaStream_t s);
 cudaError_t build_atom_index(const int* dZ, const float* dx, const float* dy, const float* dz, int n,
                              const Box& box, int nz, AtomIndex& out, BinScratch& scr, cudaStream_t s);
 
@@ -61,6 +67,7 @@ struct PotArgs {
   // then w_j)
   float* tab;
   const float* gauss;
+  const float* gbin;     // exp(-alpha_j s) at the radial bins' centres [103][kRadBins][kGaussJ]
   // batched separable builds (one instance per blockIdx.z of the pixel kernel,
   // blockIdx.y of the table kernel): element strides of atoms, off, tab and V
   // between instances (0 for one instance)
@@ -70,26 +77,79 @@ struct PotArgs {
 // Gaussian expansion of vatom per element: v(r) ~= sum_j w_j exp(-alpha_j r^2)
 // for 0.25 A <= r <= 2.2365 A (positive weights).
 constexpr int kGaussJ = 12;
-// Per-atom table of one slice (floats): for the sub-planes that can pass the
-// cut-off, in ascending reference-rounded dz_m^2, the thresholds t_k with
-// "fadd(dxy, dz_k^2) < 5 exactly when dxy < t_k", padded with -1e30 to 32;
-// the exact-height dz_m^2 in the same order; then row k = 0..19:
-// wsub sum_{k' <= k} w_j exp(-alpha_j dzv_k'^2), j < kGaussJ.
-constexpr int kTabQ = 0, kTabQV = 32, kTabT = 56, kTabStride = 304;
+// The radial function of an atom in one slice, G(rho^2) = sum over the planes
+// that pass the cut-off of wsub v(rho^2 + dz_k^2), as polynomials in rho^2 for
+// the pixel kernels.  With s = fadd(rho^2, dz_0^2) (dz_0: the nearest plane;
+// s < 5 is the cut-off test of that plane), s >= 1/16 falls into bins of 1/16
+// octave (the float's exponent and top four mantissa bits), and inside a bin
+// the thresholds t_k ("plane k passes exactly when rho^2 < t_k") separate
+// segments of constant plane count.  Each segment holds a polynomial of degree
+// four in s - (bin centre).  Degree four over 1/16 octave: at most 5e-8 of G
+// off the Gaussian sum for every element (1.3e-7 of its derivative); eight bins
+// per octave or degree three would cost 2e-6.
+constexpr int kRadBin0 = 0x3D800000 >> 19;  // bin key of s = 1/16
+constexpr int kRadBins = 100;               // up to s = 5
+// Per-atom table (floats): header {dz_0^2 as the cut-off rounds it, at the
+// exact height, first bin (int), planes n (int)}; thresholds ascending, +inf
+// padded; exact-height dz_k^2 ascending; rows k = 0..19 of
+// wsub sum_{k' <= k} w_j exp(-alpha_j (dzv_k'^2 - dzv_0^2)); per bin -1 .. 100
+// the next three thresholds and the first segment (int, + kRadMore when the
+// pixel needs more than these: more than three thresholds, or bin -1, the
+// clamp region); per segment (bin - first bin + thresholds passed, below
+// kRadSegs; segment kRadSegs is zero, for bins -1 and 100, out of reach) c_4,
+// then c_0..c_3.
+constexpr int kRadSegs = 120, kRadMore = 1024;
+constexpr int kTabHead = 0, kTabAsc = 4, kTabQV = 28, kTabT = 48, kTabBin = 288,
+              kTabC4 = kTabBin + 4 * (kRadBins + 2), kTabSeg = kTabC4 + kRadSegs + 4,
+              kTabStride = kTabSeg + 4 * (kRadSegs + 4);
 
-// tile: the conventional kernel's tile shape variant (0: 32 x 8, 1: 16 x 16,
-// 2: 64 x 4 pixels; other kinds take 32 x 8).
-// separable: conventional kind only, through the per-atom tables (a.tab,
-// a.gauss set) instead of the per-sub-plane sum.
-cudaError_t launch_potential(const PotArgs& a, int kind, cudaStream_t s, int tile = 0, bool separable = false,
-                             int nbatch = 1);
+// The separable kernels' launch: up to kSepGroup consecutive slices and nb
+// instances at once (tables: blockIdx.y = instance, blockIdx.z = slice; pixels:
+// blockIdx.z = slice * nb + instance), the slices' planes and z-bin windows in
+// parameter space, s_tab and s_V the strides of the tables and the output
+// between slices.
+struct SlicePlanes {
+  float zsub[20], zsub_lo[20];
+  int kt, kb;
+};
+constexpr int kSepGroup = 16;
+struct SepArgs {
+  PotArgs p;
+  int ns, nb;
+  int rows;  // atoms of the fullest window (bounds the table launch)
+  long long s_tab, s_V;
+  SlicePlanes pl[kSepGroup];
+  void set_slice(int i, const PotArgs& a) {
+    for (int m = 0; m < 20; ++m) {
+      pl[i].zsub[m] = a.zsub[m];
+      pl[i].zsub_lo[m] = a.zsub_lo[m];
+    }
+    pl[i].kt = a.kt;
+    pl[i].kb = a.kb;
+  }
+};
+// One slice, one instance.
+inline SepArgs sep_args(const PotArgs& a, int rows) {
+  SepArgs s{};
+  s.p = a;
+  s.rows = rows;
+  s.ns = s.nb = 1;
+  s.set_slice(0, a);
+  return s;
+}
+
+
+// tile: the per-sub-plane conventional kernel's tile shape (0: 32 x 8, 1:
+// 16 x 16, 2: 64 x 4 pixels; other kinds take 32 x 8).
+cudaError_t launch_potential(const PotArgs& a, int kind, cudaStream_t s, int tile = 0);
 int potential_tiles();
 int potential_tiles_separable();
-// The separable conventional kernel's two launches apart (launch_potential
-// with separable = true enqueues both on one stream): the per-atom tables of
-// the slice into a.tab, then the potential from them.
-cudaError_t launch_atom_tables(const PotArgs& a, cudaStream_t s, int nbatch = 1);
-cudaError_t launch_potential_from_tables(const PotArgs& a, cudaStream_t s, int tile, int nbatch = 1);
+// The separable conventional kernel's two launches: the per-atom tables of the
+// slices into a.p.tab, then the potentials from them.  tile: 0..3 = 16 x 16,
+// 16 x 32, 32 x 16, 32 x 32 pixels (two, four, four and eight per thread), -1 =
+// by grid and pixel size.
+cudaError_t launch_atom_tables(const SepArgs& a, cudaStream_t s, bool segments = true);
+cudaError_t launch_potential_from_tables(const SepArgs& a, cudaStream_t s, int tile);
 
 // Adjoint of the conventional potential of one slice with respect to atom x, y:
 // dxy[2 perm[l] + {0,1}] += dL/d{x,y} of sorted atoms l in [a0, a1) (the CSR

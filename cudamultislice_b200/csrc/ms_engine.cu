@@ -342,7 +342,6 @@ class Engine {
     MS_TRY(d_yin_.resize(n));
     MS_TRY(d_zin_.resize(n));
     MS_TRY(d_atoms_.resize(n));
-    if (d_tab_.n < (size_t)n * kTabStride) MS_TRY(d_tab_.resize((size_t)n * kTabStride));
     MS_TRY(d_off_.resize(nbins + 1));
     MS_TRY(d_key_.resize(n));
     MS_TRY(d_idx_.resize(n));
@@ -356,11 +355,12 @@ class Engine {
     BinScratch scr{d_key_.p, d_idx_.p, d_cursor_.p, d_blocksum_.p};
     MS_TRY(build_atom_index(d_Zin_.p, d_xin_.p, d_yin_.p, d_zin_.p, n, box_, nz, idx, scr, stream_));
     launches += 8;
-    MS_TRY(cudaStreamSynchronize(stream_));
+    // the z-bins' first atoms on the host: atom ranges of the slices' windows
+    have_index_ = false;
+    if (int rc = fetch_zbin_starts(d_off_.p, 0, nz, 1, hzoff_)) return rc;
     natoms_ = n;
     nzb_ = nz;
     have_index_ = true;
-    hzoff_.clear();
     stack_valid_ = false;
     fd_stack_valid_ = false;
     return MS_OK;
@@ -416,8 +416,11 @@ class Engine {
         gauss[(r * 2 + 1) * kGaussJ + j] = (float)kGaussFit[r][1 + kGaussJ + j];
       }
     }
-    MS_TRY(d_gauss_.resize(gauss.size()));
+    // (the expansions, then their values at the radial bins' centres)
+    MS_TRY(d_gauss_.resize(gauss.size() + (size_t)103 * kRadBins * kGaussJ));
     MS_TRY(copy_sync(d_gauss_.p, gauss.data(), sizeof(float) * gauss.size(), cudaMemcpyHostToDevice));
+    MS_TRY(build_gauss_bins(d_gauss_.p, d_gauss_.p + gauss.size(), stream_));
+    ++launches;
     hfp_ = fp;
     hgauss_ = gauss;
     gauss_row_ok_.assign(103, -1);
@@ -1627,7 +1630,9 @@ class Engine {
                               d_tdsz_.p + (size_t)k * n, n, box_, nz, idx, scr, stream_));
       launches += 8;
     }
-    return separable_stack(S, d_fpstack_.p, N, nb, d_tds_atoms_.p, d_tds_off_.p, n, nbins + 1);
+    std::vector<int> zoff;
+    if (int rc = fetch_zbin_starts(d_tds_off_.p, nbins + 1, nz, nb, zoff)) return rc;
+    return separable_stack(S, d_fpstack_.p, N, nb, d_tds_atoms_.p, d_tds_off_.p, n, nbins + 1, nullptr, &zoff);
   }
 
   // ---- frozen-phonon series (the GUI's pass loop, MainWindow.xaml.cs:353-402) ----
@@ -1676,8 +1681,6 @@ class Engine {
     // (separable kernel); the handle's index is the last configuration's
     // afterwards, as one upload at a time leaves it
     const bool batch_pot = fused && kind == POT_CONVENTIONAL && separable_ok();
-    if (batch_pot && pot_tile_ < 0)
-      if (int rc = tune_pot_tile()) return rc;
     MS_TRY(cudaEventRecord(ev0_, stream_));
     for (int start = 0; start < nconf; start += B) {
       const int nb = std::min(B, nconf - start);
@@ -1782,7 +1785,7 @@ class Engine {
       const size_t N = (size_t)nx_ * ny_;
       MS_TRY(d_stack_.resize(N * S));
       const int kind = pot_mode_ == 1 ? POT_PROJECTED : POT_CONVENTIONAL;
-      if (kind == POT_CONVENTIONAL && pot_tile_ < 0 && !capturing_)
+      if (kind == POT_CONVENTIONAL && !separable_ok() && pot_tile_ < 0 && !capturing_)
         if (int rc = tune_pot_tile()) return rc;
       // device time of the stack (ms_get_last_device_ms)
       MS_TRY(cudaEventRecord(ev0_, stream_));
@@ -1815,8 +1818,6 @@ class Engine {
     if (int rc = require_potential_inputs()) return rc;
     if (int rc = ensure_prop_tables(convdz_)) return rc;
     plan_for(1);  // (tuning synchronises: before the streams fork)
-    if (pot_tile_ < 0)
-      if (int rc = tune_pot_tile()) return rc;
     const size_t N = (size_t)nx_ * ny_;
     MS_TRY(d_stack_.resize(N * S));
     MS_TRY(cudaEventRecord(ev0_, stream_));
@@ -2169,7 +2170,7 @@ class Engine {
       MS_TRY(d_dV_.resize(dLdV ? N * S : 2 * N));
       if (dLdxy) {
         MS_TRY(d_dxy_.resize(2 * (size_t)natoms_));
-        if (int rc = zbin_starts()) return rc;
+        if (int rc = ensure_tables(window_atoms(hzoff_, nzb_, 1))) return rc;
       }
     }
     invalidate_graph();  // the sweep below leaves d_psi_ at psi_S
@@ -2301,13 +2302,29 @@ class Engine {
     return MS_OK;
   }
 
-  // First sorted atom of every 1-A z-bin (CSR offsets at bin k * 2500), k = 0..nz.
-  int zbin_starts() {
-    if ((int)hzoff_.size() == nzb_ + 1) return MS_OK;
-    hzoff_.assign(nzb_ + 1, 0);
-    MS_TRY(cudaMemcpy2DAsync(hzoff_.data(), sizeof(int), d_off_.p, sizeof(int) * kBins2, sizeof(int), nzb_ + 1,
-                             cudaMemcpyDeviceToHost, stream_));
-    MS_TRY(cudaStreamSynchronize(stream_));
+  // First sorted atom of every 1-A z-bin (CSR offsets at bin k * 2500), k =
+  // 0..nz, of nb indices lying off_stride apart; waits for the stream.
+  int fetch_zbin_starts(const int* off, long long off_stride, int nz, int nb, std::vector<int>& out) {
+    const size_t n = (size_t)nb * (nz + 1);
+    MS_TRY(d_zstart_.resize(n));
+    MS_TRY(ms::zbin_starts(off, off_stride, nz, nb, d_zstart_.p, stream_));
+    ++launches;
+    out.resize(n);
+    MS_TRY(copy_sync(out.data(), d_zstart_.p, sizeof(int) * n, cudaMemcpyDeviceToHost));
+    return MS_OK;
+  }
+  // Atoms in the fullest z-bin window of a slice (pot_args: at most 2 lbz_ + 1
+  // bins) over nb indices: rows of one atom-table buffer.
+  size_t window_atoms(const std::vector<int>& zoff, int nz, int nb) const {
+    int most = 0;
+    for (int k = 0; k < nb; ++k) {
+      const int* z = zoff.data() + (size_t)k * (nz + 1);
+      for (int i = 0; i < nz; ++i) most = std::max(most, z[std::min(i + 2 * lbz_ + 1, nz)] - z[i]);
+    }
+    return (size_t)std::max(most, 1);
+  }
+  int ensure_tables(size_t rows) {
+    if (d_tab_.n < rows * kTabStride) MS_TRY(d_tab_.resize(rows * kTabStride));
     return MS_OK;
   }
 
@@ -2740,31 +2757,59 @@ class Engine {
 
   // Separable potentials of slices 1..S into out + (it - 1) * N (and, for a
   // batch of nb indices set up as in tds_potential_batch, instance k at
-  // out + k * S * N), npix table buffers deep: the tables of the next slices
-  // are built on the side stream while earlier slices' potentials run.  Slice
-  // it's potential runs on pixel stream it % npix (stream 0 is the handle's):
-  // consecutive slices are independent, and on several streams the last CTAs
-  // of one launch overlap the first of the next.  The tables' side stream has
-  // the higher priority, so the next slices' tables are not queued behind
-  // potential CTAs.  Event order: tables(it) after
-  // potential(it - npix), which read the same buffer; potential(it) after
-  // tables(it).  The side stream joins the handle's stream through the last
+  // out + k * S * N), in groups of consecutive slices: one table launch and
+  // one potential launch per group, each over the group's slices and
+  // instances.  Three table buffers: the tables of the next groups are built
+  // on the side stream while earlier groups' potentials run; group g's
+  // potentials run on pixel stream g % kPixStreams (stream 0 is the handle's),
+  // so that the last CTAs of one launch overlap the first of the next.  The
+  // tables' side stream has the higher priority, so the next group's tables
+  // are not queued behind potential CTAs.  Event order: tables(g) after
+  // potentials(g - 3), which read the same buffer; potentials(g) after
+  // tables(g).  The side stream joins the handle's stream through the last
   // potentials' dependence on their tables.
+  //
+  // Slices per group: a buffer of at most kTabBytes (three stay inside L2), at
+  // most kSepGroup, and at least six groups a stack (short stacks), so that
+  // slice passes that follow group by group start early.  A launch per slice
+  // left small grids to the launches and the table kernel's latency (256^2, 42
+  // slices: 14 us of tables per slice against 4 us in groups of seven).
+  static constexpr size_t kTabBytes = 24u << 20;
   int separable_stack(int S, float* out, size_t N, int nb, const float4* atoms = nullptr, const int* off = nullptr,
                       long long b_atoms = 0, long long b_off = 0,
-                      const std::function<int(int, cudaEvent_t)>& after_slice = nullptr, int npix = kPixStreams) {
-    npix = std::min(std::max(npix, 1), kPixStreams);
-    if (pot_tile_ < 0 && !capturing_)
-      if (int rc = tune_pot_tile()) return rc;
-    const int tile = std::min(std::max(pot_tile_, 0), potential_tiles_separable() - 1);
-    const size_t per = (size_t)nb * natoms_ * kTabStride;  // one buffer
-    if (d_tab_.n < npix * per) MS_TRY(d_tab_.resize(npix * per));
+                      const std::function<int(int, cudaEvent_t)>& after_slice = nullptr,
+                      const std::vector<int>* zoff = nullptr) {
+    const int tile = separable_tile_option();
+    const size_t rows = window_atoms(zoff ? *zoff : hzoff_, nzb_, nb);
+    const size_t per = (size_t)nb * rows * kTabStride;  // one slice's tables
+    const int gs = (int)std::max<size_t>(
+        1, std::min<size_t>({kTabBytes / (per * sizeof(float)), (size_t)kSepGroup, (size_t)(S + 5) / 6}));
+    const int groups = (S + gs - 1) / gs, npix = std::min(groups, kPixStreams);
+    if (int rc = ensure_tables(npix * gs * nb * rows)) return rc;
     MS_TRY(cudaEventRecord(ev_fork_, stream_));
     MS_TRY(cudaStreamWaitEvent(side_, ev_fork_, 0));
     for (int k = 1; k < npix; ++k) MS_TRY(cudaStreamWaitEvent(pix_[k], ev_fork_, 0));
     int rc = MS_OK;
-    for (int it = 1; it <= S && rc == MS_OK; ++it)
-      rc = separable_slice(it, out, N, nb, per, tile, atoms, off, b_atoms, b_off, S, after_slice, npix);
+    for (int g = 0; g < groups && rc == MS_OK; ++g) {
+      const int it0 = 1 + g * gs, ns = std::min(gs, S + 1 - it0), buf = g % npix;
+      SepArgs a = sep_args(pot_args(POT_CONVENTIONAL, it0, out + (size_t)(it0 - 1) * N), (int)rows);
+      for (int i = 1; i < ns; ++i) a.set_slice(i, pot_args(POT_CONVENTIONAL, it0 + i, nullptr));
+      a.ns = ns;
+      a.nb = nb;
+      a.s_tab = (long long)per;
+      a.s_V = (long long)N;
+      a.p.tab = d_tab_.p + (size_t)buf * gs * per;
+      if (atoms) {
+        a.p.atoms = atoms;
+        a.p.off = off;
+        a.p.b_atoms = b_atoms;
+        a.p.b_off = b_off;
+        a.p.b_tab = (long long)(rows * kTabStride);
+        a.p.b_V = (long long)S * N;
+      }
+      rc = separable_group(a, g, buf, npix, tile);
+      for (int i = 0; i < ns && rc == MS_OK && after_slice; ++i) rc = after_slice(it0 + i, ev_pix_[buf]);
+    }
     // join the other pixel streams (also on failure, so that the handle's
     // stream orders after everything enqueued)
     for (int k = 1; k < npix; ++k) {
@@ -2775,34 +2820,24 @@ class Engine {
     last_pot_sum_ = 2;
     return MS_OK;
   }
-  // One slice of separable_stack: its atom tables on the side stream (into
-  // table buffer it % npix, once the potential of slice it - npix, which read
-  // that buffer, is done), then its potential on pixel stream it % npix.
-  int separable_slice(int it, float* out, size_t N, int nb, size_t per, int tile, const float4* atoms,
-                      const int* off, long long b_atoms, long long b_off, int S,
-                      const std::function<int(int, cudaEvent_t)>& after_slice, int npix) {
-    const int buf = it % npix;
-    cudaStream_t ps = pix_[buf];
-    PotArgs a = pot_args(POT_CONVENTIONAL, it, out + (size_t)(it - 1) * N);
-    a.tab = d_tab_.p + buf * per;
-    if (atoms) {
-      a.atoms = atoms;
-      a.off = off;
-      a.b_atoms = b_atoms;
-      a.b_off = b_off;
-      a.b_tab = (long long)natoms_ * kTabStride;
-      a.b_V = (long long)S * N;
-    }
-    if (it > npix) MS_TRY(cudaStreamWaitEvent(side_, ev_pix_[buf], 0));
-    MS_TRY(launch_atom_tables(a, side_, nb));
+  // Group g of separable_stack: its tables on the side stream (into buffer
+  // buf, once the potentials of group g - npix, which read it, are done), then
+  // its potentials on pixel stream buf.
+  int separable_group(const SepArgs& a, int g, int buf, int npix, int tile) {
+    if (g >= npix) MS_TRY(cudaStreamWaitEvent(side_, ev_pix_[buf], 0));
+    MS_TRY(launch_atom_tables(a, side_));
     MS_TRY(cudaEventRecord(ev_tab_[buf], side_));
-    MS_TRY(cudaStreamWaitEvent(ps, ev_tab_[buf], 0));
-    MS_TRY(launch_potential_from_tables(a, ps, tile, nb));
-    MS_TRY(cudaEventRecord(ev_pix_[buf], ps));
+    MS_TRY(cudaStreamWaitEvent(pix_[buf], ev_tab_[buf], 0));
+    MS_TRY(launch_potential_from_tables(a, pix_[buf], tile));
+    MS_TRY(cudaEventRecord(ev_pix_[buf], pix_[buf]));
     launches += 2;
-    if (after_slice)
-      if (int rc = after_slice(it, ev_pix_[buf])) return rc;
     return MS_OK;
+  }
+  // One slice's tables and potential on the handle's stream.
+  cudaError_t launch_separable(const PotArgs& a, int tile) {
+    const SepArgs sa = sep_args(a, (int)window_atoms(hzoff_, nzb_, 1));
+    if (cudaError_t e = launch_atom_tables(sa, stream_)) return e;
+    return launch_potential_from_tables(sa, stream_, tile);
   }
 
   // Whether element row r's Gaussian expansion holds for the loaded table:
@@ -2845,18 +2880,27 @@ class Engine {
     const bool sep = kind == POT_CONVENTIONAL && separable_ok();
     if (kind == POT_CONVENTIONAL && pot_sum_ == 2 && !sep)
       return fail(MS_ERR_UNSUPPORTED, "an element of the specimen has no valid Gaussian expansion");
-    if (kind == POT_CONVENTIONAL && pot_tile_ < 0 && !capturing_)
+    if (kind == POT_CONVENTIONAL && !sep && pot_tile_ < 0 && !capturing_)
       if (int rc = tune_pot_tile()) return rc;
+    if (sep)
+      if (int rc = ensure_tables(window_atoms(hzoff_, nzb_, 1))) return rc;
     const PotArgs a = pot_args(kind, it, out);
-    const int ntile = sep ? potential_tiles_separable() : potential_tiles();
-    MS_TRY(launch_potential(a, kind, stream_, kind == POT_CONVENTIONAL ? std::min(std::max(pot_tile_, 0), ntile - 1) : 0,
-                            sep));
+    if (sep)
+      MS_TRY(launch_separable(a, separable_tile_option()));
+    else
+      MS_TRY(launch_potential(a, kind, stream_,
+                              kind == POT_CONVENTIONAL ? std::min(std::max(pot_tile_, 0), potential_tiles() - 1) : 0));
     launches += sep ? 2 : 1;
     last_pot_sum_ = kind == POT_CONVENTIONAL ? (sep ? 2 : 1) : last_pot_sum_;
     return MS_OK;
   }
 
-  // Tile shape of the conventional potential kernel for this grid, tuned on
+  // The separable kernel's tile: forced by MS_OPT_POTENTIAL_TILE, else -1 (by
+  // grid and pixel size, launch_potential_from_tables).
+  int separable_tile_option() const {
+    return pot_tile_forced_ ? std::min(pot_tile_, potential_tiles_separable() - 1) : -1;
+  }
+  // Tile shape of the per-sub-plane potential kernel for this grid, tuned on
   // the device the first time it is needed: each shape builds the mid-slab
   // slice (one warm-up launch, then three timed) and the fastest is kept.
   int tune_pot_tile() {
@@ -2867,17 +2911,16 @@ class Engine {
     MS_TRY(d_V_.resize(N));
     float best_t = INFINITY;
     int best = 0;
-    const bool sep = separable_ok();
-    for (int t = 0; t < (sep ? potential_tiles_separable() : potential_tiles()); ++t) {
+    for (int t = 0; t < potential_tiles(); ++t) {
       const PotArgs a = pot_args(POT_CONVENTIONAL, it, d_V_.p);
-      MS_TRY(launch_potential(a, POT_CONVENTIONAL, stream_, t, sep));
+      MS_TRY(launch_potential(a, POT_CONVENTIONAL, stream_, t));
       MS_TRY(cudaEventRecord(ev0_, stream_));
-      for (int k = 0; k < 3; ++k) MS_TRY(launch_potential(a, POT_CONVENTIONAL, stream_, t, sep));
+      for (int k = 0; k < 3; ++k) MS_TRY(launch_potential(a, POT_CONVENTIONAL, stream_, t));
       MS_TRY(cudaEventRecord(ev1_, stream_));
       MS_TRY(cudaEventSynchronize(ev1_));
       float ms = 0.0f;
       MS_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
-      launches += sep ? 8 : 4;
+      launches += 4;
       if (ms < best_t) {
         best_t = ms;
         best = t;
@@ -2894,6 +2937,7 @@ class Engine {
     a.coef = d_coef_.p;
     a.tab = d_tab_.p;
     a.gauss = d_gauss_.p;
+    a.gbin = d_gauss_.p + 103 * 2 * kGaussJ;
     a.V = out;
     a.nx = nx_;
     a.ny = ny_;
@@ -3032,6 +3076,7 @@ class Engine {
   // current slice, the loaded rows (FP64), per-row check (-1 not yet checked)
   static constexpr double kGaussTol = 2e-7;
   DevBuf<float> d_gauss_, d_tab_;
+  DevBuf<int> d_zstart_;
   DevBuf<float> d_tdsx_, d_tdsy_, d_tdsz_;  // displaced positions of a frozen-phonon batch
   DevBuf<float4> d_tds_atoms_;              // their atom indices [config][n], [config][nbins + 1]
   DevBuf<int> d_tds_off_;

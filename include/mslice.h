@@ -90,10 +90,11 @@ enum {
                                in 512-thread CTAs (units of 4, 2, 8 columns, tight poll);
                                8-9 as 3 and 2 with the ordering carried by the release
                                reduction and the acquire poll alone (no full fences) */
-  MS_OPT_POTENTIAL_TILE = 9, /* conventional potential kernel tile: -1 = tuned on the device
-                               per grid (default); per-sub-plane kernel 0, 1, 2 = 32 x 8,
-                               16 x 16, 64 x 4 pixels; separable kernel 0..3 = 16 x 32,
-                               32 x 16 (two pixels per thread), 16 x 64, 32 x 32 (four) */
+  MS_OPT_POTENTIAL_TILE = 9, /* conventional potential kernel tile: -1 = default (separable:
+                               by grid and pixel size; per sub-plane: tuned on the device
+                               per grid); per-sub-plane kernel 0, 1, 2 = 32 x 8, 16 x 16,
+                               64 x 4 pixels; separable kernel 0..3 = 16 x 16 (two pixels per
+                               thread), 16 x 32, 32 x 16 (four), 32 x 32 (eight) */
   MS_OPT_POTENTIAL_SUM = 10, /* how the conventional potential sums an atom's 20 sub-planes
                                (binnedAtomPKernel3, U.cu:582-653): 0 = separable where it
                                applies (default), else per sub-plane; 1 = per (pixel, atom,
@@ -101,8 +102,10 @@ enum {
                                MS_ERR_UNSUPPORTED.  Separable: each element's vatom as 12
                                Gaussians in r^2 (checked against the loaded parameterisation
                                to 2e-7 of v on 0.25..2.2365 A), so that an atom's sub-plane
-                               sum costs 12 exponentials per pixel; the same sub-planes pass
-                               the reference's FP32 cut-off test as term by term. */
+                               sum is a function of the distance in the plane alone,
+                               expanded once per atom and slice into piecewise polynomials
+                               (5e-8 of the sum); the same sub-planes pass the reference's
+                               FP32 cut-off test as term by term. */
   MS_OPT_BUILD_OVERLAP = 11 /* ms_run_conventional when the potential stack must be built:
                                1 = run each slice's fused passes on a second stream while the
                                next slices' potentials are built (default; separable
