@@ -682,7 +682,8 @@ class Engine {
     MS_TRY(d_fdX_.resize(N));
     MS_TRY(d_fdQ_.resize(N));
     MS_TRY(d_fdS_.resize(N));
-    if (!fd_state_) {
+    const bool start = !fd_state_;  // (the initial wave need not be band-limited)
+    if (start) {
       if (int rc = ensure_real()) return rc;
       // spectrum FFT2(psi_n) = FFT_col(FFT_row(psi_n)) stored column-major,
       // X = FFT_row(psi_n) / nx (so that IFFT_row(X) = psi_n)
@@ -710,7 +711,7 @@ class Engine {
     a.fd_rc = make_float2((float)rcx, (float)rcy);
     a.fd_ratio = make_float2((float)((1.0 - aa * aa) / den), (float)(-2.0 * aa / den));
     a.fd_kv = (float)(dz * dz * 4.0 * 3.14159 * (double)sigma2_ / lam);
-    MS_TRY(pass_a(a, A_INV | A_FD | A_FWD, 1));
+    MS_TRY(pass_a(a, start ? (A_INV | A_FD | A_FWD | A_BO) : (A_INV | A_FD | A_FWD | A_BI | A_BO), 1));
     PassBArgs b = passb_args(d_fdQ_.p, d_fdX_.p, 0);
     b.spec = d_fdS_.p;
     const double cf = dz * dz * 4.0 * 3.14159 * 3.14159;
@@ -732,13 +733,13 @@ class Engine {
     const long long N = (long long)nx_ * ny_;
     if (int rc = potential_slice(POT_FD, it, d_f_.p)) return rc;
     MS_TRY(pw_real_to_complex(d_f_.p, d_t1_.p, g, stream_, &launches));
-    MS_TRY(pass_a(passa_args(d_t1_.p, d_t1_.p, 0), A_FWD, 1));
+    MS_TRY(pass_a(passa_args(d_t1_.p, d_t1_.p, 0), A_FWD | A_BO, 1));
     PassBArgs bl = passb_args(d_t1_.p, d_t1_.p, 0);
     bl.scale = 1.0f / (float)N;
     MS_TRY(pass_b(bl, B_BANDLIMIT, 1));
     PassAArgs vr = passa_args(d_t1_.p, nullptr, 0);
     vr.out_f = out;
-    MS_TRY(pass_a(vr, A_INV | A_REAL, 1));
+    MS_TRY(pass_a(vr, A_INV | A_REAL | A_BI, 1));
     launches += 3;
     return MS_OK;
   }
@@ -974,6 +975,7 @@ class Engine {
     if (use_fused() && domain_ == 1) {
       PassBArgs b = passb_args(d_psi_.p, d_psi_.p, 0);
       b.acc = d_tds_.p;
+      b.band = 1;
       b.scale = (float)nx_;  // FFT_rows(psi) = nx * X for the row-frequency state X
       MS_TRY(pass_b(b, B_CBED, 1));
       ++launches;
@@ -1063,6 +1065,7 @@ class Engine {
         scale = (float)nx_ / (float)N;  // FFT_rows(psi) = nx * X
       }
       b = passb_args(src, d_t2_.p, 0);
+      b.band = domain_ == 1;
       b.ctf = CtfParams{(double)wavel, (double)Cs_, (double)df_, (double)A2_, (double)phi2_, 0.0, 0.0, beta,
                         (double)delta_, objap2};
       b.scale = scale;
@@ -1070,7 +1073,7 @@ class Engine {
       PassAArgs a = passa_args(d_t2_.p, nullptr, 0);
       a.out_f = d_f_.p;
       a.scale = 1.0f;
-      MS_TRY(pass_a(a, A_INV | A_INTENSITY, 1));
+      MS_TRY(pass_a(a, A_INV | A_INTENSITY | (b.band ? A_BI : 0), 1));
       launches += 2;
     } else {
       if (int rc = ensure_real()) return rc;
@@ -1155,13 +1158,14 @@ class Engine {
       }
       for (int i = 0; i < n; ++i) {
         PassBArgs b = passb_args(src, d_t2_.p, 0);
+        b.band = domain_ == 1;
         b.ctf = CtfParams{(double)wavel, cs ? (double)cs[i] : (double)Cs_, (double)df[i], (double)A2_, (double)phi2_,
                           0.0, 0.0, beta, (double)delta_, objap2};
         b.scale = scale;
         MS_TRY(pass_b(b, B_CTF, 1));
         PassAArgs a = passa_args(d_t2_.p, nullptr, 0);
         a.out_f = d_img_.p + (size_t)i * N;
-        MS_TRY(pass_a(a, A_INV | A_INTENSITY, 1));
+        MS_TRY(pass_a(a, A_INV | A_INTENSITY | (b.band ? A_BI : 0), 1));
         launches += 2;
       }
     } else {
@@ -1551,13 +1555,15 @@ class Engine {
         a.batch_stride_wave = N;
         a.batch_stride_V = 0;
         a.tr = d_tstack_.p + (size_t)(it - 1) * N;
-        MS_TRY(launch_pass_a(a, vr, it == 1 ? (A_MULT_TC | A_FWD) : (A_INV | A_MULT_TC | A_FWD), nb, st));
+        MS_TRY(launch_pass_a(a, vr, it == 1 ? (A_MULT_TC | A_FWD | A_BO) : (A_INV | A_MULT_TC | A_FWD | A_BI | A_BO), nb,
+                             st));
         PassBArgs b = passb_args(d_bwave_.p, d_bwave_.p, vc);
         b.batch_stride_wave = N;
         if (it < S) {
           MS_TRY(launch_pass_b(b, vc, B_PROPAGATE, nb, st));
         } else {
           b.sig = d_bsig_.p + start;
+          b.band = 1;
           b.kin2 = rs_kin2_;
           b.kout2 = rs_kout2_;
           b.scale = 1.0f / (float)N;
@@ -1733,7 +1739,7 @@ class Engine {
           a.batch_stride_wave = N;
           a.batch_stride_V = (long long)S * N;
           a.V = d_fpstack_.p + (size_t)(it - 1) * N;
-          MS_TRY(pass_a(a, it == 1 ? (A_MULT_T | A_FWD) : (A_INV | A_MULT_T | A_FWD), nb));
+          MS_TRY(pass_a(a, it == 1 ? (A_MULT_T | A_FWD | A_BO) : (A_INV | A_MULT_T | A_FWD | A_BI | A_BO), nb));
           PassBArgs b = passb_args(d_bwave_.p, d_bwave_.p, 0);
           b.batch_stride_wave = N;
           MS_TRY(pass_b(b, B_PROPAGATE, nb));
@@ -1744,6 +1750,7 @@ class Engine {
         PassBArgs b = passb_args(d_bwave_.p, d_bwave_.p, 0);
         b.batch_stride_wave = N;
         b.acc = d_fpdiff_.p;
+        b.band = 1;
         b.scale = (float)nx_;  // FFT2(psi) = nx FFT_col(X)
         MS_TRY(pass_b(b, B_CBED, nb));
         ++launches;
@@ -1752,12 +1759,13 @@ class Engine {
         PassBArgs b = passb_args(d_bwave_.p, d_bwave_.p, 0);
         b.batch_stride_wave = N;
         b.ctf = ctf;
+        b.band = 1;
         b.scale = (float)nx_ / (float)N;
         MS_TRY(pass_b(b, B_CTF, nb));
         PassAArgs a = passa_args(d_bwave_.p, nullptr, 0);
         a.batch_stride_wave = N;
         a.out_f = d_fpimg_.p;
-        MS_TRY(pass_a(a, A_INV | A_INTENSITY, nb));
+        MS_TRY(pass_a(a, A_INV | A_INTENSITY | A_BI, nb));
         MS_TRY(pw_add_batch(d_fpimg_.p, N, nb, d_fpsum_.p, 1.0f / (float)nconf, g, stream_, &launches));
         launches += 2;
       }
@@ -2070,7 +2078,8 @@ class Engine {
         for (int k = 0; k < steps && rc == MS_OK; ++k) {
           PassAArgs a = passa_args(k == 0 ? d_psi0_.p : d_psi_.p, d_psi_.p, 0);
           a.V = d_stack_.p + (size_t)(k % S) * N;
-          cudaError_t e1 = pass_a(a, k == 0 ? (A_MULT_T | A_FWD) : (A_INV | A_MULT_T | A_FWD), 1);
+          cudaError_t e1 =
+              pass_a(a, k == 0 ? (A_MULT_T | A_FWD | A_BO) : (A_INV | A_MULT_T | A_FWD | A_BI | A_BO), 1);
           cudaEventRecord(ev[2 * k + 1], stream_);
           cudaError_t e2 = pass_b(passb_args(d_psi_.p, d_psi_.p, 0), B_PROPAGATE, 1);
           cudaEventRecord(ev[2 * k + 2], stream_);
@@ -2184,6 +2193,8 @@ class Engine {
     // timed from here: the potential stack (when the atoms changed), the sweeps
     MS_TRY(cudaEventRecord(ev0_, stream_));
     if (int rc = build_stack(&Sall)) return rc;
+    constexpr int kSaveFirst = A_SAVE | A_MULT_T | A_FWD | A_BO;
+    constexpr int kSaveNext = A_INV | A_SAVE | A_MULT_T | A_FWD | A_BI | A_BO;
     // forward sweep; checkpoint c (c = 1..nck-1) holds X_{cK}; the waves of
     // the last segment (psi_{clast} .. psi_{S-1}) are kept as they pass
     const int clast = ((S - 1) / K) * K;
@@ -2195,7 +2206,7 @@ class Engine {
         PassAArgs a = passa_args(n == 1 ? d_psi0_.p : d_psi_.p, d_psi_.p, 0);
         a.V = d_stack_.p + (size_t)(n - 1) * N;
         a.out2 = d_seg_.p + (size_t)(n - 1 - clast) * N;
-        MS_TRY(pass_a(a, n == 1 ? (A_SAVE | A_MULT_T | A_FWD) : (A_INV | A_SAVE | A_MULT_T | A_FWD), 1));
+        MS_TRY(pass_a(a, n == 1 ? kSaveFirst : kSaveNext, 1));
         MS_TRY(pass_b(passb_args(d_psi_.p, d_psi_.p, 0), B_PROPAGATE, 1));
         domain_ = 1;
       } else if (int rc = enqueue_fused_step(d_stack_.p + (size_t)(n - 1) * N, n == 1)) {
@@ -2208,6 +2219,7 @@ class Engine {
     const float objap2 = (((objap * 0.001f) / wavel) * ((objap * 0.001f) / wavel));
     for (int d = 0; d < nd; ++d) {
       PassBArgs b = passb_args(d_psi_.p, d_Phi_.p, 0);
+      b.band = 1;
       b.ctf = CtfParams{(double)wavel, (double)Cs_, (double)defoci[d], (double)A2_, (double)phi2_, 0.0, 0.0,
                         (double)(beta_ / 1000), (double)delta_, objap2};
       b.scale = (float)nx_ / (float)N;  // FFT_rows(psi) = nx X
@@ -2216,7 +2228,7 @@ class Engine {
       a.T = d_T_.p + (size_t)d * N;
       a.loss = d_loss_.p;
       a.out_f = images ? d_img_.p + (size_t)d * N : nullptr;
-      MS_TRY(pass_a(a, grad ? (A_INV | A_RESID | A_FWD) : (A_INV | A_RESID), 1));
+      MS_TRY(pass_a(a, grad ? (A_INV | A_RESID | A_FWD | A_BI | A_BO) : (A_INV | A_RESID | A_BI), 1));
       launches += 2;
       if (grad) {
         b.in = d_U_.p;
@@ -2239,7 +2251,7 @@ class Engine {
           a.V = d_stack_.p + (size_t)(n - 1) * N;
           a.out2 = d_seg_.p + (size_t)(n - 1 - c) * N;
           const bool real_in = (n == 1);
-          MS_TRY(pass_a(a, real_in ? (A_SAVE | A_MULT_T | A_FWD) : (A_INV | A_SAVE | A_MULT_T | A_FWD), 1));
+          MS_TRY(pass_a(a, real_in ? kSaveFirst : kSaveNext, 1));
           MS_TRY(pass_b(passb_args(d_t1_.p, d_t1_.p, 0), B_PROPAGATE, 1));
           launches += 2;
           cur = d_t1_.p;
@@ -2250,7 +2262,7 @@ class Engine {
         } else if (e - 1 == 0) {
           MS_TRY(cudaMemcpyAsync(last, d_psi0_.p, sizeof(float2) * N, cudaMemcpyDeviceToDevice, stream_));
         } else {
-          MS_TRY(pass_a(passa_args(cur, last, 0), A_INV, 1));
+          MS_TRY(pass_a(passa_args(cur, last, 0), A_INV | A_BI, 1));
           ++launches;
         }
         // adjoint steps e .. c+1
@@ -2267,7 +2279,7 @@ class Engine {
           if (!dLdV && dLdxy) MS_TRY(cudaStreamWaitEvent(stream_, ev_adj_[n & 1], 0));
           a.out_f = dV;
           a.scale = 1.0f / (float)nx_;
-          MS_TRY(pass_a(a, A_INV | A_ADJ | A_FWD, 1));
+          MS_TRY(pass_a(a, A_INV | A_ADJ | A_FWD | A_BI | A_BO, 1));
           launches += 2;
           if (dLdxy) {
             const PotArgs pa = pot_args(POT_CONVENTIONAL, n, nullptr);
@@ -2361,6 +2373,8 @@ class Engine {
     PassBArgs b = passb_args(w.p, w.p, variant);
     b.batch_stride_wave = N;
     b.ctf = CtfParams{(double)wavel_, (double)Cs_, (double)df_, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 1e30f};
+    // (the passes that multiply are timed as the slice loop runs them, on the band)
+    if (pass == 0 && (op & (A_MULT_T | A_MULT_TC)) != 0) op |= ((op & A_INV) ? A_BI : 0) | ((op & A_FWD) ? A_BO : 0);
     auto launch = [&]() {
       return pass == 0 ? launch_pass_a(a, variant, op, batch, stream_) : launch_pass_b(b, variant, op, batch, stream_);
     };
@@ -2582,7 +2596,7 @@ class Engine {
     cudaMemsetAsync(w.p, 0, sizeof(float2) * batch * N, stream_);
     cudaMemsetAsync(V.p, 0, sizeof(float) * N, stream_);
     if (tc) cudaMemsetAsync(T.p, 0, sizeof(float2) * N, stream_);
-    const int row_op = tc ? (A_INV | A_MULT_TC | A_FWD) : (A_INV | A_MULT_T | A_FWD);
+    const int row_op = (tc ? (A_INV | A_MULT_TC | A_FWD) : (A_INV | A_MULT_T | A_FWD)) | A_BI | A_BO;
     if (ensure_prop_tables(convdz_) != MS_OK) return best;
     const int reps = 8, nv = plan_variants();
     auto row_args = [&](int v) {
@@ -2707,7 +2721,7 @@ class Engine {
     // the current wave in whichever domain it is held
     PassAArgs a = passa_args(first ? d_psi0_.p : d_psi_.p, d_psi_.p, 0);
     a.V = V;
-    const int fl = (first || domain_ == 0) ? (A_MULT_T | A_FWD) : (A_INV | A_MULT_T | A_FWD);
+    const int fl = (first || domain_ == 0) ? (A_MULT_T | A_FWD | A_BO) : (A_INV | A_MULT_T | A_FWD | A_BI | A_BO);
     MS_TRY(pass_a(a, fl, 1, s));
     MS_TRY(pass_b(passb_args(d_psi_.p, d_psi_.p, 0), B_PROPAGATE, 1, s));
     domain_ = 1;
@@ -2743,13 +2757,13 @@ class Engine {
     if (domain_ == 0) return MS_OK;
     if (domain_ == 2) {
       // fused finite differences: psi_n = IFFT_row(X), the FD state stays valid
-      MS_TRY(pass_a(passa_args(d_fdX_.p, d_psi_.p, 0), A_INV, 1));
+      MS_TRY(pass_a(passa_args(d_fdX_.p, d_psi_.p, 0), A_INV | A_BI, 1));
       ++launches;
       domain_ = 0;
       return MS_OK;
     }
     PassAArgs a = passa_args(d_psi_.p, d_psi_.p, 0);
-    MS_TRY(pass_a(a, A_INV, 1));
+    MS_TRY(pass_a(a, A_INV | A_BI, 1));
     ++launches;
     domain_ = 0;
     return MS_OK;

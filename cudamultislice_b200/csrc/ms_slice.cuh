@@ -8,6 +8,16 @@
 // Between steps the wave stays in the "row-frequency" domain; a final pass A
 // with only IFFT_row returns it to real space.  Each pass reads and writes the
 // wave once (8 MB at 1024^2: L2-resident on B200) and pass A streams V.
+//
+// The band.  kmax is at most half the smaller Nyquist frequency
+// ((n/2 - 1) / (2 n ps), U.cu:1913-1925), so the propagator (k < kmax) and the
+// finite-difference band limit (k <= kmax) keep frequency indices below n/4 in
+// magnitude only, in both directions: after the first slice half of the
+// row-frequency columns are zero.  States between passes therefore hold the
+// columns [0, nx/4) and [3nx/4, nx) only (the others are neither written nor
+// read), the column pass runs on those nx/2 columns, and of its spectrum only
+// the rows [0, ny/4) and [3ny/4, ny) are multiplied.  The dropped values are
+// exact zeros of the same sums, so results do not change.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,6 +40,9 @@ enum PassAFlags : int {
   A_ADJ = 256,      // adjoint of x t: dV = -2 sigma Im(conj(h) t psi) to out_f
                     // (psi from in2), line <- conj(t) line
   A_MULT_TC = 512,  // x t from a precomputed transmission slice (PassAArgs.tr)
+  A_BI = 1024,      // the input is a band-limited state: columns outside the band
+                    // count as zero and are not read
+  A_BO = 2048,      // only the band's columns of the result are written
 };
 enum PassBMode : int {
   B_FWD_ONLY = 0,    // FFT_col
@@ -96,6 +109,8 @@ struct PassBArgs {
   float2 fd_c;         // B_FD: rc dz^2 4 pi^2 (pi = 3.14159, gradKernel U.cu:959)
   float kin2, kout2;   // B_DETECT: annulus kin^2 <= kx^2+ky^2 < kout^2 (FP32 decision)
   int accumulate;      // B_CTF_ADJ: add to out instead of storing
+  int band;            // B_CTF, B_CTF_ADJ, B_CBED, B_DETECT: the band's columns only (the
+                       // propagating, band-limiting and FD modes always)
   int nx, ny;
   long long batch_stride_wave;
   // columns of 2048 and 4096 points, propagation, one instance: when set, the

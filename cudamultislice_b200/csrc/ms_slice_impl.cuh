@@ -109,6 +109,11 @@ __host__ __device__ constexpr int col_slot() {
   return ((PL::N + PL::N / PL::R1 + 15) / 16) * 16 + 16 / col_interleave<PL>();
 }
 
+// Whether register j of a line's E (points t + P j) lies in the band, and the
+// column that unit c of the band's n/2 columns is.
+__host__ __device__ constexpr bool in_band(int j, int E) { return j < E / 4 || j >= E - E / 4; }
+MS_D int band_column(int c, int nx) { return c < nx / 4 ? c : c + nx / 2; }
+
 // Programmatic dependent launch: the passes are launched with programmatic
 // stream serialisation, so a pass may start while the previous kernel of the
 // stream drains.  Every pass signals its dependents at entry and waits for its
@@ -258,7 +263,8 @@ MS_D void pass_a_body(PassAArgs a) {
   float2 v[E];
   const float2* in = a.in + row0;
 #pragma unroll
-  for (int j = 0; j < E; ++j) v[j] = in[t + P * j];
+  for (int j = 0; j < E; ++j)
+    v[j] = ((FLAGS & A_BI) == 0 || in_band(j, E)) ? in[t + P * j] : make_float2(0.f, 0.f);
   RowOperands<PL, FLAGS> op;
   op.load(a, inst, line, row0, t);
 
@@ -294,7 +300,8 @@ MS_D void pass_a_body(PassAArgs a) {
       for (int j = 0; j < E; ++j) v[j] = cscale(v[j], a.scale);
     }
 #pragma unroll
-    for (int j = 0; j < E; ++j) o[t + P * j] = v[j];
+    for (int j = 0; j < E; ++j)
+      if ((FLAGS & A_BO) == 0 || in_band(j, E)) o[t + P * j] = v[j];
   }
 }
 
@@ -317,6 +324,11 @@ __host__ __device__ constexpr bool col_stages_ky() { return col_uses_ky<MODE>() 
 template <class PL, int MODE>
 __host__ __device__ constexpr bool col_stages_py() { return col_uses_py<MODE>() && PL::N <= 1024; }
 
+// Modes that keep the band's frequencies only, in both directions.
+template <int MODE>
+__host__ __device__ constexpr bool col_band_limited() {
+  return MODE == B_PROPAGATE || MODE == B_PROPAGATE_ADJ || MODE == B_BANDLIMIT || MODE == B_FD;
+}
 template <class PL, int MODE>
 MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restrict__ sky,
                   const float2* __restrict__ spy, int col, int t, long long base) {
@@ -328,6 +340,10 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
     const float2 pxv = a.px[col];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
+      if (!in_band(j, E)) {
+        v[j] = make_float2(0.f, 0.f);
+        continue;
+      }
       const int n = t + P * j;
       const float ky = sky[n];
       // CreatePropsKernel (U.cu:419): keep sqrtf(kx^2+ky^2) < kmax
@@ -341,6 +357,10 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
     const float2 pxv = a.px[col];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
+      if (!in_band(j, E)) {
+        v[j] = make_float2(0.f, 0.f);
+        continue;
+      }
       const int n = t + P * j;
       const float ky = sky[n];
       const bool keep = fadd_x(kx2, fmul_x(ky, ky)) < a.k2_lt;
@@ -361,6 +381,10 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
     const float kx2 = fmul_x(kx, kx);
 #pragma unroll
     for (int j = 0; j < E; ++j) {
+      if (!in_band(j, E)) {
+        v[j] = make_float2(0.f, 0.f);
+        continue;
+      }
       const float ky = sky[t + P * j];
       const bool keep = fadd_x(kx2, fmul_x(ky, ky)) < a.k2_le;  // sqrt(k^2) <= kmax
       v[j] = keep ? cscale(v[j], scale) : make_float2(0.f, 0.f);
@@ -372,6 +396,10 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
     float2* sp = a.spec + base;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
+      if (!in_band(j, E)) {
+        v[j] = make_float2(0.f, 0.f);
+        continue;
+      }
       const int n = t + P * j;
       const float ky = sky[n];
       const float ky2 = fmul_x(ky, ky);
@@ -395,11 +423,12 @@ __global__ void __launch_bounds__(cols_per_cta<PL>() * PL::P, col_min_ctas<PL>()
   extern __shared__ float2 smem[];
   const int nx = a.nx;
   const int c0 = blockIdx.x * CB;
+  const bool band = col_band_limited<MODE>() || a.band;
   const long long base = (long long)blockIdx.y * a.batch_stride_wave;
   const float scale = a.scale;
   const int g = threadIdx.x / GS, gr = threadIdx.x % GS;
   const int cl = g * CW + gr % CW, t = gr / CW;
-  const int col = c0 + cl;
+  const int col = band ? band_column(c0 + cl, nx) : c0 + cl;
   float2* sm = smem + cl * LS;
 
   // constant frequency tables for the pointwise work (written before any pass
@@ -641,7 +670,7 @@ __global__ void __launch_bounds__(CB * PL::P, CB == 2 ? 2 : 1)
   extern __shared__ __align__(1024) float2 smem_tma[];
   __shared__ __align__(8) unsigned long long mbar;
   float2* stage = smem_tma;  // [NY][CB], then the exchange slots
-  const int c0 = blockIdx.x * CB;
+  const int c0 = band_column(blockIdx.x * CB, a.nx);
   const int cl = threadIdx.x % CB, t = threadIdx.x / CB;
   const int col = c0 + cl;
   float2* sm = smem_tma + cl * LS;
@@ -698,7 +727,7 @@ cudaError_t run_b(const PassBArgs& a, int batch, cudaStream_t s) {
   constexpr int CB = cols_per_cta<PL>();
   constexpr int TCB = 2;  // columns per CTA of the staged pass (two CTAs per SM)
   if constexpr (MODE == B_PROPAGATE && PL::N >= 2048 && TCB * PL::P <= 1024) {
-    if (a.err && batch == 1 && a.nx % TCB == 0 && a.ny == PL::N &&
+    if (a.err && batch == 1 && a.nx % (4 * TCB) == 0 && a.ny == PL::N &&
         ((uintptr_t)a.in % 16) == 0 && ((uintptr_t)a.out % 16) == 0 && ((size_t)a.nx * sizeof(float2)) % 16 == 0) {
       CUtensorMap tin, tout;
       if (wave_tensor_map(&tin, a.in, a.nx, a.ny, TCB) && wave_tensor_map(&tout, a.out, a.nx, a.ny, TCB)) {
@@ -712,7 +741,7 @@ cudaError_t run_b(const PassBArgs& a, int batch, cudaStream_t s) {
         static unsigned long long done = 0;
         if (cudaError_t e = set_smem_once(done, kernel, smem)) return e;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(a.nx / TCB, 1);
+        cfg.gridDim = dim3(a.nx / 2 / TCB, 1);
         cfg.blockDim = dim3(TCB * PL::P);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
@@ -725,30 +754,35 @@ cudaError_t run_b(const PassBArgs& a, int batch, cudaStream_t s) {
   const size_t smem = (size_t)CB * col_slot<PL>() * sizeof(float2) +
                       (col_stages_ky<PL, MODE>() ? (size_t)(PL::N + 1) / 2 * sizeof(float2) : 0) +
                       (col_stages_py<PL, MODE>() ? (size_t)PL::N * sizeof(float2) : 0);
-  if (a.nx % CB) return cudaErrorInvalidValue;
+  const int cols = (col_band_limited<MODE>() || a.band) ? a.nx / 2 : a.nx;
+  if (a.nx % 4 || cols % CB) return cudaErrorInvalidValue;
   auto kernel = k_pass_b<PL, MODE>;
   static unsigned long long done = 0;
   if (cudaError_t e = set_smem_once(done, kernel, smem)) return e;
-  return launch_pdl(kernel, dim3(a.nx / CB, batch), CB * PL::P, smem, s, a);
+  return launch_pdl(kernel, dim3(cols / CB, batch), CB * PL::P, smem, s, a);
 }
 
 template <class PL>
 cudaError_t dispatch_a_plan(const PassAArgs& a, int flags, int batch, cudaStream_t s) {
   switch (flags) {
     case A_FWD: return run_a<PL, A_FWD>(a, batch, s);
+    case A_FWD | A_BO: return run_a<PL, A_FWD | A_BO>(a, batch, s);
     case A_INV: return run_a<PL, A_INV>(a, batch, s);
-    case A_MULT_T | A_FWD: return run_a<PL, A_MULT_T | A_FWD>(a, batch, s);
-    case A_INV | A_MULT_T | A_FWD: return run_a<PL, A_INV | A_MULT_T | A_FWD>(a, batch, s);
+    case A_INV | A_BI: return run_a<PL, A_INV | A_BI>(a, batch, s);
+    case A_MULT_T | A_FWD | A_BO: return run_a<PL, A_MULT_T | A_FWD | A_BO>(a, batch, s);
+    case A_INV | A_MULT_T | A_FWD | A_BI | A_BO: return run_a<PL, A_INV | A_MULT_T | A_FWD | A_BI | A_BO>(a, batch, s);
     case A_INV | A_INTENSITY: return run_a<PL, A_INV | A_INTENSITY>(a, batch, s);
-    case A_INV | A_REAL: return run_a<PL, A_INV | A_REAL>(a, batch, s);
-    case A_INV | A_FD | A_FWD: return run_a<PL, A_INV | A_FD | A_FWD>(a, batch, s);
-    case A_SAVE | A_MULT_T | A_FWD: return run_a<PL, A_SAVE | A_MULT_T | A_FWD>(a, batch, s);
-    case A_INV | A_SAVE | A_MULT_T | A_FWD: return run_a<PL, A_INV | A_SAVE | A_MULT_T | A_FWD>(a, batch, s);
-    case A_INV | A_RESID: return run_a<PL, A_INV | A_RESID>(a, batch, s);
-    case A_INV | A_RESID | A_FWD: return run_a<PL, A_INV | A_RESID | A_FWD>(a, batch, s);
-    case A_INV | A_ADJ | A_FWD: return run_a<PL, A_INV | A_ADJ | A_FWD>(a, batch, s);
-    case A_MULT_TC | A_FWD: return run_a<PL, A_MULT_TC | A_FWD>(a, batch, s);
-    case A_INV | A_MULT_TC | A_FWD: return run_a<PL, A_INV | A_MULT_TC | A_FWD>(a, batch, s);
+    case A_INV | A_INTENSITY | A_BI: return run_a<PL, A_INV | A_INTENSITY | A_BI>(a, batch, s);
+    case A_INV | A_REAL | A_BI: return run_a<PL, A_INV | A_REAL | A_BI>(a, batch, s);
+    case A_INV | A_FD | A_FWD | A_BO: return run_a<PL, A_INV | A_FD | A_FWD | A_BO>(a, batch, s);
+    case A_INV | A_FD | A_FWD | A_BI | A_BO: return run_a<PL, A_INV | A_FD | A_FWD | A_BI | A_BO>(a, batch, s);
+    case A_SAVE | A_MULT_T | A_FWD | A_BO: return run_a<PL, A_SAVE | A_MULT_T | A_FWD | A_BO>(a, batch, s);
+    case A_INV | A_SAVE | A_MULT_T | A_FWD | A_BI | A_BO: return run_a<PL, A_INV | A_SAVE | A_MULT_T | A_FWD | A_BI | A_BO>(a, batch, s);
+    case A_INV | A_RESID | A_BI: return run_a<PL, A_INV | A_RESID | A_BI>(a, batch, s);
+    case A_INV | A_RESID | A_FWD | A_BI | A_BO: return run_a<PL, A_INV | A_RESID | A_FWD | A_BI | A_BO>(a, batch, s);
+    case A_INV | A_ADJ | A_FWD | A_BI | A_BO: return run_a<PL, A_INV | A_ADJ | A_FWD | A_BI | A_BO>(a, batch, s);
+    case A_MULT_TC | A_FWD | A_BO: return run_a<PL, A_MULT_TC | A_FWD | A_BO>(a, batch, s);
+    case A_INV | A_MULT_TC | A_FWD | A_BI | A_BO: return run_a<PL, A_INV | A_MULT_TC | A_FWD | A_BI | A_BO>(a, batch, s);
     default: return cudaErrorInvalidValue;
   }
 }

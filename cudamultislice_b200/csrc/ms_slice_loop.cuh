@@ -12,9 +12,9 @@
 //
 // Work split (lines of N points, one warp per line, E = N/32 points per
 // thread): row r goes to CTA r % G, warp r / G; column unit u (CW adjacent
-// columns, CW warps interleaved so that every warp access covers whole 32-byte
-// sectors) to CTA u % G, group u / G.  A wave of 1024^2 puts at most 7 rows
-// and 8 columns on one SM per phase.
+// columns of the band's N/2, CW warps interleaved so that every warp access
+// covers whole 32-byte sectors) to CTA u % G, group u / G.  A wave of 1024^2
+// puts at most 7 rows and 4 columns on one SM per phase.
 //
 // Grid barrier: a monotonic arrival counter (zeroed before each launch); the
 // k-th barrier waits for k * G arrivals.  Each wait is bounded by a time limit
@@ -131,7 +131,7 @@ MS_D void loop_row(const PassAArgs& a, const float2* in, float2* out, const floa
   float2 v[E];
   float vv[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) v[j] = in[row0 + t + P * j];
+  for (int j = 0; j < E; ++j) v[j] = (!INV || in_band(j, E)) ? in[row0 + t + P * j] : make_float2(0.f, 0.f);
 #pragma unroll
   for (int j = 0; j < E; ++j) vv[j] = V[row0 + t + P * j];
   if constexpr (INV) {
@@ -142,7 +142,8 @@ MS_D void loop_row(const PassAArgs& a, const float2* in, float2* out, const floa
   transmit_line<E>(v, vv, a.sigma);
   fft::line_fft<PL>(v, sm, t, a.tw);
 #pragma unroll
-  for (int j = 0; j < E; ++j) out[row0 + t + P * j] = v[j];
+  for (int j = 0; j < E; ++j)
+    if (in_band(j, E)) out[row0 + t + P * j] = v[j];
 }
 
 // Column phase of one unit of CW columns starting at c0: FFT_col -> x P/N
@@ -152,7 +153,7 @@ MS_D void loop_col(const PassBArgs& b, float2* wave, int c0, int cl, int t, floa
                    const float* __restrict__ sky, const float2* __restrict__ spy) {
   constexpr int E = PL::E, P = PL::P, GS = CW * P;
   const int nx = b.nx;
-  const int col = c0 + cl;
+  const int col = band_column(c0, nx) + cl;
   const float2* src = wave + (long long)t * nx + col;
   const int step = P * nx;
   float2 v[E];
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(NT, 1) k_slice_loop(LoopArgs L) {
     if (!loop_barrier<TIGHT, FENCED>(L.sync, ++epoch)) return;
     // ---- column phase ----
     if (s + 1 < L.S) prefetch_rows<PL>(V + L.vstride, G);
-    for (int u = g * G + blockIdx.x; u < L.b.nx / CW; u += GROUPS * G)
+    for (int u = g * G + blockIdx.x; u < L.b.nx / 2 / CW; u += GROUPS * G)
       loop_col<PL, CW>(L.b, L.wave, u * CW, cl, t, smem + (g * CW + cl) * SH::COL_SLOT, sky, spy);
     if (s + 1 < L.S && !loop_barrier<TIGHT>(L.sync, ++epoch)) return;
   }
@@ -245,7 +246,7 @@ MS_D void batch_row(const LoopGroup& G, int s, int inst, int line, int t, float2
   const long long q0 = inst * G.inst_stride + (long long)s * G.slice_stride + (long long)line * NX;
   float2 v[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) v[j] = w[t + P * j];
+  for (int j = 0; j < E; ++j) v[j] = (first || in_band(j, E)) ? w[t + P * j] : make_float2(0.f, 0.f);
   if constexpr (!TC) {
     float vv[E];
 #pragma unroll
@@ -270,7 +271,8 @@ MS_D void batch_row(const LoopGroup& G, int s, int inst, int line, int t, float2
   }
   fft::line_fft<PL>(v, sm, t, G.a.tw);
 #pragma unroll
-  for (int j = 0; j < E; ++j) w[t + P * j] = v[j];
+  for (int j = 0; j < E; ++j)
+    if (in_band(j, E)) w[t + P * j] = v[j];
 }
 
 // Column phase of one unit of a batched instance: FFT_col, then either the
@@ -285,7 +287,7 @@ MS_D void batch_col(const LoopGroup& G, int inst, int c0, int cl, int t, float2*
   const int nx = NY;
   const long long nn = (long long)NY * NY;
   float2* base = G.wave + inst * nn;
-  const int col = c0 + cl;
+  const int col = band_column(c0, nx) + cl;
   const float2* src = base + (long long)t * nx + col;
   const int step = P * nx;
   float2 v[E];
@@ -374,7 +376,7 @@ __global__ void __launch_bounds__(256, 1) k_batch_loop(BatchLoopArgs L) {
   constexpr int RSLOT = SA::ROW_SLOT > SB::ROW_SLOT ? SA::ROW_SLOT : SB::ROW_SLOT;
   static_assert(SH::LINES_ROWS * RSLOT <= SH::EXCH && GROUPS * CW * CSLOT <= SH::EXCH, "exchange slots overflow");
   const long long rows0 = (long long)G0.B * N0, rows1 = has1 ? (long long)G1.B * N1 : 0;
-  const long long units0 = (long long)G0.B * (N0 / CW), units1 = has1 ? (long long)G1.B * (N1 / CW) : 0;
+  const long long units0 = (long long)G0.B * (N0 / 2 / CW), units1 = has1 ? (long long)G1.B * (N1 / 2 / CW) : 0;
   unsigned int epoch = 0;
   for (int s = 0; s < L.S; ++s) {
     const bool first = s == 0, last = s + 1 == L.S;
@@ -391,11 +393,11 @@ __global__ void __launch_bounds__(256, 1) k_batch_loop(BatchLoopArgs L) {
     for (long long u = (long long)g * G + blockIdx.x; u < units0 + units1; u += (long long)GROUPS * G) {
       float2* sm = smem + (g * CW + cl) * CSLOT;
       if (u < units0) {
-        batch_col<PL0, CW>(G0, (int)(u / (N0 / CW)), (int)(u % (N0 / CW)) * CW, cl, t, sm, sky0, spy0,
+        batch_col<PL0, CW>(G0, (int)(u / (N0 / 2 / CW)), (int)(u % (N0 / 2 / CW)) * CW, cl, t, sm, sky0, spy0,
                            last && G0.sig != nullptr);
       } else {
         const long long v = u - units0;
-        batch_col<PL1, CW>(G1, (int)(v / (N1 / CW)), (int)(v % (N1 / CW)) * CW, cl, t, sm, sky1, spy1,
+        batch_col<PL1, CW>(G1, (int)(v / (N1 / 2 / CW)), (int)(v % (N1 / 2 / CW)) * CW, cl, t, sm, sky1, spy1,
                            last && G1.sig != nullptr);
       }
     }
