@@ -208,7 +208,7 @@ class Engine {
         return MS_OK;
       case MS_OPT_LOOP_VARIANT:
         if (value < -1 || value >= slice_loop_variants())
-          return fail(MS_ERR_INVALID, "loop variant must be -1 (tuned) or a variant index");
+          return fail(MS_ERR_INVALID, "loop variant must be -1 (by grid) or a variant index");
         forced_loop_ = value;
         invalidate_graph();
         return MS_OK;
@@ -1858,14 +1858,20 @@ class Engine {
     int S = 0;
     if (use_fused() && pot_mode_ == 0 && overlap_build_ && have_index_ && have_fp_ && have_freq_) {
       if (int rc = get_slices(true, &S)) return rc;
-      if (S >= 1 && (!stack_valid_ || nstack_ != S) && separable_ok()) return run_conventional_streamed(S, nslices);
+      // 256^2 and 512^2 with the persistent loop: build first, then the loop in
+      // one launch (two pass launches a slice bound those runs on the host:
+      // 256^2, 42 slices 0.90 ms against 0.69; 512^2, 102 slices 1.82 against
+      // 1.70; at 1024^2 the overlap wins, 4.62 against 4.79)
+      const bool build_first = use_loop() && nx_ < 1024;
+      if (S >= 1 && (!stack_valid_ || nstack_ != S) && separable_ok() && !build_first)
+        return run_conventional_streamed(S, nslices);
     }
     if (int rc = build_stack(&S)) return rc;
     if (int rc = ensure_prop_tables(convdz_)) return rc;
     const bool loop = use_loop();
     if (use_fused()) {
       if (loop) {
-        if (int rc = prepare_loop(S)) return rc;
+        if (int rc = prepare_loop()) return rc;
       } else {
         plan_for(1);  // tune outside the capture (tuning allocates and synchronises)
       }
@@ -1926,54 +1932,16 @@ class Engine {
   bool use_loop() const {
     return use_fused() && !loop_off_ && forced_plan_ < 0 && slice_loop_supported(nx_, ny_);
   }
-  // Chooses the loop kernel variant for this grid (forced by
-  // MS_OPT_LOOP_VARIANT, else tuned once: every variant runs a short loop of
-  // up to 16 slices over the resident stack, three times after two warm-up
-  // launches, and the fastest is kept).  Needs the potential stack; outside
-  // stream capture (it synchronises).
-  int prepare_loop(int S) {
-    if (loop_grid_ > 0 && loop_grid_n_ == nx_ && loop_tuned_for_ == forced_loop_) return MS_OK;
-    int best_v = -1, best_grid = 0;
-    float best_t = INFINITY;
-    const int St = std::min(S, 16);
-    for (int v = 0; v < slice_loop_variants(); ++v) {
-      if (forced_loop_ >= 0 && v != forced_loop_) continue;
-      int grid = 0;
-      if (slice_loop_prepare(nx_, v, &grid) != cudaSuccess) {
-        cudaGetLastError();
-        continue;
-      }
-      if (forced_loop_ >= 0) {
-        best_v = v;
-        best_grid = grid;
-        break;
-      }
-      loop_v_ = v;
-      loop_grid_ = grid;
-      for (int k = 0; k < 2; ++k)
-        if (int rc = enqueue_loop(d_stack_.p, St, k == 0)) return rc;
-      MS_TRY(cudaEventRecord(ev0_, stream_));
-      for (int k = 0; k < 3; ++k)
-        if (int rc = enqueue_loop(d_stack_.p, St, false)) return rc;
-      MS_TRY(cudaEventRecord(ev1_, stream_));
-      MS_TRY(cudaMemcpyAsync(h_loop_err_, d_loop_sync_.p + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream_));
-      MS_TRY(cudaStreamSynchronize(stream_));
-      launches += 5;
-      if (*h_loop_err_ != 0) return loop_timeout_fail();
-      float ms = 0.0f;
-      MS_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
-      if (ms < best_t) {
-        best_t = ms;
-        best_v = v;
-        best_grid = grid;
-      }
-    }
-    if (best_v < 0) return fail(MS_ERR_CUDA, "no persistent slice-loop variant could be prepared on this device");
-    loop_v_ = best_v;
-    loop_grid_ = best_grid;
+  // The loop kernel variant for this grid (forced by MS_OPT_LOOP_VARIANT, else
+  // slice_loop_variant), its shared-memory limit raised and its grid found.
+  int prepare_loop() {
+    const int v = forced_loop_ >= 0 ? forced_loop_ : slice_loop_variant(nx_);
+    if (loop_grid_ > 0 && loop_grid_n_ == nx_ && loop_v_ == v) return MS_OK;
+    int grid = 0;
+    MS_TRY(slice_loop_prepare(nx_, v, &grid));
+    loop_v_ = v;
+    loop_grid_ = grid;
     loop_grid_n_ = nx_;
-    loop_tuned_for_ = forced_loop_;
-    domain_ = 0;  // tuning left scratch in the wave; every run starts from psi0
     return MS_OK;
   }
   int potential_sum_info(int* last, int* next) {
@@ -1993,17 +1961,16 @@ class Engine {
     int S = 0;
     if (int rc = build_stack(&S)) return rc;
     if (int rc = ensure_prop_tables(convdz_)) return rc;
-    if (int rc = prepare_loop(S)) return rc;
+    if (int rc = prepare_loop()) return rc;
     *variant = loop_v_;
     *columns = slice_loop_columns(loop_v_);
     *grid = loop_grid_;
     return MS_OK;
   }
   LoopArgs loop_args(const float* Vstack, int S) {
-    const int v = slice_loop_plan(nx_, loop_v_);
     LoopArgs L{};
-    L.a = passa_args(d_psi0_.p, d_psi_.p, v);
-    L.b = passb_args(d_psi_.p, d_psi_.p, v);
+    L.a = passa_args(d_psi0_.p, d_psi_.p, slice_loop_plan(nx_, loop_v_, false));
+    L.b = passb_args(d_psi_.p, d_psi_.p, slice_loop_plan(nx_, loop_v_, true));
     L.psi0 = d_psi0_.p;
     L.wave = d_psi_.p;
     L.Vstack = Vstack;
@@ -2042,7 +2009,7 @@ class Engine {
     const size_t N = (size_t)nx_ * ny_;
     const bool loop = use_loop() && steps <= S;
     if (loop) {
-      if (int rc = prepare_loop(S)) return rc;
+      if (int rc = prepare_loop()) return rc;
     }
     MS_TRY(cudaStreamSynchronize(stream_));
     // whole steps, back to back (the persistent loop: one launch per repetition)
@@ -3163,7 +3130,7 @@ class Engine {
   DevBuf<unsigned int> d_loop_sync_;
   DevBuf<int> d_pass_err_;  // error word of the column pass's tensor-copy waits
   unsigned int* h_loop_err_ = nullptr;
-  int loop_grid_ = 0, loop_grid_n_ = 0, loop_v_ = 0, forced_loop_ = -1, loop_tuned_for_ = -2;
+  int loop_grid_ = 0, loop_grid_n_ = 0, loop_v_ = 0, forced_loop_ = -1;
   bool loop_off_ = false;
   unsigned int loop_extra_ = 0;
   unsigned long long loop_limit_ns_ = 1000000000ull;

@@ -119,6 +119,26 @@ struct Dif {
   }
 };
 
+// The network for inputs that are zero in the middle half (R/4 <= index <
+// 3R/4), not read: the first stage's butterflies have one live input each.
+template <int R, bool PK, int J = 0>
+MS_D void dft_band_first(float2 (&x)[R]) {
+  if constexpr (J < R / 4) {
+    x[J + R / 2] = twc<J, R, false>(x[J]);
+  } else {
+    const float2 b = x[J + R / 2];  // 0 + b, and (0 - b) W_R^J = b W_R^(J + R/2)
+    x[J] = b;
+    x[J + R / 2] = twc<J + R / 2, R, false>(b);
+  }
+  if constexpr (J + 1 < R / 2) dft_band_first<R, PK, J + 1>(x);
+}
+template <int R, bool PK>
+MS_D void dft_band(float2 (&x)[R]) {
+  static_assert(R % 4 == 0, "band input needs a first radix of at least 4");
+  dft_band_first<R, PK>(x);
+  Dif<R, R / 4, false, PK>::run(x);
+}
+
 template <int R, bool INV, bool PK = false>
 MS_D void dft(float2 (&x)[R]) {
   if constexpr (R > 1) Dif<R, R / 2, INV, PK>::run(x);
@@ -202,8 +222,14 @@ struct PassR {
 
 // Twiddles of pass IDX for this thread's butterflies, loaded ahead of the
 // barrier that precedes the pass so their latency overlaps the wait.  Plans
-// with more than 16 twiddles per thread load them at use instead.
-template <class PL, int IDX>
+// with more than 16 twiddles per thread load them at use instead.  TS: the
+// table lies in shared memory.
+template <bool TS>
+MS_D float2 twiddle(const float2* __restrict__ tw) {
+  if constexpr (TS) return *tw;
+  else return __ldg(tw);
+}
+template <class PL, int IDX, bool TS>
 struct TwiddleRegs {
   static constexpr int R = PassR<PL, IDX>::R, NB = PL::E / R;
   static constexpr bool PREFETCH = NB * (R - 1) <= 16;
@@ -215,7 +241,7 @@ struct TwiddleRegs {
       for (int b = 0; b < NB; ++b) {
         const int k = (t + PL::P * b) & (NS - 1);
 #pragma unroll
-        for (int r = 1; r < R; ++r) w[b * (R - 1) + r - 1] = __ldg(tw + TWO + r * NS + k);
+        for (int r = 1; r < R; ++r) w[b * (R - 1) + r - 1] = twiddle<TS>(tw + TWO + r * NS + k);
       }
     }
   }
@@ -223,19 +249,21 @@ struct TwiddleRegs {
     if constexpr (PREFETCH) {
       return w[b * (R - 1) + r - 1];
     } else {
-      return __ldg(tw + PassR<PL, IDX>::TW + r * PassR<PL, IDX>::NS + k);
+      return twiddle<TS>(tw + PassR<PL, IDX>::TW + r * PassR<PL, IDX>::NS + k);
     }
   }
 };
 
 // Stockham pass IDX >= 1: the previous pass has written the slot but not yet
 // synchronised.  Forward transform only; the inverse is conj(FFT(conj(x))).
-template <class PL, int IDX, int GS = 0>
+// BOUT: registers outside the band (the middle half) are left undefined, so
+// the compiler drops the butterfly outputs nothing reads.
+template <class PL, int IDX, int GS = 0, bool BOUT = false, bool TS = false>
 MS_D void forward_pass(float2 (&v)[PL::E], float2* __restrict__ sm, int t, const float2* __restrict__ tw) {
   constexpr int N = PL::N, E = PL::E, P = PL::P;
   constexpr int R = PassR<PL, IDX>::R, NS = PassR<PL, IDX>::NS, LR = ilog2(R);
   constexpr bool LAST = (IDX == PL::NPASS - 1);
-  TwiddleRegs<PL, IDX> tr;
+  TwiddleRegs<PL, IDX, TS> tr;
   tr.load(tw, t);
   line_sync<PL, GS>();
   if constexpr (LAST) {
@@ -249,7 +277,11 @@ MS_D void forward_pass(float2 (&v)[PL::E], float2* __restrict__ sm, int t, const
       for (int r = 1; r < R; ++r) x[r] = cmul(x[r], tr.get(tw, b, r, i));
       dft<R, false, PL::PK>(x);
 #pragma unroll
-      for (int q = 0; q < R; ++q) v[b + q * (E / R)] = x[brev(q, LR)];
+      for (int q = 0; q < R; ++q) {
+        constexpr int EE = E;
+        const int o = b + q * (E / R);
+        if (!BOUT || o < EE / 4 || o >= EE - EE / 4) v[o] = x[brev(q, LR)];
+      }
     }
     line_sync<PL, GS>();
   } else {
@@ -275,7 +307,7 @@ MS_D void forward_pass(float2 (&v)[PL::E], float2* __restrict__ sm, int t, const
 #pragma unroll
       for (int q = 0; q < R; ++q) sm[padi<PL>(base + q * NS)] = x[brev(q, LR)];
     }
-    forward_pass<PL, IDX + 1, GS>(v, sm, t, tw);
+    forward_pass<PL, IDX + 1, GS, BOUT, TS>(v, sm, t, tw);
   }
 }
 
@@ -283,7 +315,9 @@ MS_D void forward_pass(float2 (&v)[PL::E], float2* __restrict__ sm, int t, const
 // group.  `sm` is this line's shared slot (PL::SLOT points), `tw` the plan's
 // twiddle table.  Every thread of the line's barrier group (line_sync<PL, GS>)
 // must call this: it synchronises.  On return the slot may be reused.
-template <class PL, int GS = 0>
+// BIN: the registers of the middle half count as zero and are not read; BOUT:
+// those of the result are left undefined; TS: tw lies in shared memory.
+template <class PL, int GS = 0, bool BIN = false, bool BOUT = false, bool TS = false>
 MS_D void line_fft(float2 (&v)[PL::E], float2* __restrict__ sm, int t, const float2* __restrict__ tw) {
   constexpr int E = PL::E, P = PL::P, R1 = PL::R1, L1 = ilog2(R1);
 #pragma unroll
@@ -291,12 +325,13 @@ MS_D void line_fft(float2 (&v)[PL::E], float2* __restrict__ sm, int t, const flo
     float2 x[R1];
 #pragma unroll
     for (int r = 0; r < R1; ++r) x[r] = v[b + r * (E / R1)];
-    dft<R1, false, PL::PK>(x);
+    if constexpr (BIN) dft_band<R1, PL::PK>(x);
+    else dft<R1, false, PL::PK>(x);
     const int i = t + P * b;
 #pragma unroll
     for (int q = 0; q < R1; ++q) sm[padi<PL>(i * R1 + q)] = x[brev(q, L1)];
   }
-  forward_pass<PL, 1, GS>(v, sm, t, tw);
+  forward_pass<PL, 1, GS, BOUT, TS>(v, sm, t, tw);
 }
 
 template <int E>

@@ -191,12 +191,14 @@ cudaError_t batch_loop_prepare(int n0, int n1, bool tc, int* grid);
 cudaError_t launch_batch_loop(const BatchLoopArgs& L, int grid, cudaStream_t s);
 
 // Grids the persistent loop is provided for (square 256, 512, 1024), and the
-// FFT plan variant (twiddle tables) that loop kernel variant `variant` uses.
+// FFT plan variants (twiddle tables) that loop kernel variant `variant` uses
+// for rows and columns.
 bool slice_loop_supported(int nx, int ny);
-int slice_loop_plan(int n, int variant);
-// Kernel variants of the loop (column unit width, grid-barrier form), and the
-// columns per unit of one variant.
+int slice_loop_plan(int n, int variant, bool columns);
+// Kernel variants of the loop (column unit width, warps per column, grid-barrier
+// form), the one that runs a grid of n, and the columns per unit of one variant.
 int slice_loop_variants();
+int slice_loop_variant(int n);
 int slice_loop_columns(int variant);
 // Raises a loop variant's shared-memory limit and returns its grid (one CTA
 // per SM, all resident).

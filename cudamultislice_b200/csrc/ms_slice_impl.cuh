@@ -329,15 +329,30 @@ template <int MODE>
 __host__ __device__ constexpr bool col_band_limited() {
   return MODE == B_PROPAGATE || MODE == B_PROPAGATE_ADJ || MODE == B_BANDLIMIT || MODE == B_FD;
 }
+// The column's own factors.  The persistent loop loads them with the column's
+// points (its barriers empty L1); the pass kernels at use: their registers are
+// capped, and held across the first transform they cost more than the wait
+// (2-10% of a pass).
+struct ColFactors {
+  float kx;
+  float2 px;
+  template <int MODE>
+  MS_D static ColFactors load(const PassBArgs& a, int col) {
+    ColFactors f{0.0f, make_float2(0.f, 0.f)};
+    if (col_uses_ky<MODE>()) f.kx = a.kx[col];
+    if (col_uses_py<MODE>()) f.px = a.px[col];
+    return f;
+  }
+};
 template <class PL, int MODE>
-MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restrict__ sky,
+MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const ColFactors& f, const float* __restrict__ sky,
                   const float2* __restrict__ spy, int col, int t, long long base) {
   constexpr int NY = PL::N, E = PL::E, P = PL::P;
   const float scale = a.scale;
+  const float kx = f.kx;
   if constexpr (MODE == B_PROPAGATE) {
-    const float kx = a.kx[col];
     const float kx2 = fmul_x(kx, kx);
-    const float2 pxv = a.px[col];
+    const float2 pxv = f.px;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
       if (!in_band(j, E)) {
@@ -352,9 +367,8 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
       v[j] = keep ? cmul(cmul(v[j], pxv), spy[n]) : make_float2(0.f, 0.f);
     }
   } else if constexpr (MODE == B_PROPAGATE_ADJ) {
-    const float kx = a.kx[col];
     const float kx2 = fmul_x(kx, kx);
-    const float2 pxv = a.px[col];
+    const float2 pxv = f.px;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
       if (!in_band(j, E)) {
@@ -367,7 +381,6 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
       v[j] = keep ? cscale(cmul(cmul(v[j], cconj(pxv)), cconj(spy[n])), scale) : make_float2(0.f, 0.f);
     }
   } else if constexpr (MODE == B_CTF || MODE == B_CTF_ADJ) {
-    const float kx = a.kx[col];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
       const int n = t + P * j;
@@ -377,7 +390,6 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
     }
   } else if constexpr (MODE == B_BANDLIMIT) {
     // BandLimitKernel (U.cu:1025-1042): keep k <= kmax
-    const float kx = a.kx[col];
     const float kx2 = fmul_x(kx, kx);
 #pragma unroll
     for (int j = 0; j < E; ++j) {
@@ -391,7 +403,6 @@ MS_D void col_mid(float2 (&v)[PL::E], const PassBArgs& a, const float* __restric
     }
   } else if constexpr (MODE == B_FD) {
     // Psi_{n+1} = BL (FFT2(q) + c k^2 Psi_n)
-    const float kx = a.kx[col];
     const float kx2 = fmul_x(kx, kx);
     float2* sp = a.spec + base;
 #pragma unroll
@@ -464,7 +475,7 @@ __global__ void __launch_bounds__(cols_per_cta<PL>() * PL::P, col_min_ctas<PL>()
       if constexpr (MODE == B_INV_ONLY) {
         fft::conj_all(v);
       } else if constexpr (TWO) {
-        col_mid<PL, MODE>(v, a, sky, spy, col, t, base);
+        col_mid<PL, MODE>(v, a, ColFactors::load<MODE>(a, col), sky, spy, col, t, base);
         fft::conj_all(v);
       }
     } else {
@@ -703,7 +714,7 @@ __global__ void __launch_bounds__(CB * PL::P, CB == 2 ? 2 : 1)
 #pragma unroll 1
   for (int it = 0; it < 2; ++it) {
     fft::line_fft<fft::PaddedPlan<PL>, GS>(v, sm, t, a.tw);
-    if (it == 0) col_mid<PL, B_PROPAGATE>(v, a, a.ky, a.py, col, t, 0);
+    if (it == 0) col_mid<PL, B_PROPAGATE>(v, a, ColFactors::load<B_PROPAGATE>(a, col), a.ky, a.py, col, t, 0);
     fft::conj_all(v);
   }
   __syncthreads();  // (every exchange done: the buffer is the staging area again)

@@ -6,17 +6,20 @@ namespace ms {
 
 namespace {
 
+template <int N, bool WIDE>
+using LoopPL = typename PlanSel<N, LoopPlan<N, WIDE>::V>::T;
 template <int N, int V>
-using LoopPL = typename PlanSel<N, LoopPlan<N, (LoopVariant<V>::NT > 256)>::V>::T;
-
+using LoopSH = LoopShape<LoopPL<N, false>, LoopPL<N, LoopVariant<V>::WIDE>, LoopVariant<V>::CW>;
+template <int N, int V>
+constexpr auto loop_kernel() {
+  using LV = LoopVariant<V>;
+  return k_slice_loop<LoopPL<N, false>, LoopPL<N, LV::WIDE>, LV::CW, LV::TIGHT, LV::FENCED>;
+}
 
 template <int N, int V>
 cudaError_t loop_prepare(int* grid) {
-  using PL = LoopPL<N, V>;
-  using LV = LoopVariant<V>;
-  using SH = LoopShape<PL, LV::CW, LV::NT>;
-  static_assert(PL::P * LV::NT == 32 * 256 || PL::P * LV::NT == 64 * 512, "plan and CTA size must match");
-  auto kernel = k_slice_loop<PL, LV::CW, LV::TIGHT, LV::NT, LV::FENCED>;
+  using SH = LoopSH<N, V>;
+  auto kernel = loop_kernel<N, V>();
   static unsigned long long done = 0;
   if (cudaError_t e = set_smem_once(done, kernel, SH::SMEM)) return e;
   int dev = 0, sms = 0, per_sm = 0;
@@ -30,9 +33,7 @@ cudaError_t loop_prepare(int* grid) {
 
 template <int N, int V>
 cudaError_t loop_launch(const LoopArgs& L, int grid, cudaStream_t s) {
-  using PL = LoopPL<N, V>;
-  using LV = LoopVariant<V>;
-  using SH = LoopShape<PL, LV::CW, LV::NT>;
+  using SH = LoopSH<N, V>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(SH::NT);
@@ -43,7 +44,7 @@ cudaError_t loop_launch(const LoopArgs& L, int grid, cudaStream_t s) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_slice_loop<PL, LV::CW, LV::TIGHT, LV::NT, LV::FENCED>, L);
+  return cudaLaunchKernelEx(&cfg, loop_kernel<N, V>(), L);
 }
 
 template <int V>
@@ -69,8 +70,9 @@ cudaError_t launch_v(const LoopArgs& L, int grid, cudaStream_t s) {
 
 bool slice_loop_supported(int nx, int ny) { return nx == ny && (nx == 256 || nx == 512 || nx == 1024); }
 
-int slice_loop_plan(int n, int variant) {
-  const bool wide = variant >= 5 && variant <= 7;
+int slice_loop_plan(int n, int variant, bool columns) {
+  const bool wide = columns && (variant == 5 || variant == 6);
+  static_assert(LoopVariant<5>::WIDE && LoopVariant<6>::WIDE && !LoopVariant<7>::WIDE, "the wide variants");
   switch (n) {
     case 256: return wide ? LoopPlan<256, true>::V : LoopPlan<256, false>::V;
     case 512: return wide ? LoopPlan<512, true>::V : LoopPlan<512, false>::V;
@@ -80,6 +82,13 @@ int slice_loop_plan(int n, int variant) {
 }
 
 int slice_loop_variants() { return kLoopVariants; }
+
+// Unfenced barriers everywhere (fenced: 1.2-1.5 us a slice more).  1024^2: four
+// columns of one warp each per SM keep every scheduler busy (11.4 us a slice;
+// two-warp columns 11.4, units of two 12.4-12.7).  512^2 and 256^2 have one or
+// two columns per SM: two warps each, units of two (6.3 and 5.0 us; one-warp
+// units of four 6.5 and 5.0).
+int slice_loop_variant(int n) { return n >= 1024 ? 9 : 6; }
 
 int slice_loop_columns(int variant) {
   switch (variant) {

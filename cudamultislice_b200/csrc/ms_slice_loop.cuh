@@ -62,95 +62,146 @@ MS_D unsigned long long global_ns() {
   return t;
 }
 
-// Grid barrier number `epoch` (1, 2, ...).  Returns false (in every thread of
-// the CTA) when the grid must stop: this CTA's wait ran out or another CTA
-// reported an error.  TIGHT = false: the arrival is an atomic add and the
-// wait polls with a short sleep; TIGHT = true: the arrival is a release
-// reduction (no round trip) and the wait polls back to back, checking the
-// clock and the error word every 32 polls.  FENCED: full fences around the
-// arrival and after the wait (as cooperative groups' grid sync); without
-// them the release reduction and the acquire load carry the ordering (both
-// are cumulative over what the CTA's bar.sync has ordered before them).
+// Grid barrier number `epoch` (1, 2, ...) in two halves, so that work which no
+// other CTA's result feeds runs between the arrival and the wait.
+//
+// TIGHT = false: the wait polls with a short sleep, inside full fences; TIGHT =
+// true: it polls back to back, checking the clock and the error word every 32
+// polls, and starts only when the arrival's own return value shows that others
+// are still to come (148 CTAs polling from the start slow the last arrivals:
+// 1.24 us a barrier with a release reduction, 1.15 with this).  FENCED: full
+// fences around the arrival and after the wait (as cooperative groups' grid
+// sync); without them the acquire-release arrival and the acquire load carry
+// the ordering (both are cumulative over what the CTA's bar.sync has ordered
+// before them).  Measured and left out: arrivals spread over eight counters
+// (1.37 us), relaxed polls with a fence after the wait (1.38), one CTA of a
+// cluster for two or four (2.1), an arrival per warp (1.9).
 template <bool TIGHT, bool FENCED = true>
-MS_D bool loop_barrier(const LoopSync& s, unsigned int epoch) {
+MS_D unsigned int loop_arrive(const LoopSync& s) {
   __syncthreads();
-  int ok = 1;
+  unsigned int seen = 0;
   if (threadIdx.x == 0) {
     if constexpr (FENCED || !TIGHT) __threadfence();
-    if constexpr (TIGHT)
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(s.count) : "memory");
-    else
-      atomicAdd(s.count, 1u);
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(s.count) : "memory");
+    ++seen;
+  }
+  return seen;
+}
+// `seen`: loop_arrive's result.  Returns false (in every thread of the CTA)
+// when the grid must stop: this CTA's wait ran out or another CTA reported an
+// error.
+template <bool TIGHT, bool FENCED = true>
+MS_D bool loop_wait(const LoopSync& s, unsigned int epoch, unsigned int seen) {
+  int ok = 1;
+  if (threadIdx.x == 0) {
     const unsigned int target = epoch * gridDim.x + s.expect_extra;
-    const unsigned long long t0 = global_ns();
-    for (unsigned int it = 0;; ++it) {
-      unsigned int v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(s.count) : "memory");
-      if (v >= target) break;
-      if (!TIGHT || (it & 31) == 31) {
-        if (*reinterpret_cast<volatile int*>(s.error) != 0) {
-          ok = 0;
-          break;
+    if (seen < target) {
+      const unsigned long long t0 = global_ns();
+      for (unsigned int it = 0;; ++it) {
+        unsigned int v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(s.count) : "memory");
+        if (v >= target) break;
+        if (!TIGHT || (it & 31) == 31) {
+          if (*reinterpret_cast<volatile int*>(s.error) != 0) {
+            ok = 0;
+            break;
+          }
+          if (global_ns() - t0 > s.limit_ns) {
+            atomicExch(s.error, kLoopTimeout);
+            ok = 0;
+            break;
+          }
         }
-        if (global_ns() - t0 > s.limit_ns) {
-          atomicExch(s.error, kLoopTimeout);
-          ok = 0;
-          break;
-        }
+        if constexpr (!TIGHT) __nanosleep(32);
       }
-      if constexpr (!TIGHT) __nanosleep(32);
     }
     if constexpr (FENCED || !TIGHT) __threadfence();
   }
   return __syncthreads_and(ok) != 0;
 }
+template <bool TIGHT, bool FENCED = true>
+MS_D bool loop_barrier(const LoopSync& s, unsigned int epoch) {
+  return loop_wait<TIGHT, FENCED>(s, epoch, loop_arrive<TIGHT, FENCED>(s));
+}
 
-template <class PL, int CW, int NT_>
+// PL: rows, PC: columns (the same length; the columns may take more threads
+// per line: a CTA has at most four columns of a 1024^2 phase).
+template <class PL, class PC, int CW>
 struct LoopShape {
   static constexpr int N = PL::N, E = PL::E, P = PL::P;
-  static_assert(P == 32 || P == 64, "the persistent loop runs lines of one or two warps");
-  static constexpr int NT = NT_;                 // threads per CTA
+  static_assert(P == 32 && PC::N == N && (PC::P == 32 || PC::P == 64), "rows of one warp, columns of one or two");
+  static constexpr int NT = 256;                 // threads per CTA
   static constexpr int LINES = NT / P;           // rows per CTA per round
-  static constexpr int GS = CW * P;              // threads of one column unit
+  static constexpr int GS = CW * PC::P;          // threads of one column unit
   static constexpr int GROUPS = NT / GS;         // column units per CTA per round
   static_assert(GROUPS >= 1 && NT % GS == 0, "column units must tile the CTA");
   static constexpr int ROW_SLOT = PL::SLOT;
-  static constexpr int COL_SLOT = ((N + N / PL::R1 + 15) / 16) * 16 + 16 / CW;
+  static constexpr int COL_SLOT = ((N + N / PC::R1 + 15) / 16) * 16 + 16 / CW;
   static constexpr int EXCH = (LINES * ROW_SLOT > GROUPS * CW * COL_SLOT) ? LINES * ROW_SLOT : GROUPS * CW * COL_SLOT;
-  // exchange slots, then ky (N floats, padded to float2) and py (N float2)
-  static constexpr size_t SMEM = ((size_t)EXCH + (N + 1) / 2 + N) * sizeof(float2);
+  // exchange slots, then ky (N floats, padded to float2), py (N float2) and the
+  // twiddle tables of rows and columns (one when the plans are the same): the
+  // barriers' acquires empty L1, and every phase fetched them from L2 again
+  static constexpr int KY = EXCH, PY = KY + (N + 1) / 2, TWR = PY + N;
+  static constexpr bool ONE_TW = PL::E == PC::E;
+  static constexpr int TWC = ONE_TW ? TWR : TWR + PL::TWSIZE;
+  static constexpr size_t SMEM = ((size_t)TWC + PC::TWSIZE) * sizeof(float2);
 };
 
-// Row phase of one line: [IFFT_row] -> x exp(i sigma V) -> FFT_row, in place
-// on the wave (or from psi0 on the first slice).
+// The transmission exp(i sigma V) of a line's points: the polynomial-only
+// sincos when every phase of the warp is within a quarter turn of 0
+// (bit-identical, the usual case for slices of a few angstroms), else the
+// reduced one.
+template <int E>
+MS_D void transmission_line(float2 (&tr)[E], const float* __restrict__ V, int t, float sigma) {
+  constexpr int P = 32;
+  float ph[E];
+  bool small = true;
+#pragma unroll
+  for (int j = 0; j < E; ++j) ph[j] = V[t + P * j];
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    ph[j] = fmul_x(sigma, ph[j]);
+    small = small && sincos_small_ok(ph[j]);
+  }
+  if (__all_sync(0xffffffffu, small)) {
+#pragma unroll
+    for (int j = 0; j < E; j += 2)
+      sincos_small2(ph[j], ph[j + 1], &tr[j].y, &tr[j].x, &tr[j + 1].y, &tr[j + 1].x);
+  } else {
+#pragma unroll
+    for (int j = 0; j < E; j += 2)
+      sincos_red2(ph[j], ph[j + 1], &tr[j].y, &tr[j].x, &tr[j + 1].y, &tr[j + 1].x);
+  }
+}
+
+// Row phase of one line: [IFFT_row] -> x t -> FFT_row, in place on the wave's
+// band (or from psi0 on the first slice).
 template <class PL, bool INV>
-MS_D void loop_row(const PassAArgs& a, const float2* in, float2* out, const float* __restrict__ V, int line, int t,
-                   float2* sm) {
+MS_D void loop_row(const float2* in, float2* out, const float2 (&tr)[PL::E], int line, int t, float2* sm,
+                   const float2* stw) {
   constexpr int NX = PL::N, E = PL::E, P = PL::P;
   const long long row0 = (long long)line * NX;
   float2 v[E];
-  float vv[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) v[j] = (!INV || in_band(j, E)) ? in[row0 + t + P * j] : make_float2(0.f, 0.f);
-#pragma unroll
-  for (int j = 0; j < E; ++j) vv[j] = V[row0 + t + P * j];
   if constexpr (INV) {
     fft::conj_all(v);
-    fft::line_fft<PL>(v, sm, t, a.tw);
+    fft::line_fft<PL, 0, true, false, true>(v, sm, t, stw);
     fft::conj_all(v);
   }
-  transmit_line<E>(v, vv, a.sigma);
-  fft::line_fft<PL>(v, sm, t, a.tw);
+#pragma unroll
+  for (int j = 0; j < E; ++j) v[j] = cmul(v[j], tr[j]);
+  fft::line_fft<PL, 0, false, true, true>(v, sm, t, stw);
 #pragma unroll
   for (int j = 0; j < E; ++j)
     if (in_band(j, E)) out[row0 + t + P * j] = v[j];
 }
 
-// Column phase of one unit of CW columns starting at c0: FFT_col -> x P/N
-// (band-limited) -> IFFT_col, in place.
+// Column phase of one unit of CW columns starting at the band's column c0:
+// FFT_col -> x P/N (band-limited) -> IFFT_col, in place.
 template <class PL, int CW>
 MS_D void loop_col(const PassBArgs& b, float2* wave, int c0, int cl, int t, float2* sm,
-                   const float* __restrict__ sky, const float2* __restrict__ spy) {
+                   const float* __restrict__ sky, const float2* __restrict__ spy, const float2* stw) {
   constexpr int E = PL::E, P = PL::P, GS = CW * P;
   const int nx = b.nx;
   const int col = band_column(c0, nx) + cl;
@@ -159,16 +210,12 @@ MS_D void loop_col(const PassBArgs& b, float2* wave, int c0, int cl, int t, floa
   float2 v[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) v[j] = src[j * step];
-#pragma unroll 1
-  for (int it = 0; it < 2; ++it) {
-    fft::line_fft<fft::PaddedPlan<PL>, GS>(v, sm, t, b.tw);
-    if (it == 0) {
-      col_mid<PL, B_PROPAGATE>(v, b, sky, spy, col, t, 0);
-      fft::conj_all(v);
-    } else {
-      fft::conj_all(v);
-    }
-  }
+  const ColFactors cf = ColFactors::load<B_PROPAGATE>(b, col);
+  fft::line_fft<fft::PaddedPlan<PL>, GS, false, true, true>(v, sm, t, stw);
+  col_mid<PL, B_PROPAGATE>(v, b, cf, sky, spy, col, t, 0);
+  fft::conj_all(v);
+  fft::line_fft<fft::PaddedPlan<PL>, GS, true, false, true>(v, sm, t, stw);
+  fft::conj_all(v);
   int ostep;
   asm volatile("mov.b32 %0, %1;" : "=r"(ostep) : "r"(step));
   float2* dst = wave + (long long)t * nx + col;
@@ -177,7 +224,7 @@ MS_D void loop_col(const PassBArgs& b, float2* wave, int c0, int cl, int t, floa
 }
 
 // Bulk L2 prefetch of the potential rows this CTA's lines read in the next
-// row phase (issued during the column phase; one 4-byte-per-point row each).
+// row phase (issued before the column phase; one 4-byte-per-point row each).
 template <class PL>
 MS_D void prefetch_rows(const float* V, int G) {
   constexpr int NX = PL::N, P = PL::P;
@@ -190,40 +237,55 @@ MS_D void prefetch_rows(const float* V, int G) {
   }
 }
 
-template <class PL, int CW, bool TIGHT, int NT, bool FENCED = true>
-__global__ void __launch_bounds__(NT, 1) k_slice_loop(LoopArgs L) {
-  using SH = LoopShape<PL, CW, NT>;
-  constexpr int N = PL::N, P = PL::P, GS = SH::GS, GROUPS = SH::GROUPS;
+template <class PL, class PC, int CW, bool TIGHT, bool FENCED>
+__global__ void __launch_bounds__(256, 1) k_slice_loop(LoopArgs L) {
+  using SH = LoopShape<PL, PC, CW>;
+  constexpr int N = PL::N, E = PL::E, P = PL::P, GS = SH::GS, GROUPS = SH::GROUPS;
   extern __shared__ float2 smem[];
-  float* sky = reinterpret_cast<float*>(smem + SH::EXCH);
-  float2* spy = smem + SH::EXCH + (N + 1) / 2;
+  float* sky = reinterpret_cast<float*>(smem + SH::KY);
+  float2* spy = smem + SH::PY;
+  float2 *stwr = smem + SH::TWR, *stwc = smem + SH::TWC;
   for (int i = threadIdx.x; i < N; i += SH::NT) {
     sky[i] = L.b.ky[i];
     spy[i] = L.b.py[i];
   }
+  for (int i = threadIdx.x; i < PL::TWSIZE; i += SH::NT) stwr[i] = L.a.tw[i];
+  if constexpr (!SH::ONE_TW)
+    for (int i = threadIdx.x; i < PC::TWSIZE; i += SH::NT) stwc[i] = L.b.tw[i];
   __syncthreads();
   const int G = gridDim.x;
   const int li = threadIdx.x / P, lt = threadIdx.x % P;  // row line of the CTA, index within it
   // this thread's column-unit coordinates
   const int g = threadIdx.x / GS, gr = threadIdx.x % GS;
   const int cl = gr % CW, t = gr / CW;
+  const int line0 = li * G + blockIdx.x;  // this warp's (first) row of every slice
+  float2* sm = smem + li * SH::ROW_SLOT;
   unsigned int epoch = 0;
+  // the transmission of this warp's row for the coming slice
+  float2 tr[E];
+  if (line0 < N) transmission_line<E>(tr, L.Vstack + (long long)line0 * N, lt, L.a.sigma);
   for (int s = 0; s < L.S; ++s) {
     const float* V = L.Vstack + (long long)s * L.vstride;
     // ---- row phase ----
-    for (int line = li * G + blockIdx.x; line < N; line += SH::LINES * G) {
-      float2* sm = smem + li * SH::ROW_SLOT;
+    for (int line = line0; line < N; line += SH::LINES * G) {
+      if (line != line0) transmission_line<E>(tr, V + (long long)line * N, lt, L.a.sigma);  // (small grids of CTAs)
       if (s == 0)
-        loop_row<PL, false>(L.a, L.psi0, L.wave, V, line, lt, sm);
+        loop_row<PL, false>(L.psi0, L.wave, tr, line, lt, sm, stwr);
       else
-        loop_row<PL, true>(L.a, L.wave, L.wave, V, line, lt, sm);
+        loop_row<PL, true>(L.wave, L.wave, tr, line, lt, sm, stwr);
     }
     if (!loop_barrier<TIGHT, FENCED>(L.sync, ++epoch)) return;
     // ---- column phase ----
-    if (s + 1 < L.S) prefetch_rows<PL>(V + L.vstride, G);
+    const bool more = s + 1 < L.S;
+    if (more) prefetch_rows<PL>(V + L.vstride, G);
     for (int u = g * G + blockIdx.x; u < L.b.nx / 2 / CW; u += GROUPS * G)
-      loop_col<PL, CW>(L.b, L.wave, u * CW, cl, t, smem + (g * CW + cl) * SH::COL_SLOT, sky, spy);
-    if (s + 1 < L.S && !loop_barrier<TIGHT>(L.sync, ++epoch)) return;
+      loop_col<PC, CW>(L.b, L.wave, u * CW, cl, t, smem + (g * CW + cl) * SH::COL_SLOT, sky, spy, stwc);
+    if (!more) return;
+    // the next slice's transmission needs no other CTA's columns: it is formed
+    // while the arrivals come in
+    const unsigned int seen = loop_arrive<TIGHT, FENCED>(L.sync);
+    if (line0 < N) transmission_line<E>(tr, V + L.vstride + (long long)line0 * N, lt, L.a.sigma);
+    if (!loop_wait<TIGHT, FENCED>(L.sync, ++epoch, seen)) return;
   }
 }
 
@@ -253,7 +315,7 @@ MS_D void batch_row(const LoopGroup& G, int s, int inst, int line, int t, float2
     for (int j = 0; j < E; ++j) vv[j] = G.Vstack[q0 + t + P * j];
     if (!first) {
       fft::conj_all(v);
-      fft::line_fft<PL>(v, sm, t, G.a.tw);
+      fft::line_fft<PL, 0, true>(v, sm, t, G.a.tw);
       fft::conj_all(v);
     }
     transmit_line<E>(v, vv, G.a.sigma);
@@ -263,13 +325,13 @@ MS_D void batch_row(const LoopGroup& G, int s, int inst, int line, int t, float2
     for (int j = 0; j < E; ++j) tc[j] = G.tstack[q0 + t + P * j];
     if (!first) {
       fft::conj_all(v);
-      fft::line_fft<PL>(v, sm, t, G.a.tw);
+      fft::line_fft<PL, 0, true>(v, sm, t, G.a.tw);
       fft::conj_all(v);
     }
 #pragma unroll
     for (int j = 0; j < E; ++j) v[j] = cmul(v[j], tc[j]);
   }
-  fft::line_fft<PL>(v, sm, t, G.a.tw);
+  fft::line_fft<PL, 0, false, true>(v, sm, t, G.a.tw);
 #pragma unroll
   for (int j = 0; j < E; ++j)
     if (in_band(j, E)) w[t + P * j] = v[j];
@@ -293,10 +355,10 @@ MS_D void batch_col(const LoopGroup& G, int inst, int c0, int cl, int t, float2*
   float2 v[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) v[j] = src[j * step];
+  const ColFactors cf = ColFactors::load<B_PROPAGATE>(G.b, col);
   if (detect) {
     fft::line_fft<fft::PaddedPlan<PL>, GS>(v, sm, t, G.b.tw);
-    const float kx = G.b.kx[col];
-    const float kx2 = fmul_x(kx, kx);
+    const float kx2 = fmul_x(cf.kx, cf.kx);
     float acc = 0.0f;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
@@ -311,14 +373,11 @@ MS_D void batch_col(const LoopGroup& G, int inst, int c0, int cl, int t, float2*
     if ((threadIdx.x & 31) == 0 && d != 0.0) atomicAdd(G.sig + inst, d * (double)G.b.scale);
     return;
   }
-#pragma unroll 1
-  for (int it = 0; it < 2; ++it) {
-    fft::line_fft<fft::PaddedPlan<PL>, GS>(v, sm, t, G.b.tw);
-    if (it == 0) {
-      col_mid<PL, B_PROPAGATE>(v, G.b, sky, spy, col, t, 0);
-    }
-    fft::conj_all(v);
-  }
+  fft::line_fft<fft::PaddedPlan<PL>, GS, false, true>(v, sm, t, G.b.tw);
+  col_mid<PL, B_PROPAGATE>(v, G.b, cf, sky, spy, col, t, 0);
+  fft::conj_all(v);
+  fft::line_fft<fft::PaddedPlan<PL>, GS, true>(v, sm, t, G.b.tw);
+  fft::conj_all(v);
   int ostep;
   asm volatile("mov.b32 %0, %1;" : "=r"(ostep) : "r"(step));
   float2* dst = base + (long long)t * nx + col;
@@ -328,8 +387,8 @@ MS_D void batch_col(const LoopGroup& G, int inst, int c0, int cl, int t, float2*
 
 template <class PL0, class PL1, int CW>
 struct BatchShape {
-  using A = LoopShape<PL0, CW, 256>;
-  using B = LoopShape<PL1, CW, 256>;
+  using A = LoopShape<PL0, PL0, CW>;
+  using B = LoopShape<PL1, PL1, CW>;
   static constexpr int NT = 256;
   static constexpr int LINES_ROWS = NT / 32;  // row lines in flight per CTA
   static constexpr int EXCH = A::EXCH > B::EXCH ? A::EXCH : B::EXCH;
@@ -405,25 +464,29 @@ __global__ void __launch_bounds__(256, 1) k_batch_loop(BatchLoopArgs L) {
   }
 }
 
-// Variants of the loop kernel (chosen per grid by the engine's autotuner):
-// narrow (lines of one warp, 256-thread CTAs) or wide (lines of two warps,
-// 512-thread CTAs: twice the warps per SM, one more exchange pass), the
-// column unit width CW and the barrier form.
+// Variants of the loop kernel: columns of one warp or two (WIDE: twice the
+// warps per column, one more exchange), the column unit width CW and the
+// barrier form.
 constexpr int kLoopVariants = 10;
+template <int CW_, bool WIDE_, bool TIGHT_, bool FENCED_>
+struct LoopForm {
+  static constexpr int CW = CW_;
+  static constexpr bool WIDE = WIDE_, TIGHT = TIGHT_, FENCED = FENCED_;
+};
 template <int V> struct LoopVariant;
-template <> struct LoopVariant<0> { static constexpr int CW = 4, NT = 256; static constexpr bool TIGHT = false, FENCED = true; };
-template <> struct LoopVariant<1> { static constexpr int CW = 8, NT = 256; static constexpr bool TIGHT = false, FENCED = true; };
-template <> struct LoopVariant<2> { static constexpr int CW = 4, NT = 256; static constexpr bool TIGHT = true, FENCED = true; };
-template <> struct LoopVariant<3> { static constexpr int CW = 8, NT = 256; static constexpr bool TIGHT = true, FENCED = true; };
-template <> struct LoopVariant<4> { static constexpr int CW = 2, NT = 256; static constexpr bool TIGHT = true, FENCED = true; };
-template <> struct LoopVariant<5> { static constexpr int CW = 4, NT = 512; static constexpr bool TIGHT = true, FENCED = true; };
-template <> struct LoopVariant<6> { static constexpr int CW = 2, NT = 512; static constexpr bool TIGHT = true, FENCED = true; };
-template <> struct LoopVariant<7> { static constexpr int CW = 8, NT = 512; static constexpr bool TIGHT = true, FENCED = true; };
-template <> struct LoopVariant<8> { static constexpr int CW = 8, NT = 256; static constexpr bool TIGHT = true, FENCED = false; };
-template <> struct LoopVariant<9> { static constexpr int CW = 4, NT = 256; static constexpr bool TIGHT = true, FENCED = false; };
+template <> struct LoopVariant<0> : LoopForm<4, false, false, true> {};
+template <> struct LoopVariant<1> : LoopForm<8, false, false, true> {};
+template <> struct LoopVariant<2> : LoopForm<4, false, true, true> {};
+template <> struct LoopVariant<3> : LoopForm<8, false, true, true> {};
+template <> struct LoopVariant<4> : LoopForm<2, false, true, true> {};
+template <> struct LoopVariant<5> : LoopForm<4, true, true, false> {};
+template <> struct LoopVariant<6> : LoopForm<2, true, true, false> {};
+template <> struct LoopVariant<7> : LoopForm<2, false, true, false> {};
+template <> struct LoopVariant<8> : LoopForm<8, false, true, false> {};
+template <> struct LoopVariant<9> : LoopForm<4, false, true, false> {};
 
 // FFT plan variant (PlanSel) of the loop per line length: the packed plan with
-// one warp per line (narrow loop variants) or two warps per line (wide).
+// one warp per line (rows, and columns of the narrow variants) or two (wide).
 template <int N, bool WIDE>
 struct LoopPlan;
 template <> struct LoopPlan<256, false> { static constexpr int V = 4; };

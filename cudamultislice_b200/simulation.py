@@ -103,7 +103,7 @@ class ManagedMultisliceSimulation:
         self._chk(self._L.ms_set_option(self._h, 5, 0 if persistent else 1))
 
     def SetLoopVariant(self, variant: int):
-        """Persistent slice loop kernel variant: -1 tuned (default), 0..4 forced."""
+        """Persistent slice loop kernel variant: -1 by grid size (default), 0..9 forced."""
         self._chk(self._L.ms_set_option(self._h, 8, int(variant)))
 
     def SliceLoop(self):

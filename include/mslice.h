@@ -82,14 +82,14 @@ enum {
   MS_OPT_LOOP_WAIT_TEST = 7, /* test hook: > 0 makes every grid barrier wait for that many
                                arrivals more than the grid has, so the wait bound runs out
                                (0 = off, the default) */
-  MS_OPT_LOOP_VARIANT = 8,  /* persistent slice loop kernel variant: -1 = tuned on the
-                               device once per grid (default); 0..9 = force one: 0-4 run
-                               lines of one warp in 256-thread CTAs (column units of 4, 8,
-                               4, 8, 2 columns; barrier sleep-poll for 0-1, release
-                               reduction with tight poll for 2-4); 5-7 lines of two warps
-                               in 512-thread CTAs (units of 4, 2, 8 columns, tight poll);
-                               8-9 as 3 and 2 with the ordering carried by the release
-                               reduction and the acquire poll alone (no full fences) */
+  MS_OPT_LOOP_VARIANT = 8,  /* persistent slice loop kernel variant: -1 = by grid size
+                               (default); 0..9 = force one.  Rows run one warp per line in
+                               256-thread CTAs; columns one warp each (0-4, 7-9; units of 4,
+                               8, 4, 8, 2, and 2, 8, 4 columns) or two (5, 6; units of 4, 2);
+                               barriers: sleep-poll inside full fences (0-1), tight poll
+                               inside full fences (2-4), tight poll with the ordering
+                               carried by the acquire-release arrival and the acquire poll
+                               alone (5-9) */
   MS_OPT_POTENTIAL_TILE = 9, /* conventional potential kernel tile: -1 = default (separable:
                                by grid and pixel size; per sub-plane: tuned on the device
                                per grid); per-sub-plane kernel 0, 1, 2 = 32 x 8, 16 x 16,
@@ -109,9 +109,10 @@ enum {
   MS_OPT_BUILD_OVERLAP = 11 /* ms_run_conventional when the potential stack must be built:
                                1 = run each slice's fused passes on a second stream while the
                                next slices' potentials are built (default; separable
-                               potential, fused path); 0 = build the stack, then run the
-                               slices.  Runs over a resident stack replay the persistent
-                               loop either way. */
+                               potential, fused path; grids below 1024^2 that run the
+                               persistent loop build first, which is faster there); 0 =
+                               build the stack, then run the slices.  Runs over a resident
+                               stack replay the persistent loop either way. */
 };
 
 /* ---- lifecycle ---- */
@@ -387,8 +388,8 @@ ms_status ms_get_fft_plan(ms_sim* sim, int batch, int* row_variant, int* col_var
  * device-tuned choice. */
 ms_status ms_get_raster_tuning(ms_sim* sim, int* batch, int* persistent);
 /* The persistent slice loop this grid runs: kernel variant (-1 when the loop
- * does not run here), columns per column unit, CTAs (one per SM); tunes the
- * variant first if needed (MS_OPT_LOOP_VARIANT). */
+ * does not run here), columns per column unit, CTAs (one per SM)
+ * (MS_OPT_LOOP_VARIANT). */
 ms_status ms_get_slice_loop(ms_sim* sim, int* variant, int* columns, int* grid);
 /* Number of this library's kernels launched by the handle so far. */
 ms_status ms_get_launch_count(ms_sim* sim, long long* out);
