@@ -19,9 +19,11 @@
 #include <fstream>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <sstream>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -86,6 +88,57 @@ struct DevBuf {
   }
 };
 
+// Pinned chunks for large copies to and from pageable buffers, shared by the
+// handles of the process (pinning 4 MB takes a millisecond or two, as long as
+// the copies it speeds up): at most kSets sets, each lent to one copy at a
+// time, freed when the last handle goes.
+class StagePool {
+ public:
+  static constexpr int kThreads = 8, kSets = 4;
+  static constexpr size_t kChunk = 512u << 10;
+  static StagePool& get() {
+    static StagePool p;
+    return p;
+  }
+  void add_handle() {
+    std::lock_guard<std::mutex> lk(mu_);
+    ++handles_;
+  }
+  void drop_handle() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (--handles_ > 0) return;
+    for (char* p : free_) cudaFreeHost(p);
+    sets_ -= (int)free_.size();
+    free_.clear();
+  }
+  // kThreads chunks, or null when all sets are out or pinning fails.
+  char* take() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (!free_.empty()) {
+      char* p = free_.back();
+      free_.pop_back();
+      return p;
+    }
+    char* p = nullptr;
+    if (sets_ >= kSets || cudaHostAlloc((void**)&p, kThreads * kChunk, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    ++sets_;
+    return p;
+  }
+  void give(char* p) {
+    std::lock_guard<std::mutex> lk(mu_);
+    free_.push_back(p);
+  }
+
+ private:
+  StagePool() { free_.reserve(kSets); }
+  std::mutex mu_;
+  std::vector<char*> free_;
+  int sets_ = 0, handles_ = 0;
+};
+
 // Element symbols for Z = 1..103 (the rows of fparams.dat).
 static const char* const kElements[103] = {
     "H",  "He", "Li", "Be", "B",  "C",  "N",  "O",  "F",  "Ne", "Na", "Mg", "Al", "Si", "P",  "S",  "Cl", "Ar",
@@ -113,11 +166,14 @@ static int znum(const std::string& s, bool full) {
 // ---------------------------------------------------------------------------
 class Engine {
  public:
-  explicit Engine(int device) : device_(device) {}
+  explicit Engine(int device) : device_(device) { StagePool::get().add_handle(); }
   ~Engine() {
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (fd_graph_) cudaGraphExecDestroy(fd_graph_);
     if (h_loop_err_) cudaFreeHost(h_loop_err_);
+    for (cudaEvent_t e : ev_stage_)
+      if (e) cudaEventDestroy(e);
+    StagePool::get().drop_handle();
     if (have_plan_) cufftDestroy(plan_);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
@@ -952,8 +1008,7 @@ class Engine {
     if (!have_waves_) return fail(MS_ERR_STATE, "wavefunctions not initialised");
     if (!dst) return fail(MS_ERR_INVALID, "null destination");
     if (int rc = ensure_real()) return rc;
-    MS_TRY(cudaMemcpyAsync(dst, d_psi_.p, sizeof(float2) * nx_ * ny_, cudaMemcpyDeviceToHost, stream_));
-    MS_TRY(cudaStreamSynchronize(stream_));
+    if (int rc = copy_large(dst, d_psi_.p, sizeof(float2) * nx_ * ny_, true)) return rc;
     return check_pass_err();
   }
 
@@ -1178,9 +1233,7 @@ class Engine {
         MS_TRY(pw_abs2(d_t2_.p, d_img_.p + (size_t)i * N, 1.0f, g, stream_, &launches));
       }
     }
-    MS_TRY(cudaMemcpyAsync(images, d_img_.p, sizeof(float) * N * n, cudaMemcpyDeviceToHost, stream_));
-    MS_TRY(cudaStreamSynchronize(stream_));
-    return MS_OK;
+    return copy_large(images, d_img_.p, sizeof(float) * N * n, true);
   }
 
   int im_value(int x, int y, float* out) {
@@ -2150,7 +2203,7 @@ class Engine {
       }
     }
     invalidate_graph();  // the sweep below leaves d_psi_ at psi_S
-    MS_TRY(cudaMemcpyAsync(d_T_.p, targets, sizeof(float) * N * nd, cudaMemcpyHostToDevice, stream_));
+    if (int rc = copy_large(d_T_.p, targets, sizeof(float) * N * nd, false)) return rc;
     MS_TRY(cudaMemsetAsync(d_loss_.p, 0, sizeof(double), stream_));
     // (after any atom-position adjoint still on the second pixel stream, which
     // an earlier call that failed part-way may have left unjoined)
@@ -2270,9 +2323,9 @@ class Engine {
     MS_TRY(cudaEventRecord(ev1_, stream_));
     MS_TRY(cudaMemcpyAsync(loss, d_loss_.p, sizeof(double), cudaMemcpyDeviceToHost, stream_));
     if (images)
-      MS_TRY(cudaMemcpyAsync(images, d_img_.p, sizeof(float) * N * nd, cudaMemcpyDeviceToHost, stream_));
+      if (int rc = copy_large(images, d_img_.p, sizeof(float) * N * nd, true)) return rc;
     if (grad && dLdV)
-      MS_TRY(cudaMemcpyAsync(dLdV, d_dV_.p, sizeof(float) * N * S, cudaMemcpyDeviceToHost, stream_));
+      if (int rc = copy_large(dLdV, d_dV_.p, sizeof(float) * N * S, true)) return rc;
     if (grad && dLdxy)
       MS_TRY(cudaMemcpyAsync(dLdxy, d_dxy_.p, sizeof(double) * 2 * natoms_, cudaMemcpyDeviceToHost, stream_));
     MS_TRY(cudaStreamSynchronize(stream_));
@@ -2437,12 +2490,85 @@ class Engine {
     return e == cudaSuccess ? cudaStreamSynchronize(stream_) : e;
   }
 
+  // Large copies between device memory and a caller's pageable buffer, ordered
+  // after the handle's stream: a few helper threads, each with its own pinned
+  // chunk, move chunk by chunk, so that the transfers overlap the host copies
+  // and the page faults of a fresh buffer are taken in parallel.  (The
+  // driver's own path for pageable memory is one thread: 33 MB into a fresh
+  // numpy array 5-7 ms, here under 2.)  Buffers below kStageMin, pinned ones
+  // and those that cannot be staged go straight to cudaMemcpyAsync.  To the
+  // host the call returns when the buffer is filled, from it when the buffer
+  // may be reused.
+  static constexpr size_t kStageMin = 2u << 20;
+  int copy_large(void* dst, const void* src, size_t bytes, bool to_host) {
+    constexpr size_t chunk = StagePool::kChunk;
+    const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t nt = std::min({(size_t)StagePool::kThreads, hw, bytes / kStageMin * 2});
+    char* pins = nullptr;
+    if (nt >= 2) {
+      cudaPointerAttributes at{};
+      if (cudaPointerGetAttributes(&at, to_host ? dst : src) != cudaSuccess)
+        cudaGetLastError();
+      else if (at.type == cudaMemoryTypeUnregistered && ensure_stage_events() == cudaSuccess)
+        pins = StagePool::get().take();
+    }
+    if (!pins) {
+      MS_TRY(cudaMemcpyAsync(dst, src, bytes, kind, stream_));
+      if (to_host) MS_TRY(cudaStreamSynchronize(stream_));
+      return MS_OK;
+    }
+    const size_t chunks = (bytes + chunk - 1) / chunk;
+    cudaError_t rc[StagePool::kThreads] = {};
+    auto work = [&](size_t t) {
+      cudaError_t e = cudaSetDevice(device_);
+      char* pin = pins + t * chunk;
+      for (size_t c = t; c < chunks && e == cudaSuccess; c += nt) {
+        const size_t o = c * chunk, n = std::min(chunk, bytes - o);
+        if (!to_host) std::memcpy(pin, static_cast<const char*>(src) + o, n);
+        e = to_host ? cudaMemcpyAsync(pin, static_cast<const char*>(src) + o, n, kind, stream_)
+                    : cudaMemcpyAsync(static_cast<char*>(dst) + o, pin, n, kind, stream_);
+        if (e == cudaSuccess) e = cudaEventRecord(ev_stage_[t], stream_);
+        if (e == cudaSuccess) e = cudaEventSynchronize(ev_stage_[t]);  // (filled, or free again)
+        if (to_host && e == cudaSuccess) std::memcpy(static_cast<char*>(dst) + o, pin, n);
+      }
+      rc[t] = e;
+    };
+    {
+      std::thread th[StagePool::kThreads];
+      size_t started = 1;
+      try {
+        for (; started < nt; ++started) th[started] = std::thread(work, started);
+      } catch (const std::system_error&) {
+        // (no more threads: this one takes the remaining shares)
+      }
+      work(0);
+      for (size_t t = started; t < nt; ++t) work(t);
+      for (size_t t = 1; t < started; ++t) th[t].join();
+    }
+    bool ok = true;
+    for (cudaError_t e : rc) ok = ok && e == cudaSuccess;
+    // (after a failure a transfer may still be in flight on a chunk)
+    if (!ok) cudaStreamSynchronize(stream_);
+    StagePool::get().give(pins);
+    for (cudaError_t e : rc) MS_TRY(e);
+    return MS_OK;
+  }
+
   int fail(int code, const std::string& m) {
     err = m;
     return code;
   }
 
  private:
+  cudaEvent_t ev_stage_[StagePool::kThreads] = {};  // copy_large's chunks
+  cudaError_t ensure_stage_events() {
+    for (cudaEvent_t& e : ev_stage_)
+      if (!e)
+        if (cudaError_t r = cudaEventCreateWithFlags(&e, cudaEventDisableTiming)) return r;
+    return cudaSuccess;
+  }
+
   static constexpr float FLT_MAX_ = 3.40282347e+38f;
 
   int cuda_fail(cudaError_t e, const char* what) {
