@@ -699,14 +699,13 @@ __global__ void k_gauss_bins(const float* __restrict__ gauss, float* __restrict_
       (float)exp2(-(double)gauss[blockIdx.y * 2 * kGaussJ + j] * (double)m);
 }
 
-// The tables of the slices' atoms, LPA lanes of a warp per atom.  SEGS: with
-// the bins and segments (the forward; the position adjoint reads the rows T
-// only).  Bound: issue, about 730 warp instructions an atom at 16 lanes, half
+// The tables of the slices' atoms, LPA lanes of a warp per atom.  DERIV: the
+// segments hold dG/d(rho^2) (position adjoint) in place of G.  Bound: issue, about 730 warp instructions an atom at 16 lanes, half
 // of them the segments' moments (their exponentials come from gbin), and for
 // few atoms the chain of dependent steps: 32 lanes halve the loops over
 // planes, bins and segments at 1.4 times the instructions (see
 // launch_atom_tables).
-template <bool SEGS, int LPA>
+template <bool DERIV, int LPA>
 __global__ void __launch_bounds__(kTabThreads) k_atom_tables(const __grid_constant__ SepArgs q) {
   constexpr int NA = kTabThreads / LPA;  // atoms per CTA and round
   __shared__ float s_d2[NA][20];
@@ -714,8 +713,8 @@ __global__ void __launch_bounds__(kTabThreads) k_atom_tables(const __grid_consta
   __shared__ float s_asc[NA][20];
   __shared__ int s_tb[NA][20];
   __shared__ __align__(16) float s_T[NA][20][kGaussJ];
-  __shared__ int s_range[SEGS ? NA : 1][2];
-  __shared__ unsigned short s_seg[SEGS ? NA : 1][SEGS ? kRadSegs : 1];
+  __shared__ int s_range[NA][2];
+  __shared__ unsigned short s_seg[NA][kRadSegs];
   constexpr float kLn2 = 0.6931471805599453f;
   // (the planes are read from parameter space)
   const PotArgs& a = q.p;
@@ -800,83 +799,93 @@ __global__ void __launch_bounds__(kTabThreads) k_atom_tables(const __grid_consta
       }
     }
     __syncwarp();
-    if constexpr (SEGS) {
-      // bins: the thresholds below each, the next ones, and which (bin,
-      // thresholds passed) each segment is
-      if (valid && n > 0) {
-        if (j < 2) {  // bins -1 and 100, and the zero segment
-          *reinterpret_cast<float4*>(tab + kTabBin + 4 * (j ? kRadBins + 1 : 0)) =
-              make_float4(1e30f, 1e30f, 1e30f, __int_as_float(kRadSegs + (j ? 0 : kRadMore)));
-          if (j) tab[kTabC4 + kRadSegs] = 0.0f;
-          else *reinterpret_cast<float4*>(tab + kTabSeg + 4 * kRadSegs) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        for (int b = b0 + j; b < kRadBins; b += LPA) {
-          int c = 0;  // thresholds below the bin (s_tb ascends)
-#pragma unroll
-          for (int st = 16; st >= 1; st >>= 1)
-            if (c + st <= n && s_tb[la][c + st - 1] < b) c += st;
-          int e = c;  // ... and through it
-          while (e < n && s_tb[la][e] <= b) ++e;
-          auto asc = [&](int k) { return k < n ? s_asc[la][k] : 1e30f; };
-          *reinterpret_cast<float4*>(tab + kTabBin + 4 * (b + 1)) =
-              make_float4(asc(c), asc(c + 1), asc(c + 2), __int_as_float(b - b0 + c + (e - c > 3 ? kRadMore : 0)));
-          // (segments below the first bin's and past the last bin's counts do not exist)
-          if (b == b0) s_range[la][0] = c;
-          if (b == kRadBins - 1) s_range[la][1] = b - b0 + min(e, n - 1) + 1;
-          for (; c <= min(e, n - 1); ++c) s_seg[la][b - b0 + c] = (unsigned short)(b | c << 8);
-        }
+    // bins: the thresholds below each, the next ones, and which (bin,
+    // thresholds passed) each segment is
+    if (valid && n > 0) {
+      if (j < 2) {  // bins -1 and 100, and the zero segment
+        *reinterpret_cast<float4*>(tab + kTabBin + 4 * (j ? kRadBins + 1 : 0)) =
+            make_float4(1e30f, 1e30f, 1e30f, __int_as_float(kRadSegs + (j ? 0 : kRadMore)));
+        if (j) tab[kTabC4 + kRadSegs] = 0.0f;
+        else *reinterpret_cast<float4*>(tab + kTabSeg + 4 * kRadSegs) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      __syncwarp();
-      if (valid && n > 0) {
-        // (Gaussians in pairs on the packed FP32x2 pipe)
-        f2p al[kGaussJ / 2];
+      for (int b = b0 + j; b < kRadBins; b += LPA) {
+        int c = 0;  // thresholds below the bin (s_tb ascends)
 #pragma unroll
-        for (int i = 0; i < kGaussJ / 2; ++i) al[i] = pk2(-kLn2 * g[2 * i], -kLn2 * g[2 * i + 1]);
-        const float* gb = a.gbin + (size_t)zi * kRadBins * kGaussJ;
-        // (unrolled: the next segments' gbin rows load while these are summed)
-#pragma unroll 2
-        for (int sg = s_range[la][0] + j; sg < s_range[la][1]; sg += LPA) {
-          const int bc = s_seg[la][sg], b = bc & 255, c = bc >> 8;
-          const ulonglong2* T = reinterpret_cast<const ulonglong2*>(s_T[la][n - 1 - c]);
-          const ulonglong2* E = reinterpret_cast<const ulonglong2*>(gb + b * kGaussJ);
-          // moments sum_j T_K[j] exp(-alpha_j s_c) (-alpha_j)^i, i = 0..5
-          f2p mp[6];
-#pragma unroll
-          for (int k = 0; k < 6; ++k) mp[k] = 0ull;
-#pragma unroll
-          for (int i = 0; i < kGaussJ / 4; ++i) {
-            const ulonglong2 e = __ldg(E + i), t = T[i];
-            f2p xa = mul2(t.x, e.x), xb = mul2(t.y, e.y);
-#pragma unroll
-            for (int k = 0; k < 5; ++k) {
-              mp[k] = add2(mp[k], add2(xa, xb));
-              if (k < 4) {
-                xa = mul2(xa, al[2 * i]);
-                xb = mul2(xb, al[2 * i + 1]);
-              }
-            }
-            mp[5] = fma2(xa, al[2 * i], fma2(xb, al[2 * i + 1], mp[5]));
-          }
-          float mo[6];
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            float lo, hi;
-            up2(mp[k], lo, hi);
-            mo[k] = lo + hi;
-          }
-          // half the bin's width: 2^e / 32; Taylor to degree five, the last
-          // term economised over the bin (tau^5 ~ 5/4 h^2 tau^3 - 5/16 h^4 tau)
-          const float h = __int_as_float(((b + kRadBin0) << 19) & 0x7F800000) * 0.03125f, h2 = h * h;
-          const float c5 = mo[5] * (1.0f / 120.0f);
-          *reinterpret_cast<float4*>(tab + kTabSeg + 4 * sg) =
-              make_float4(mo[0], fmaf(-0.3125f * h2 * h2, c5, mo[1]), 0.5f * mo[2],
-                          fmaf(1.25f * h2, c5, mo[3] * (1.0f / 6.0f)));
-          tab[kTabC4 + sg] = mo[4] * (1.0f / 24.0f);
-        }
+        for (int st = 16; st >= 1; st >>= 1)
+          if (c + st <= n && s_tb[la][c + st - 1] < b) c += st;
+        int e = c;  // ... and through it
+        while (e < n && s_tb[la][e] <= b) ++e;
+        auto asc = [&](int k) { return k < n ? s_asc[la][k] : 1e30f; };
+        *reinterpret_cast<float4*>(tab + kTabBin + 4 * (b + 1)) =
+            make_float4(asc(c), asc(c + 1), asc(c + 2), __int_as_float(b - b0 + c + (e - c > 3 ? kRadMore : 0)));
+        // (segments below the first bin's and past the last bin's counts do not exist)
+        if (b == b0) s_range[la][0] = c;
+        if (b == kRadBins - 1) s_range[la][1] = b - b0 + min(e, n - 1) + 1;
+        for (; c <= min(e, n - 1); ++c) s_seg[la][b - b0 + c] = (unsigned short)(b | c << 8);
       }
-      __syncwarp();
     }
+    __syncwarp();
+    if (valid && n > 0) {
+      // (Gaussians in pairs on the packed FP32x2 pipe)
+      f2p al[kGaussJ / 2];
+#pragma unroll
+      for (int i = 0; i < kGaussJ / 2; ++i) al[i] = pk2(-kLn2 * g[2 * i], -kLn2 * g[2 * i + 1]);
+      const float* gb = a.gbin + (size_t)zi * kRadBins * kGaussJ;
+      // (unrolled: the next segments' gbin rows load while these are summed)
+#pragma unroll 2
+      for (int sg = s_range[la][0] + j; sg < s_range[la][1]; sg += LPA) {
+        const int bc = s_seg[la][sg], b = bc & 255, c = bc >> 8;
+        const ulonglong2* T = reinterpret_cast<const ulonglong2*>(s_T[la][n - 1 - c]);
+        const ulonglong2* E = reinterpret_cast<const ulonglong2*>(gb + b * kGaussJ);
+        // moments sum_j T_K[j] exp(-alpha_j s_c) (-alpha_j)^i, i = 0..5
+        f2p mp[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) mp[k] = 0ull;
+#pragma unroll
+        for (int i = 0; i < kGaussJ / 4; ++i) {
+          const ulonglong2 e = __ldg(E + i), t = T[i];
+          f2p xa = mul2(t.x, e.x), xb = mul2(t.y, e.y);
+          if constexpr (DERIV) {
+            xa = mul2(xa, al[2 * i]);
+            xb = mul2(xb, al[2 * i + 1]);
+          }
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            mp[k] = add2(mp[k], add2(xa, xb));
+            if (k < 4) {
+              xa = mul2(xa, al[2 * i]);
+              xb = mul2(xb, al[2 * i + 1]);
+            }
+          }
+          mp[5] = fma2(xa, al[2 * i], fma2(xb, al[2 * i + 1], mp[5]));
+        }
+        float mo[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          float lo, hi;
+          up2(mp[k], lo, hi);
+          mo[k] = lo + hi;
+        }
+        // half the bin's width: 2^e / 32; Taylor to degree five, the last
+        // term economised over the bin (tau^5 ~ 5/4 h^2 tau^3 - 5/16 h^4 tau)
+        const float h = __int_as_float(((b + kRadBin0) << 19) & 0x7F800000) * 0.03125f, h2 = h * h;
+        const float c5 = mo[5] * (1.0f / 120.0f);
+        *reinterpret_cast<float4*>(tab + kTabSeg + 4 * sg) =
+            make_float4(mo[0], fmaf(-0.3125f * h2 * h2, c5, mo[1]), 0.5f * mo[2],
+                        fmaf(1.25f * h2, c5, mo[3] * (1.0f / 6.0f)));
+        tab[kTabC4 + sg] = mo[4] * (1.0f / 24.0f);
+      }
+    }
+    __syncwarp();
   }
+}
+
+// Exact-position residual of fadd(off, fmul(i, ps)): off + i ps minus that
+// rounded value (error of the product by FMA, of the sum by two-sum).
+__device__ __forceinline__ float position_residual(float off, float i, float ps, float pos) {
+  const float p = fmul_x(i, ps), e = __fmaf_rn(i, ps, -p);
+  const float bb = fsub_x(pos, off);
+  return fadd_x(fadd_x(fsub_x(off, fsub_x(pos, bb)), fsub_x(p, bb)), e);
 }
 
 // A pixel inside the clamp region (s < 1/16): of the n planes, K pass the
@@ -918,14 +927,6 @@ __device__ __noinline__ float clamp_value(const float* __restrict__ tab, const f
 // barriers (30.2 us); tables staged in shared memory cost occupancy and more
 // L2 traffic (34.8 us).
 constexpr int kSepChunk = 128;  // candidates staged at a time
-
-// Exact-position residual of fadd(off, fmul(i, ps)): off + i ps minus that
-// rounded value (error of the product by FMA, of the sum by two-sum).
-__device__ __forceinline__ float position_residual(float off, float i, float ps, float pos) {
-  const float p = fmul_x(i, ps), e = __fmaf_rn(i, ps, -p);
-  const float bb = fsub_x(pos, off);
-  return fadd_x(fadd_x(fsub_x(off, fsub_x(pos, bb)), fsub_x(p, bb)), e);
-}
 
 constexpr int kSepThreads = 128;
 constexpr int kSepSegs = 2 * kSepThreads;  // CSR segments at a time
@@ -1273,82 +1274,85 @@ __device__ __forceinline__ float vatom_deriv_f(const float* __restrict__ c, floa
 }
 
 // Adjoint of the separable potential with respect to the atoms' x and y: for
-// the slice's dL/dV field G and V(p) = sum_atoms sum_j exp(-alpha_j rho^2)
-// T_K(p)[j] (the same K, the same exact-position values as k_potential_sep),
-//   dL/dX = 2 sum_p G(p) (px - X) sum_j alpha_j exp(-alpha_j rho^2) T_K[j],
+// the slice's dL/dV field G and V(p) = sum_atoms g(rho^2) (the same planes K and
+// exact-position values as k_potential_sep),
+//   dL/dX = -2 sum_p G(p) (px - X) g'(rho^2),
 // likewise for Y (the cut-off decisions are not differentiated, as in the
-// per-sub-plane adjoint).  Pixels with a sub-plane inside the 0.25 A clamp
-// take the per-sub-plane derivative.  (The forward's piecewise polynomials do
-// not serve here: their rounding, 1e-7, is the same over a whole ring of
-// pixels and the sum over the ring does not average it out: dL/dxy went from
-// 1.7e-6 to 8.7e-6 off FP64 with derivative segments.)  blockIdx.x: the atom of the window (its
-// table row), blockIdx.y: one of gridDim.y interleaved row sets of its
-// +-2.3 A pixel square; FP64 block sums, added atomically in input order.
-__global__ void __launch_bounds__(kPotThreads) k_potential_sep_adjoint(PotArgs a, const float* __restrict__ G,
+// per-sub-plane adjoint).  g' comes from the atom's derivative segments
+// (k_atom_tables<true>).  Pixels with a sub-plane inside the 0.25 A clamp
+// sum the per-sub-plane derivative instead: at the edge of its range the
+// Gaussian expansion's derivative is only good to about 1e-5 (dL/dxy 8.7e-6 off
+// FP64 with it, 1.3e-6 with the direct sum).  blockIdx.x: the atom of the
+// window (its table row), blockIdx.y: one of gridDim.y interleaved row sets of
+// its +-2.3 A pixel square, a row per warp; FP64 block sums, added atomically
+// in input order.
+// Bound: issue, about 45 instructions per pixel; with the 12 exponentials and
+// the gathered row of T_K per pixel, and integer divisions to find the pixel,
+// a slice of 280 atoms on 151^2 pixels each took 28 us.
+constexpr int kAdjThreads = 256;
+__global__ void __launch_bounds__(kAdjThreads) k_potential_sep_adjoint(PotArgs a, const float* __restrict__ G,
                                                                        const int* __restrict__ perm, int a0,
                                                                        double* __restrict__ dxy) {
-  __shared__ float s_asc[32];
-  __shared__ float s_qv[20];
-  __shared__ __align__(16) float s_al[kGaussJ];
-  __shared__ double s_red[2][kPotThreads / 32];
-  constexpr float kLn2 = 0.6931471805599453f;
+  __shared__ double s_red[2][kAdjThreads / 32];
   const int l = a0 + blockIdx.x;
   const float4 at = a.atoms[l];
   const float* tab = a.tab + (size_t)blockIdx.x * kTabStride;
-  const float* cz = a.coef + (__float_as_int(at.w) - 1) * kCoefPerZ;
   const float4 hd = __ldg(reinterpret_cast<const float4*>(tab + kTabHead));
   const int n = __float_as_int(hd.w);
-  if (threadIdx.x < 32) s_asc[threadIdx.x] = threadIdx.x < 24 ? tab[kTabAsc + threadIdx.x] : 1e30f;
-  if (threadIdx.x < 20) s_qv[threadIdx.x] = tab[kTabQV + threadIdx.x];
-  if (threadIdx.x < kGaussJ) s_al[threadIdx.x] = a.gauss[(__float_as_int(at.w) - 1) * 2 * kGaussJ + threadIdx.x];
-  __syncthreads();
+  if (n == 0) return;  // (no sub-plane of the slice within reach)
+  const float* cz = a.coef + (__float_as_int(at.w) - 1) * kCoefPerZ;
+  const float4* bins = reinterpret_cast<const float4*>(tab + kTabBin) - (kRadBin0 - 1);
+  const float4* seg = reinterpret_cast<const float4*>(tab + kTabSeg);
   const int xl = max((int)floorf((at.x - 2.3f - a.xoff) / a.ps), 0);
   const int xh = min((int)ceilf((at.x + 2.3f - a.xoff) / a.ps), a.nx - 1);
   const int yl = max((int)floorf((at.y - 2.3f - a.yoff) / a.ps), 0);
   const int yh = min((int)ceilf((at.y + 2.3f - a.yoff) / a.ps), a.ny - 1);
-  const int wx = xh - xl + 1, wy = yh - yl + 1;
-  const int ns = gridDim.y, js = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ns = gridDim.y;
   float gx = 0.0f, gy = 0.0f;
-  if (wx > 0 && wy > js) {
-    const int npx = wx * ((wy - js + ns - 1) / ns);
-    for (int w = threadIdx.x; w < npx; w += kPotThreads) {
-      const int x = xl + w % wx, y = yl + js + (w / wx) * ns;
+  for (int y = yl + (int)blockIdx.y + ns * warp; y <= yh; y += ns * (kAdjThreads / 32)) {
+    const float py = fadd_x(a.yoff, fmul_x((float)y, a.ps));
+    const float dy = fsub_x(py, at.y), dy2 = fmul_x(dy, dy);
+    if (!(dy2 < 5.0f)) continue;
+    const float dyv = dy + position_residual(a.yoff, (float)y, a.ps, py);
+    const float yv = fmaf(dyv, dyv, hd.y);
+    const float* g = G + (long long)y * a.nx;
+#pragma unroll 2
+    for (int x = xl + lane; x <= xh; x += 32) {
       const float px = fadd_x(a.xoff, fmul_x((float)x, a.ps));
-      const float py = fadd_x(a.yoff, fmul_x((float)y, a.ps));
-      const float dx = fsub_x(px, at.x), dy = fsub_x(py, at.y);
-      const float dxy2 = fadd_x(fmul_x(dx, dx), fmul_x(dy, dy));
-      int c = 0;  // thresholds passed: K = n - c planes remain
-#pragma unroll
-      for (int st = 16; st >= 1; st >>= 1)
-        if (dxy2 >= s_asc[c + st - 1]) c += st;
-      const int K = n - c;
-      if (K <= 0) continue;
-      const float dxv = dx + (float)(((double)a.xoff + (double)x * (double)a.ps) - (double)px);
-      const float dyv = dy + (float)(((double)a.yoff + (double)y * (double)a.ps) - (double)py);
-      const float dxyv = fmaf(dxv, dxv, dyv * dyv);
-      const float gp = G[(long long)y * a.nx + x];
+      const float dx = fsub_x(px, at.x);
+      const float rho = fadd_x(fmul_x(dx, dx), dy2);
+      const float s = fadd_x(rho, hd.x);
+      if (!(s < 5.0f)) continue;
+      const float dxv = dx + position_residual(a.xoff, (float)x, a.ps, px);
+      const float sv = fmaf(dxv, dxv, yv);
+      const float sc = fmaxf(s, 0.061f);  // (bin -1: the clamp region)
+      const float4 e = __ldg(bins + (__float_as_int(sc) >> 19));
+      int sg = __float_as_int(e.w) + (rho >= e.x) + (rho >= e.y) + (rho >= e.z);
       float D;  // d/d(rho^2) of the atom's value at this pixel
-      if (dxy2 + hd.x < 0.0627f) {
+      // (a margin over 1/16: the clamp itself is decided on the exact r^2)
+      if (s < 0.0627f) {
+        const float rv = sv - hd.y;
+        int c = 0;
+        while (c < n && rho >= __ldg(tab + kTabAsc + c)) ++c;
         D = 0.0f;
-        for (int k = 0; k < K; ++k) D += vatom_deriv_f(cz, dxyv + s_qv[k]);
+        for (int k = 0; k < n - c; ++k) D += vatom_deriv_f(cz, rv + __ldg(tab + kTabQV + k));
         D *= a.wsub;
       } else {
-        const float4* T = reinterpret_cast<const float4*>(tab + kTabT + (K - 1) * kGaussJ);
-        const float sv = dxyv + hd.y;  // (the rows T are relative to the nearest plane)
-        float e0 = 0.0f, e1 = 0.0f;
-#pragma unroll
-        for (int g = 0; g < kGaussJ / 4; ++g) {
-          const float4 al = *reinterpret_cast<const float4*>(&s_al[4 * g]);
-          const float4 tt = __ldg(T + g);
-          e0 = fmaf(al.x * ex2_fast(-al.x * sv), tt.x, e0);
-          e1 = fmaf(al.y * ex2_fast(-al.y * sv), tt.y, e1);
-          e0 = fmaf(al.z * ex2_fast(-al.z * sv), tt.z, e0);
-          e1 = fmaf(al.w * ex2_fast(-al.w * sv), tt.w, e1);
+        if (sg & kRadMore) {  // more than three thresholds in the bin
+          sg -= kRadMore;
+          int c = sg - (rad_bin(s) - __float_as_int(hd.z));
+          while (rho >= __ldg(tab + kTabAsc + c)) ++c, ++sg;
         }
-        D = -kLn2 * (e0 + e1);  // (s_al holds alpha_j log2(e))
+        const float tau = sv - rad_centre(sc);
+        const float4 p = __ldg(seg + sg);
+        D = fmaf(__ldg(tab + kTabC4 + sg), tau, p.w);
+        D = fmaf(D, tau, p.z);
+        D = fmaf(D, tau, p.y);
+        D = fmaf(D, tau, p.x);
       }
-      gx += gp * D * dxv;
-      gy += gp * D * dyv;
+      const float gD = __ldg(g + x) * D;
+      gx = fmaf(gD, dxv, gx);
+      gy = fmaf(gD, dyv, gy);
     }
   }
   double sx = gx, sy = gy;
@@ -1357,15 +1361,14 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_sep_adjoint(PotArgs a
     sx += __shfl_down_sync(0xffffffffu, sx, o);
     sy += __shfl_down_sync(0xffffffffu, sy, o);
   }
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     s_red[0][warp] = sx;
     s_red[1][warp] = sy;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double tx = 0.0, ty = 0.0;
-    for (int k = 0; k < kPotThreads / 32; ++k) {
+    for (int k = 0; k < kAdjThreads / 32; ++k) {
       tx += s_red[0][k];
       ty += s_red[1][k];
     }
@@ -1384,9 +1387,8 @@ cudaError_t launch_potential_adjoint(const PotArgs& a, const float* G, const int
   const int na = a1 - a0;
   const int ns = std::min(16, std::max(1, (8 * 148 + na - 1) / na));
   if (separable) {
-    // the slice's per-atom tables (a0 is the window's first atom, as there)
-    if (cudaError_t e = launch_atom_tables(sep_args(a, na), s, false)) return e;
-    k_potential_sep_adjoint<<<dim3(na, ns), kPotThreads, 0, s>>>(a, G, perm, a0, dxy);
+    if (!a.tab) return cudaErrorInvalidValue;
+    k_potential_sep_adjoint<<<dim3(na, ns), kAdjThreads, 0, s>>>(a, G, perm, a0, dxy);
     return cudaGetLastError();
   }
   k_potential_conv_adjoint<<<dim3(na, ns), kPotThreads, 0, s>>>(a, G, perm, a0, dxy);
@@ -1430,20 +1432,20 @@ cudaError_t build_atom_index(const int* dZ, const float* dx, const float* dy, co
 int potential_tiles() { return 3; }
 int potential_tiles_separable() { return 4; }
 
-template <bool SEGS, int LPA>
+template <bool DERIV, int LPA>
 static void run_atom_tables(const SepArgs& a, cudaStream_t s) {
   constexpr int NA = kTabThreads / LPA;
   const int ctas = (int)std::min<long long>(((long long)a.rows + NA - 1) / NA, 65535);
-  k_atom_tables<SEGS, LPA><<<dim3(ctas, a.nb, a.ns), kTabThreads, 0, s>>>(a);
+  k_atom_tables<DERIV, LPA><<<dim3(ctas, a.nb, a.ns), kTabThreads, 0, s>>>(a);
 }
 
 // Lanes per atom: 32 while every atom's warp is resident at once (a launch of
 // few atoms is one pass through the chain of dependent steps), else 16.
-cudaError_t launch_atom_tables(const SepArgs& a, cudaStream_t s, bool segments) {
+cudaError_t launch_atom_tables(const SepArgs& a, cudaStream_t s, bool derivative) {
   if (!a.p.tab || !a.p.gauss || !a.p.gbin || a.rows < 1 || a.nb < 1 || a.nb > 65535 || a.ns < 1 || a.ns > kSepGroup)
     return cudaErrorInvalidValue;
   const bool few = (long long)a.rows * a.nb * a.ns <= 148 * 16;
-  if (segments)
+  if (derivative)
     few ? run_atom_tables<true, 32>(a, s) : run_atom_tables<true, 16>(a, s);
   else
     few ? run_atom_tables<false, 32>(a, s) : run_atom_tables<false, 16>(a, s);

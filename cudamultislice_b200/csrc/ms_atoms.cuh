@@ -145,17 +145,18 @@ cudaError_t launch_potential(const PotArgs& a, int kind, cudaStream_t s, int til
 int potential_tiles();
 int potential_tiles_separable();
 // The separable conventional kernel's two launches: the per-atom tables of the
-// slices into a.p.tab, then the potentials from them.  tile: 0..3 = 16 x 16,
+// slices into a.p.tab (derivative: dG/d(rho^2) for the position adjoint), then
+// the potentials from them.  tile: 0..3 = 16 x 16,
 // 16 x 32, 32 x 16, 32 x 32 pixels (two, four, four and eight per thread), -1 =
 // by grid and pixel size.
-cudaError_t launch_atom_tables(const SepArgs& a, cudaStream_t s, bool segments = true);
+cudaError_t launch_atom_tables(const SepArgs& a, cudaStream_t s, bool derivative = false);
 cudaError_t launch_potential_from_tables(const SepArgs& a, cudaStream_t s, int tile);
 
 // Adjoint of the conventional potential of one slice with respect to atom x, y:
 // dxy[2 perm[l] + {0,1}] += dL/d{x,y} of sorted atoms l in [a0, a1) (the CSR
 // range of the slice's z-window), G = dL/dV of the slice [ny][nx].
-// separable: through the per-atom tables of the separable kernel (a.tab,
-// a.gauss set; a0 must be the first atom of the slice's z-window).
+// separable: through the derivative tables of the slice's atoms in a.tab (a0
+// must be the first atom of the slice's z-window, as there).
 cudaError_t launch_potential_adjoint(const PotArgs& a, const float* G, const int* perm, int a0, int a1, double* dxy,
                                      cudaStream_t s, bool separable = false);
 

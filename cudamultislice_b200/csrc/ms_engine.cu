@@ -2199,7 +2199,6 @@ class Engine {
       MS_TRY(d_dV_.resize(dLdV ? N * S : 2 * N));
       if (dLdxy) {
         MS_TRY(d_dxy_.resize(2 * (size_t)natoms_));
-        if (int rc = ensure_tables(window_atoms(hzoff_, nzb_, 1))) return rc;
       }
     }
     invalidate_graph();  // the sweep below leaves d_psi_ at psi_S
@@ -2260,6 +2259,15 @@ class Engine {
       }
     }
     if (grad) {
+      // position adjoint: the derivative tables of adj_gs slices at a time
+      // (one launch per group; a launch per slice was half of its time on
+      // small windows), those of slices adj_lo and up in place
+      const bool sep = dLdxy && separable_ok();
+      const size_t rows = sep ? window_atoms(hzoff_, nzb_, 1) : 1, per = rows * kTabStride;
+      const int adj_gs = (int)std::max<size_t>(1, std::min<size_t>(kTabBytes / (per * sizeof(float)), kSepGroup));
+      int adj_lo = S + 1;
+      if (sep)
+        if (int rc = ensure_tables(rows * adj_gs)) return rc;
       for (int c = clast; c >= 0; c -= K) {
         const int e = std::min(c + K, S);
         // psi_c .. psi_{e-1} (real space) into segment slots 0 .. e-1-c
@@ -2302,16 +2310,26 @@ class Engine {
           MS_TRY(pass_a(a, A_INV | A_ADJ | A_FWD | A_BI | A_BO, 1));
           launches += 2;
           if (dLdxy) {
-            const PotArgs pa = pot_args(POT_CONVENTIONAL, n, nullptr);
+            PotArgs pa = pot_args(POT_CONVENTIONAL, n, nullptr);
             const int a0 = hzoff_[pa.kt], a1 = hzoff_[pa.kb + 1];
-            const bool sep = separable_ok();
+            if (sep && n < adj_lo) {
+              // (after the adjoints that read the buffer: the same stream)
+              adj_lo = std::max(1, n - adj_gs + 1);
+              SepArgs ta = sep_args(pot_args(POT_CONVENTIONAL, adj_lo, nullptr), (int)rows);
+              ta.ns = n - adj_lo + 1;
+              for (int i = 1; i < ta.ns; ++i) ta.set_slice(i, pot_args(POT_CONVENTIONAL, adj_lo + i, nullptr));
+              ta.s_tab = (long long)per;
+              MS_TRY(launch_atom_tables(ta, pix_[1], true));
+              ++launches;
+            }
+            if (sep) pa.tab = d_tab_.p + (size_t)(n - adj_lo) * per;
             // on a second stream: the next slices' adjoint passes do not wait
             // for it (it reads dV and adds into dL/dxy only)
             MS_TRY(cudaEventRecord(ev_dv_, stream_));
             MS_TRY(cudaStreamWaitEvent(pix_[1], ev_dv_, 0));
             MS_TRY(launch_potential_adjoint(pa, dV, d_idx_.p, a0, a1, d_dxy_.p, pix_[1], sep));
             MS_TRY(cudaEventRecord(ev_adj_[n & 1], pix_[1]));
-            launches += sep ? 2 : 1;
+            ++launches;
           }
         }
       }
