@@ -21,17 +21,19 @@ __device__ __forceinline__ float2 ctf_weight(double lam, double Cs, double df, d
   const double kx = kxf, ky = kyf, k2 = kx * kx + ky * ky, k = sqrt(k2);
   const double factor = beta * beta / (4.0 * lam * lam);
   const double a1 = 3.141593 * k * lam * 2.0 * df + 2.0 * 3.141593 * lam * lam * lam * Cs * k2 * k;
-  const double es = exp(-factor * a1 * a1);
-  const double ed = exp(-0.25 * delta * delta * 3.141593 * 3.141593 * k2 * k2 * lam * lam);
-  const double phi = atan2(ky, kx);
-  const double chi = 3.1415926 * lam * k2 *
-                     (0.5 * Cs * lam * lam * k2 + df + A2 * sin(2.0 * (phi - phi2)) +
-                      2.0 * A3 * lam * sqrt(k2) * sin(3.0 * (phi - phi3)) / 3.0);
+  // (both envelopes in one exponential)
+  const double env = exp(-factor * a1 * a1 - 0.25 * delta * delta * 3.141593 * 3.141593 * k2 * k2 * lam * lam);
+  double defocus = df;
+  if (A2 != 0.0 || A3 != 0.0) {  // astigmatism: the azimuth is needed (uniform over the launch)
+    const double phi = atan2(ky, kx);
+    defocus += A2 * sin(2.0 * (phi - phi2)) + 2.0 * A3 * lam * k * sin(3.0 * (phi - phi3)) / 3.0;
+  }
+  const double chi = 3.1415926 * lam * k2 * (0.5 * Cs * lam * lam * k2 + defocus);
   const double twopi = 6.283185307179586;
   const float chr = (float)(chi - twopi * rint(chi / twopi));
   float s, c;
   sincosf(chr, &s, &c);
-  const float amp = (float)(es * ed) * scale;
+  const float amp = (float)env * scale;
   return make_float2(amp * c, -amp * s);
 }
 

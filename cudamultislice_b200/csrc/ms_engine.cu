@@ -248,7 +248,7 @@ class Engine {
         ckpt_ = value;
         return MS_OK;
       case MS_OPT_FFT_PLAN:
-        if (value < -1 || value >= plan_variants()) return fail(MS_ERR_INVALID, "FFT plan must be -1 (tuned) or a variant index");
+        if (value < -1 || value >= plan_variants()) return fail(MS_ERR_INVALID, "FFT plan must be -1 (by size) or a variant index");
         forced_plan_ = value;
         invalidate_graph();
         return MS_OK;
@@ -581,7 +581,6 @@ class Engine {
     if (cufftSetStream(plan_, stream_) != CUFFT_SUCCESS) return fail(MS_ERR_CUDA, "cufftSetStream failed");
     have_plan_ = true;
     fused_ok_ = fused_supported(nx, ny);
-    tuned_.clear();
     raster_batch_.clear();
     loop_grid_ = 0;
     if (!pot_tile_forced_) pot_tile_ = -1;
@@ -858,7 +857,6 @@ class Engine {
     const size_t N = (size_t)nx_ * ny_;
     if (use_fused()) {
       if (int rc = ensure_real()) return rc;
-      plan_for(1);  // tune outside the capture
       MS_TRY(d_fdX_.resize(N));
       MS_TRY(d_fdQ_.resize(N));
       MS_TRY(d_fdS_.resize(N));
@@ -1417,7 +1415,6 @@ class Engine {
     }
     rs_n_ = n;
     rs_B_ = std::min(batch, n);
-    plan_for(rs_B_, true);
     MS_TRY(d_bwave_.resize((size_t)rs_B_ * N));
     MS_TRY(d_bpos_.resize(2 * (size_t)n));
     MS_TRY(d_bsig_.resize(2 * (size_t)n));
@@ -1731,7 +1728,6 @@ class Engine {
     if (fused) {
       MS_TRY(d_fpstack_.resize((size_t)B * S * N));
       MS_TRY(d_bwave_.resize((size_t)B * N));
-      plan_for(B);
     }
     invalidate_graph();
     bool fp_loop = false;
@@ -1878,7 +1874,6 @@ class Engine {
   int run_conventional_streamed(int S, int* nslices) {
     if (int rc = require_potential_inputs()) return rc;
     if (int rc = ensure_prop_tables(convdz_)) return rc;
-    plan_for(1);  // (tuning synchronises: before the streams fork)
     const size_t N = (size_t)nx_ * ny_;
     MS_TRY(d_stack_.resize(N * S));
     MS_TRY(cudaEventRecord(ev0_, stream_));
@@ -1923,11 +1918,8 @@ class Engine {
     if (int rc = ensure_prop_tables(convdz_)) return rc;
     const bool loop = use_loop();
     if (use_fused()) {
-      if (loop) {
+      if (loop)
         if (int rc = prepare_loop()) return rc;
-      } else {
-        plan_for(1);  // tune outside the capture (tuning allocates and synchronises)
-      }
       if (!graph_exec_ || graph_S_ != S || graph_stack_ != d_stack_.p) {
         invalidate_graph();
         MS_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -2182,10 +2174,13 @@ class Engine {
     if (dLdxy && pot_mode_ != 0)
       return fail(MS_ERR_UNSUPPORTED, "atom gradients need the conventional potential (MS_OPT_POTENTIAL 0)");
     if (int rc = ensure_prop_tables(convdz_)) return rc;
-    plan_for(1);
     const size_t N = (size_t)nx_ * ny_;
     int K = S;
     if (grad) K = ckpt_ > 0 ? std::min(ckpt_, S) : auto_checkpoint_stride(S, (size_t)nx_ * ny_);
+    // (every wave stored is one segment that the forward sweep saves in real
+    // space as it passes: the same S waves of memory, without a copy and an
+    // inverse row pass per slice)
+    if (K == 1) K = S;
     const int nck = (S + K - 1) / K;
     MS_TRY(d_T_.resize(N * nd));
     MS_TRY(d_Phi_.resize(N));
@@ -2674,116 +2669,16 @@ class Engine {
   }
 
   // FFT plan variants of the row and column passes for a batch size: forced
-  // by MS_OPT_FFT_PLAN, else the autotuned choice (timed once per batch size).
+  // by MS_OPT_FFT_PLAN, else by line length and line count (pass_plan).
+  // `tc`: the row pass multiplies by a precomputed transmission (A_MULT_TC,
+  // the batched raster) rather than forming exp(i sigma V) itself.
   struct PlanChoice {
     int row = 0, col = 0;
   };
-  // `tc`: the row pass multiplies by a precomputed transmission (A_MULT_TC,
-  // the batched raster) rather than forming exp(i sigma V) itself; the two
-  // load different operands and are tuned apart.
-  PlanChoice plan_for(int batch, bool tc = false) {
+  PlanChoice plan_for(int batch, bool tc = false) const {
     if (forced_plan_ >= 0) return PlanChoice{forced_plan_, forced_plan_};
-    const int bucket = batch <= 1 ? 1 : batch < 8 ? 4 : batch < 32 ? 16 : 64;
-    const int key = bucket + (tc ? 1000 : 0);
-    for (auto& kv : tuned_)
-      if (kv.first == key) return kv.second;
-    PlanChoice c = autotune(bucket, tc);
-    tuned_.push_back({key, c});
-    return c;
-  }
-
-  // Times every plan variant of the steady-state row pass and the propagating
-  // column pass on scratch waves (batch instances), on this device, then the
-  // three fastest of each in pairs, alternating, and keeps the fastest pair.
-  // Scratch is zero-filled so the transmission's sincos stays on its fast
-  // path.  On any launch failure the variant is skipped.
-  PlanChoice autotune(int batch, bool tc) {
-    PlanChoice best;
-    const long long N = (long long)nx_ * ny_;
-    DevBuf<float2> w, T;
-    DevBuf<float> V;
-    if (w.resize((size_t)batch * N) != cudaSuccess || V.resize((size_t)N) != cudaSuccess) return best;
-    if (tc && T.resize((size_t)N) != cudaSuccess) return best;
-    cudaMemsetAsync(w.p, 0, sizeof(float2) * batch * N, stream_);
-    cudaMemsetAsync(V.p, 0, sizeof(float) * N, stream_);
-    if (tc) cudaMemsetAsync(T.p, 0, sizeof(float2) * N, stream_);
-    const int row_op = (tc ? (A_INV | A_MULT_TC | A_FWD) : (A_INV | A_MULT_T | A_FWD)) | A_BI | A_BO;
-    if (ensure_prop_tables(convdz_) != MS_OK) return best;
-    const int reps = 8, nv = plan_variants();
-    auto row_args = [&](int v) {
-      PassAArgs a = passa_args(w.p, w.p, v);
-      a.V = V.p;
-      a.tr = T.p;
-      a.batch_stride_wave = N;
-      a.batch_stride_V = 0;
-      return a;
-    };
-    auto col_args = [&](int v) {
-      PassBArgs b = passb_args(w.p, w.p, v);
-      b.batch_stride_wave = N;
-      return b;
-    };
-    auto elapsed = [&](auto&& body) {
-      float ms = INFINITY;
-      cudaEventRecord(ev0_, stream_);
-      body();
-      cudaEventRecord(ev1_, stream_);
-      if (cudaEventSynchronize(ev1_) != cudaSuccess || cudaEventElapsedTime(&ms, ev0_, ev1_) != cudaSuccess) {
-        cudaGetLastError();
-        return INFINITY;
-      }
-      return ms;
-    };
-    // each variant of each pass alone
-    std::vector<float> ta(nv, INFINITY), tb(nv, INFINITY);
-    for (int v = 0; v < nv; ++v) {
-      const PassAArgs a = row_args(v);
-      const PassBArgs b = col_args(v);
-      bool ok = true;
-      for (int k = 0; k < 2 && ok; ++k)  // first launches load the kernels
-        ok = launch_pass_a(a, v, row_op, batch, stream_) == cudaSuccess &&
-             launch_pass_b(b, v, B_PROPAGATE, batch, stream_) == cudaSuccess;
-      if (!ok || cudaStreamSynchronize(stream_) != cudaSuccess) {
-        cudaGetLastError();
-        continue;
-      }
-      ta[v] = elapsed([&] { for (int k = 0; k < reps; ++k) launch_pass_a(a, v, row_op, batch, stream_); });
-      tb[v] = elapsed([&] { for (int k = 0; k < reps; ++k) launch_pass_b(b, v, B_PROPAGATE, batch, stream_); });
-      launches += 2LL * (reps + 2);
-    }
-    // the three fastest of each, paired and timed alternating as the slice
-    // loop runs them (a pass's speed depends on its neighbour: programmatic
-    // dependent launch lets the next pass's CTAs in while this one drains)
-    auto top3 = [&](const std::vector<float>& t) {
-      std::vector<int> idx(nv);
-      for (int v = 0; v < nv; ++v) idx[v] = v;
-      std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return t[x] < t[y]; });
-      idx.resize(std::min(nv, 3));
-      return idx;
-    };
-    float best_t = INFINITY;
-    for (int r : top3(ta)) {
-      if (!(ta[r] < INFINITY)) continue;
-      for (int c : top3(tb)) {
-        if (!(tb[c] < INFINITY)) continue;
-        const PassAArgs a = row_args(r);
-        const PassBArgs b = col_args(c);
-        const float t = elapsed([&] {
-          for (int k = 0; k < reps; ++k) {
-            launch_pass_a(a, r, row_op, batch, stream_);
-            launch_pass_b(b, c, B_PROPAGATE, batch, stream_);
-          }
-        });
-        launches += 2LL * reps;
-        if (t < best_t) {
-          best_t = t;
-          best.row = r;
-          best.col = c;
-        }
-      }
-    }
-    cudaStreamSynchronize(stream_);
-    return best;
+    return PlanChoice{pass_plan(nx_, (long long)ny_ * batch, false, tc),
+                      pass_plan(ny_, (long long)nx_ * batch, true, tc)};
   }
 
   PassAArgs passa_args(const float2* in, float2* out, int variant) {
@@ -2811,7 +2706,7 @@ class Engine {
     MS_TRY(cudaMemsetAsync(d_pass_err_.p, 0, sizeof(int), stream_));
     return fail(MS_ERR_CUDA, "a column pass's tensor-copy wait ran out (bounded at one second)");
   }
-  // Row / column pass launchers with the plan tuned for `batch` instances.
+  // Row / column pass launchers with the plan for `batch` instances.
   cudaError_t pass_a(PassAArgs a, int flags, int batch = 1, cudaStream_t s = nullptr) {
     const int v = plan_for(batch).row;
     a.tw = d_twx_[v].p;
@@ -3239,7 +3134,6 @@ class Engine {
   DevBuf<float2> d_ck_, d_seg_, d_G_, d_U_, d_Phi_;
   DevBuf<float> d_T_, d_dV_, d_img_, d_fpstack_, d_fpdiff_, d_fpsum_, d_fpimg_;
   DevBuf<double> d_loss_, d_dxy_;
-  std::vector<std::pair<int, PlanChoice>> tuned_;
   std::vector<std::pair<long long, int>> raster_batch_;  // tuned probes per launch by grid
   float prop_dz_ = -1.0f;
   cufftHandle plan_ = 0;

@@ -134,8 +134,12 @@ float2 unit_fp32(double c, double s);
 
 // Line lengths 64..4096 (powers of two) in both directions.
 bool fused_supported(int nx, int ny);
-// Number of FFT plan variants per line length (autotuned by the engine).
+// Number of FFT plan variants per line length, and the one for passes over
+// `lines` lines of n points (all instances; columns: whole grids, of which the
+// pass may run the band's half).  tc: the row pass reads a precomputed
+// transmission.
 int plan_variants();
+int pass_plan(int n, long long lines, bool columns, bool tc);
 // Twiddle table of plan `variant` for lines of n points into host_out
 // (at most 2n entries); returns its length.
 int make_twiddles(int n, int variant, float2* host_out);

@@ -12,7 +12,7 @@
 
 namespace ms {
 
-// FFT plan variants per line length (chosen at run time by the autotuner):
+// FFT plan variants per line length (chosen by pass_plan):
 // variant 0 keeps the most points per thread (fewest exchanges), higher
 // variants spread a line over more threads (more warps in flight); variants
 // 3..5 are 0..2 with the butterflies on the packed FP32x2 pipe.
@@ -77,7 +77,7 @@ __host__ __device__ constexpr int rows_per_cta() {
 // The packed 32-point column plans take half the columns per CTA: twice the
 // CTAs, which a single instance (one wave) needs, and registers enough for
 // two CTAs without spilling; their unpacked twins keep the wide tiles that
-// win in batches (the autotuner chooses per batch).
+// win in batches (pass_plan chooses per batch).
 template <class PL>
 __host__ __device__ constexpr bool narrow_cols() { return PL::PK && PL::E >= 32; }
 template <class PL>
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(cols_per_cta<PL>() * PL::P, col_min_ctas<PL>()
 // (The column pass, k_pass_b above, sizes every plan by col_min_ctas.)
 // Row CTAs per SM a capped row plan is sized for (0: left to the compiler).
 // Fewer registers cost latency hiding at one instance while more CTAs win in
-// batches, so plan shapes keep a free and a capped twin and the autotuner
+// batches, so plan shapes keep a free and a capped twin and pass_plan
 // chooses: the unpacked 32-point plan is sized for two CTAs (a bound only for
 // its 256-thread CTAs, lines of 128 threads), the packed 16-point plan for
 // three; their twins stay free.

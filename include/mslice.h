@@ -60,9 +60,8 @@ enum {
                                reference kernel binnedAtomPKernel3 (U.cu:582-653);
                                1 = projected potential vzatom2 per slab (U.cu:119-152,
                                xy scan of binnedAtomPKernel2 U.cu:513-578) */
-  MS_OPT_FFT_PLAN = 3,      /* -1 = autotuned (default): every FFT plan variant of the
-                               fused passes is timed on the device once per grid and
-                               batch size and the fastest kept; 0..5 = force a variant
+  MS_OPT_FFT_PLAN = 3,      /* -1 = by line length and batch size (default, from measured
+                               times); 0..5 = force an FFT plan variant of the fused passes
                                (0: most points per thread ... 2: most threads per line;
                                3..5: 0..2 with butterflies on the packed FP32x2 pipe).
                                Variants agree to FP32 rounding, not bit for bit. */
@@ -380,8 +379,8 @@ ms_status ms_fft2(ms_sim* sim, const float* in, float* out, int nx, int ny, int 
  * second run of `steps` steps with an event between every pass. */
 ms_status ms_time_slices(ms_sim* sim, int steps, int reps, float* ms_total, float* ms_row_pass,
                          float* ms_col_pass);
-/* FFT plan variants (row pass, column pass) used for `batch` instances, tuning
- * them first if needed (MS_OPT_FFT_PLAN). */
+/* FFT plan variants (row pass, column pass) used for `batch` instances
+ * (MS_OPT_FFT_PLAN). */
 ms_status ms_get_fft_plan(ms_sim* sim, int batch, int* row_variant, int* col_variant);
 /* The last raster's probes per launch and whether its slices ran in the
  * batched persistent loop (1) or per pass (0); with batch <= 0 both are the
