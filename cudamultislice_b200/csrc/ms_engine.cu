@@ -29,6 +29,7 @@
 
 #include "../../include/mslice.h"
 #include "ms_atoms.cuh"
+#include "ms_general.cuh"
 #include "ms_philox.h"
 #include "ms_tiff.h"
 #include "ms_pointwise.cuh"
@@ -581,6 +582,7 @@ class Engine {
     if (cufftSetStream(plan_, stream_) != CUFFT_SUCCESS) return fail(MS_ERR_CUDA, "cufftSetStream failed");
     have_plan_ = true;
     fused_ok_ = fused_supported(nx, ny);
+    if (int rc = prepare_general()) return rc;
     raster_batch_.clear();
     loop_grid_ = 0;
     if (!pot_tile_forced_) pot_tile_ = -1;
@@ -1879,11 +1881,15 @@ class Engine {
     MS_TRY(cudaEventRecord(ev0_, stream_));
     MS_TRY(cudaEventRecord(ev_fork2_, stream_));
     MS_TRY(cudaStreamWaitEvent(pass_, ev_fork2_, 0));
+    const bool general = !use_fused();
     int rc = separable_stack(S, d_stack_.p, N, 1, nullptr, nullptr, 0, 0, [&](int it, cudaEvent_t done) -> int {
       MS_TRY(cudaStreamWaitEvent(pass_, done, 0));
+      const float* V = d_stack_.p + (size_t)(it - 1) * N;
+      if (general) return enqueue_general_step(V, it == 1 ? d_psi0_.p : nullptr, pass_);
       launches += 2;
-      return enqueue_fused_step(d_stack_.p + (size_t)(it - 1) * N, it == 1, pass_);
+      return enqueue_fused_step(V, it == 1, pass_);
     });
+    if (rc == MS_OK && general) rc = finish_general(pass_);
     // join the pass stream (also on failure, so that the handle's stream
     // orders after everything enqueued)
     MS_TRY(cudaEventRecord(ev_join_, pass_));
@@ -1896,7 +1902,7 @@ class Engine {
     nstack_ = S;
     stack_valid_ = true;
     tstack_valid_ = false;
-    domain_ = 1;
+    domain_ = general ? 0 : 1;
     if (nslices) *nslices = S;
     return MS_OK;
   }
@@ -1904,7 +1910,7 @@ class Engine {
   int run_conventional(int* nslices) {
     if (!have_waves_) return fail(MS_ERR_STATE, "wavefunctions not initialised");
     int S = 0;
-    if (use_fused() && pot_mode_ == 0 && overlap_build_ && have_index_ && have_fp_ && have_freq_) {
+    if ((use_fused() || use_general()) && pot_mode_ == 0 && overlap_build_ && have_index_ && have_fp_ && have_freq_) {
       if (int rc = get_slices(true, &S)) return rc;
       // 256^2 and 512^2 with the persistent loop: build first, then the loop in
       // one launch (two pass launches a slice bound those runs on the host:
@@ -1956,6 +1962,13 @@ class Engine {
       MS_TRY(cudaGraphLaunch(graph_exec_, stream_));
       launches += loop ? 1 : 2LL * S;
       domain_ = 1;
+    } else if (use_general()) {
+      MS_TRY(cudaEventRecord(ev0_, stream_));
+      for (int it = 1; it <= S; ++it)
+        if (int rc = enqueue_general_step(d_stack_.p + (size_t)(it - 1) * nx_ * ny_, it == 1 ? d_psi0_.p : nullptr,
+                                          stream_))
+          return rc;
+      if (int rc = finish_general(stream_)) return rc;
     } else {
       MS_TRY(cudaEventRecord(ev0_, stream_));
       for (int it = 1; it <= S; ++it)
@@ -2638,6 +2651,83 @@ class Engine {
     return MS_OK;
   }
 
+  // Plans, twiddles and band of the mixed-radix passes, for grids that the
+  // fused passes do not take and whose lengths they provide (general_plan).
+  int prepare_general() {
+    gen_ok_ = false;
+    gen_row_ = gen_col_ = GenPlan{};
+    if (fused_ok_) return MS_OK;
+    gen_row_ = general_plan(nx_);
+    gen_col_ = general_plan(ny_);
+    if (gen_row_.npass == 0 || gen_col_.npass == 0) return MS_OK;
+    float k2_lt, k2_le;
+    band_limit_thresholds(kmax_, &k2_lt, &k2_le);
+    // indices that pass the band limit on one axis alone: a run from 0 up and
+    // one from the end down
+    auto runs = [&](const std::vector<float>& k, int* pos, int* neg) {
+      const int n = (int)k.size();
+      *pos = *neg = 0;
+      while (*pos < n && k[*pos] * k[*pos] < k2_lt) ++*pos;
+      while (*neg < n - *pos && k[n - 1 - *neg] * k[n - 1 - *neg] < k2_lt) ++*neg;
+    };
+    runs(hkx_, &gen_cpos_, &gen_cneg_);
+    runs(hky_, &gen_rpos_, &gen_rneg_);
+    if (gen_cpos_ < 1 || gen_rpos_ < 1) return MS_OK;  // (nothing inside the band)
+    std::vector<float2> tw((size_t)std::max(nx_, ny_));
+    general_twiddles(nx_, tw.data());
+    MS_TRY(d_twx_[0].resize(nx_));
+    MS_TRY(copy_sync(d_twx_[0].p, tw.data(), sizeof(float2) * nx_, cudaMemcpyHostToDevice));
+    general_twiddles(ny_, tw.data());
+    MS_TRY(d_twy_[0].resize(ny_));
+    MS_TRY(copy_sync(d_twy_[0].p, tw.data(), sizeof(float2) * ny_, cudaMemcpyHostToDevice));
+    gen_ok_ = true;
+    return MS_OK;
+  }
+  // Conventional slices on the mixed-radix passes (the plain path when forced).
+  bool use_general() const { return gen_ok_ && !force_plain_; }
+  GenArgs gen_args(const float2* in, float2* out, bool rows) {
+    GenArgs g{};
+    g.in = in;
+    g.out = out;
+    g.sigma = sigma2_;
+    g.nx = nx_;
+    g.ny = ny_;
+    g.cpos = gen_cpos_;
+    g.cneg = gen_cneg_;
+    g.rpos = gen_rpos_;
+    g.rneg = gen_rneg_;
+    g.tw = rows ? d_twx_[0].p : d_twy_[0].p;
+    g.px = d_px_.p;
+    g.py = d_py_.p;
+    g.kx = d_kx_.p;
+    g.ky = d_ky_.p;
+    float k2_le;
+    band_limit_thresholds(kmax_, &g.k2_lt, &k2_le);
+    const double invN = 1.0 / ((double)nx_ * ny_);
+    g.scale = (float)invN;
+    g.scale_lo = (float)(invN - (double)g.scale);
+    g.plan = rows ? gen_row_ : gen_col_;
+    return g;
+  }
+  // One slice: rows (from the initial wave, from real space, or continuing
+  // from the last slice's band: `chain`), then columns, leaving the band in
+  // d_t1_; finish_general returns it to real space in d_psi_.
+  int enqueue_general_step(const float* V, const float2* real_in, cudaStream_t s) {
+    GenArgs r = gen_args(real_in ? real_in : d_t1_.p, d_t1_.p, true);
+    r.V = V;
+    MS_TRY(launch_general_rows(r, real_in ? (G_MULT | G_FWD) : (G_INV | G_MULT | G_FWD), s));
+    MS_TRY(launch_general_columns(gen_args(d_t1_.p, d_t1_.p, false), s));
+    launches += 2;
+    return MS_OK;
+  }
+  int finish_general(cudaStream_t s) {
+    MS_TRY(launch_general_rows(gen_args(d_t1_.p, d_psi_.p, true), G_INV, s));
+    ++launches;
+    domain_ = 0;
+    fd_state_ = false;
+    return MS_OK;
+  }
+
   // Propagator factors for the fused column pass: P(kx,ky) = px[kx] * py[ky]
   // with px = exp(-i pi dz lambda kx^2) / N and py = exp(-i pi dz lambda ky^2),
   // phases in FP64 (CreatePropsKernel U.cu:399-428 uses pi = 3.14159265).
@@ -2651,7 +2741,8 @@ class Engine {
     for (int i = 0; i < nx_; ++i) {
       const double ph = 3.14159265 * (double)dz * (double)wavel_ * (double)hkx_[i] * (double)hkx_[i];
       const float2 u = unit_fp32(std::cos(ph), -std::sin(ph));
-      px[i] = make_float2(u.x * fN, u.y * fN);
+      // (the mixed-radix passes scale by 1/N themselves: not a power of two)
+      px[i] = gen_ok_ ? u : make_float2(u.x * fN, u.y * fN);
     }
     for (int j = 0; j < ny_; ++j) {
       const double ph = 3.14159265 * (double)dz * (double)wavel_ * (double)hky_[j] * (double)hky_[j];
@@ -2744,8 +2835,12 @@ class Engine {
       launches += 2;
       return MS_OK;
     }
-    // plain path: the reference's launch sequence (U.cu:2101-2122)
     if (int rc = ensure_real()) return rc;
+    if (use_general()) {
+      if (int rc = enqueue_general_step(V, first ? d_psi0_.p : d_psi_.p, stream_)) return rc;
+      return finish_general(stream_);
+    }
+    // plain path: the reference's launch sequence (U.cu:2101-2122)
     fd_state_ = false;
     const Grid2 g{nx_, ny_};
     const float nf = 1.0f / std::sqrt((float)(nx_ * ny_));
@@ -3112,6 +3207,10 @@ class Engine {
   int nx_ = 0, ny_ = 0, nFD_ = 0, lbz_ = 3;
   float ps_ = 0, xoff_ = 0, yoff_ = 0, wavel_ = 0, sigma2_ = 0, dzFD_ = 0, kmax_ = 0, convdz_ = 1.0f;
   bool stem_ = false, have_calc_ = false, have_freq_ = false, fd_stable_ = false, fused_ok_ = false;
+  // mixed-radix passes (grids without the fused ones)
+  bool gen_ok_ = false;
+  GenPlan gen_row_, gen_col_;
+  int gen_cpos_ = 0, gen_cneg_ = 0, gen_rpos_ = 0, gen_rneg_ = 0;
   std::vector<float> hkx_, hky_;
   DevBuf<float> d_kx_, d_ky_;
   DevBuf<float2> d_twx_[6], d_twy_[6], d_px_, d_py_, d_P_;
