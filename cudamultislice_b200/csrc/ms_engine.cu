@@ -758,27 +758,63 @@ class Engine {
       if (int rc = fd_plane_fused(it, d_f_.p)) return rc;
       Vplane = d_f_.p;
     }
-    // coefficients of finiteDifferenceKernel (U.cu:1006-1012), pi = 3.14159
-    const double dz = dzFD_, lam = wavel_, aa = 2.0 * 3.14159 * dz / lam, den = 1.0 + aa * aa;
-    const double rcx = 1.0 / den, rcy = -aa / den;
     PassAArgs a = passa_args(d_fdX_.p, d_fdQ_.p, 0);
+    PassBArgs b = passb_args(d_fdQ_.p, d_fdX_.p, 0);
+    fd_coefficients(a, b);
     a.in2 = d_psim_.p;
     a.out2 = d_psi_.p;
     a.V = Vplane;
-    a.fd_rc = make_float2((float)rcx, (float)rcy);
-    a.fd_ratio = make_float2((float)((1.0 - aa * aa) / den), (float)(-2.0 * aa / den));
-    a.fd_kv = (float)(dz * dz * 4.0 * 3.14159 * (double)sigma2_ / lam);
     MS_TRY(pass_a(a, start ? (A_INV | A_FD | A_FWD | A_BO) : (A_INV | A_FD | A_FWD | A_BI | A_BO), 1));
-    PassBArgs b = passb_args(d_fdQ_.p, d_fdX_.p, 0);
-    b.spec = d_fdS_.p;
-    const double cf = dz * dz * 4.0 * 3.14159 * 3.14159;
-    b.fd_c = make_float2((float)(rcx * cf), (float)(rcy * cf));
-    b.scale = 1.0f / (float)N;
     MS_TRY(pass_b(b, B_FD, 1));
     launches += 2;
     std::swap(d_psim_.p, d_psi_.p);  // psi_n becomes psi_{n-1}
     domain_ = 2;                      // current wave held as X
     if (!capturing_) invalidate_graph();  // a single step leaves the FD run's graph stale too
+    return MS_OK;
+  }
+
+  // Coefficients of finiteDifferenceKernel (U.cu:1006-1012), pi = 3.14159.
+  void fd_coefficients(PassAArgs& a, PassBArgs& b) const {
+    const double dz = dzFD_, lam = wavel_, aa = 2.0 * 3.14159 * dz / lam, den = 1.0 + aa * aa;
+    const double rcx = 1.0 / den, rcy = -aa / den, cf = dz * dz * 4.0 * 3.14159 * 3.14159;
+    a.fd_rc = make_float2((float)rcx, (float)rcy);
+    a.fd_ratio = make_float2((float)((1.0 - aa * aa) / den), (float)(-2.0 * aa / den));
+    a.fd_kv = (float)(dz * dz * 4.0 * 3.14159 * (double)sigma2_ / lam);
+    b.spec = d_fdS_.p;
+    b.fd_c = make_float2((float)(rcx * cf), (float)(rcy * cf));
+    b.scale = 1.0f / (float)((long long)nx_ * ny_);
+  }
+  // All S steps in the persistent FD loop (square 256, 512, 1024 grids unless
+  // MS_OPT_SLICE_LOOP or a forced FFT plan turns it off): the same state as S
+  // single steps leave.
+  int run_fd_loop(int S, int grid) {
+    FdLoopArgs L{};
+    L.a = passa_args(d_psi_.p, d_fdX_.p, fd_loop_plan(nx_, false));
+    L.b = passb_args(d_fdX_.p, d_fdX_.p, fd_loop_plan(nx_, true));
+    fd_coefficients(L.a, L.b);
+    L.psi = d_psi_.p;
+    L.psim = d_psim_.p;
+    L.wave = d_fdX_.p;
+    L.planes = d_fdstack_.p;
+    L.pstride = (long long)nx_ * ny_;
+    L.S = S;
+    L.sync.count = d_loop_sync_.p;
+    L.sync.error = reinterpret_cast<int*>(d_loop_sync_.p + 1);
+    L.sync.limit_ns = loop_limit_ns_;
+    L.sync.expect_extra = loop_extra_;
+    *h_loop_err_ = 0;
+    MS_TRY(cudaMemsetAsync(d_loop_sync_.p, 0, 2 * sizeof(unsigned int), stream_));
+    MS_TRY(cudaEventRecord(ev0_, stream_));
+    MS_TRY(launch_fd_loop(L, grid, stream_));
+    MS_TRY(cudaEventRecord(ev1_, stream_));
+    MS_TRY(cudaMemcpyAsync(h_loop_err_, d_loop_sync_.p + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream_));
+    ++launches;
+    MS_TRY(cudaStreamSynchronize(stream_));
+    if (*h_loop_err_ != 0) return loop_timeout_fail();
+    MS_TRY(cudaEventElapsedTime(&last_device_ms_, ev0_, ev1_));
+    fd_state_ = true;
+    domain_ = 2;
+    drop_conv_graph();  // (single steps may swap the wave buffers from here)
     return MS_OK;
   }
 
@@ -862,6 +898,14 @@ class Engine {
       MS_TRY(d_fdX_.resize(N));
       MS_TRY(d_fdQ_.resize(N));
       MS_TRY(d_fdS_.resize(N));
+      int grid = 0;
+      if (use_loop() && fd_loop_prepare(nx_, &grid) == cudaSuccess) {
+        drop_fd_graph();
+        if (int rc = run_fd_loop(S, grid)) return rc;
+        if (out_steps) *out_steps = S;
+        return MS_OK;
+      }
+      cudaGetLastError();
       if (!fd_graph_ || fd_graph_S_ != S || fd_graph_stack_ != d_fdstack_.p || fd_graph_psi_ != d_psi_.p ||
           fd_graph_psim_ != d_psim_.p) {
         drop_fd_graph();

@@ -166,6 +166,24 @@ struct LoopArgs {
   int S;                // slices
   LoopSync sync;
 };
+// Finite-difference loop on square 256, 512 and 1024 grids.
+struct FdLoopArgs {
+  PassAArgs a;          // rows: twiddles, fd_rc, fd_ratio, fd_kv
+  PassBArgs b;          // columns: twiddles, kx, ky, k2_le, scale 1/N, fd_c; spec receives the last spectrum
+  const float2* psi;    // psi_0, real space
+  float2* psim;         // psi_{-1} in, psi_{S-1} out, real space
+  float2* wave;         // row-frequency state of psi_S out (scratch before)
+  const float* planes;  // band-limited potential planes [S][ny][nx]
+  long long pstride;    // floats between planes
+  int S;
+  LoopSync sync;
+};
+int fd_loop_plan(int n, bool columns);
+// The loop's grid (one CTA per SM); an error where it cannot run (the caller
+// then takes the per-pass form).
+cudaError_t fd_loop_prepare(int n, int* grid);
+cudaError_t launch_fd_loop(const FdLoopArgs& L, int grid, cudaStream_t s);
+
 // Batched persistent loop: B instances of one or two square grid sizes
 // stepped through the same S slices by one cooperative launch.
 struct LoopGroup {

@@ -140,6 +140,75 @@ cudaError_t launch_slice_loop(const LoopArgs& L, int variant, int grid, cudaStre
   }
 }
 
+// ---- finite-difference loop ----
+namespace {
+template <int N>
+struct FdForm {
+  static constexpr bool WIDE = N < 1024;  // (as slice_loop_variant)
+  static constexpr int CW = WIDE ? 2 : 4;
+  using PL = LoopPL<N, false>;
+  using PC = LoopPL<N, WIDE>;
+  using SH = LoopShape<PL, PC, CW>;
+};
+template <int N>
+cudaError_t fd_prepare(int* grid) {
+  using F = FdForm<N>;
+  auto kernel = k_fd_loop<typename F::PL, typename F::PC, F::CW>;
+  static unsigned long long done = 0;
+  if (cudaError_t e = set_smem_once(done, kernel, F::SH::SMEM)) return e;
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
+  if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, F::SH::NT, F::SH::SMEM)) return e;
+  // one row per warp, one column unit per group
+  if (per_sm < 1 || F::SH::LINES * sms < N || F::SH::GROUPS * sms < N / 2 / F::CW) return cudaErrorLaunchOutOfResources;
+  *grid = sms;
+  return cudaSuccess;
+}
+template <int N>
+cudaError_t fd_launch(const FdLoopArgs& L, int grid, cudaStream_t s) {
+  using F = FdForm<N>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(F::SH::NT);
+  cfg.dynamicSmemBytes = F::SH::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_fd_loop<typename F::PL, typename F::PC, F::CW>, L);
+}
+}  // namespace
+
+int fd_loop_plan(int n, bool columns) {
+  const bool wide = columns && n < 1024;
+  switch (n) {
+    case 256: return wide ? LoopPlan<256, true>::V : LoopPlan<256, false>::V;
+    case 512: return wide ? LoopPlan<512, true>::V : LoopPlan<512, false>::V;
+    case 1024: return LoopPlan<1024, false>::V;
+    default: return -1;
+  }
+}
+cudaError_t fd_loop_prepare(int n, int* grid) {
+  switch (n) {
+    case 256: return fd_prepare<256>(grid);
+    case 512: return fd_prepare<512>(grid);
+    case 1024: return fd_prepare<1024>(grid);
+    default: return cudaErrorInvalidValue;
+  }
+}
+cudaError_t launch_fd_loop(const FdLoopArgs& L, int grid, cudaStream_t s) {
+  if (L.a.nx != L.a.ny || L.b.nx != L.a.nx || L.S < 1 || grid < 1) return cudaErrorInvalidValue;
+  switch (L.a.nx) {
+    case 256: return fd_launch<256>(L, grid, s);
+    case 512: return fd_launch<512>(L, grid, s);
+    case 1024: return fd_launch<1024>(L, grid, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 // ---- batched loop ----
 namespace {
 template <int N>

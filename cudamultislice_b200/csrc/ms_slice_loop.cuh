@@ -290,6 +290,149 @@ __global__ void __launch_bounds__(256, 1) k_slice_loop(LoopArgs L) {
 }
 
 // ---------------------------------------------------------------------------
+// Finite-difference loop: all steps of MultisliceStep (U.cu:2040-2083) on the
+// band-limited potential planes in one cooperative launch, with the two phases
+// and barriers of the slice loop.  Every warp keeps its row of psi_{n-1}, and
+// every column thread its part of the spectrum FFT2(psi_n), in registers from
+// step to step: a step moves the row-frequency band twice and one plane, where
+// the per-pass form also wrote and read psi_n, psi_{n-1} and the spectrum.
+// One row per warp and one column unit per group: the launch checks that the
+// grid of CTAs is large enough.
+// us a step, per-pass kernels in a graph against this: 256^2 6.5 and 4.6, 512^2
+// 9.9 and 5.9, 1024^2 14.5 and 11.2.
+// ---------------------------------------------------------------------------
+template <class PL, class PC, int CW>
+__global__ void __launch_bounds__(256, 1) k_fd_loop(FdLoopArgs L) {
+  using SH = LoopShape<PL, PC, CW>;
+  constexpr int N = PL::N, E = PL::E, P = PL::P, EC = PC::E, PPC = PC::P, GS = SH::GS;
+  extern __shared__ float2 smem[];
+  float* sky = reinterpret_cast<float*>(smem + SH::KY);
+  float2 *stwr = smem + SH::TWR, *stwc = smem + SH::TWC;
+  for (int i = threadIdx.x; i < N; i += SH::NT) sky[i] = L.b.ky[i];
+  for (int i = threadIdx.x; i < PL::TWSIZE; i += SH::NT) stwr[i] = L.a.tw[i];
+  if constexpr (!SH::ONE_TW)
+    for (int i = threadIdx.x; i < PC::TWSIZE; i += SH::NT) stwc[i] = L.b.tw[i];
+  __syncthreads();
+  const int G = gridDim.x;
+  const int li = threadIdx.x / P, lt = threadIdx.x % P;
+  const int line = li * G + blockIdx.x;
+  const bool has_row = line < N;
+  const long long row0 = (long long)line * N;
+  float2* smr = smem + li * SH::ROW_SLOT;
+  const int g = threadIdx.x / GS, gr = threadIdx.x % GS;
+  const int cl = gr % CW, t = gr / CW, unit = g * G + blockIdx.x;
+  const bool has_col = unit < N / 2 / CW;
+  const int col = has_col ? band_column(unit * CW, N) + cl : 0;
+  float2* smc = smem + (g * CW + cl) * SH::COL_SLOT;
+  float2* wcol = L.wave + (long long)t * N + col;
+  const float kx = L.b.kx[col], kx2 = fmul_x(kx, kx);
+  unsigned int epoch = 0;
+
+  float2 prev[E];      // psi_{n-1} of this warp's row
+  float2 spec[EC / 2]; // FFT2(psi_n): this thread's points of its column, band rows
+  float V[E];
+  // spectrum of the initial wave
+  {
+    if (has_row) {
+      float2 v[E];
+#pragma unroll
+      for (int j = 0; j < E; ++j) v[j] = L.psi[row0 + lt + P * j];
+      fft::line_fft<PL, 0, false, true, true>(v, smr, lt, stwr);
+#pragma unroll
+      for (int j = 0; j < E; ++j)
+        if (in_band(j, E)) L.wave[row0 + lt + P * j] = v[j];
+#pragma unroll
+      for (int j = 0; j < E; ++j) prev[j] = L.psim[row0 + lt + P * j];
+    }
+    if (!loop_barrier<true, false>(L.sync, ++epoch)) return;
+    if (has_col) {
+      float2 v[EC];
+#pragma unroll
+      for (int j = 0; j < EC; ++j) v[j] = wcol[(long long)j * PPC * N];
+      fft::line_fft<fft::PaddedPlan<PC>, GS, false, true, true>(v, smc, t, stwc);
+#pragma unroll
+      for (int j = 0; j < EC; ++j)
+        if (in_band(j, EC)) spec[j < EC / 4 ? j : j - EC / 2] = v[j];
+    }
+    const unsigned int seen = loop_arrive<true, false>(L.sync);
+    if (has_row) {
+#pragma unroll
+      for (int j = 0; j < E; ++j) V[j] = L.planes[row0 + lt + P * j];
+    }
+    if (!loop_wait<true, false>(L.sync, ++epoch, seen)) return;
+  }
+  for (int s = 0; s < L.S; ++s) {
+    const bool more = s + 1 < L.S;
+    // ---- row phase: psi_n, the three-level update without its Laplacian ----
+    if (has_row) {
+      float2 v[E];
+      if (s == 0) {
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = L.psi[row0 + lt + P * j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = in_band(j, E) ? L.wave[row0 + lt + P * j] : make_float2(0.f, 0.f);
+        fft::conj_all(v);
+        fft::line_fft<PL, 0, true, false, true>(v, smr, lt, stwr);
+        fft::conj_all(v);
+      }
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        const float f = 2.0f - L.a.fd_kv * V[j];
+        const float2 q = csub(cmul(L.a.fd_rc, cscale(v[j], f)), cmul(L.a.fd_ratio, prev[j]));
+        prev[j] = v[j];
+        v[j] = q;
+      }
+      fft::line_fft<PL, 0, false, true, true>(v, smr, lt, stwr);
+#pragma unroll
+      for (int j = 0; j < E; ++j)
+        if (in_band(j, E)) L.wave[row0 + lt + P * j] = v[j];
+      if (!more) {
+#pragma unroll
+        for (int j = 0; j < E; ++j) L.psim[row0 + lt + P * j] = prev[j];
+      }
+    }
+    if (!loop_barrier<true, false>(L.sync, ++epoch)) return;
+    // ---- column phase: + rc dz^2 4 pi^2 k^2 FFT2(psi_n), band limit ----
+    if (more) prefetch_rows<PL>(L.planes + (long long)(s + 1) * L.pstride, G);
+    if (has_col) {
+      float2 v[EC];
+#pragma unroll
+      for (int j = 0; j < EC; ++j) v[j] = wcol[(long long)j * PPC * N];
+      fft::line_fft<fft::PaddedPlan<PC>, GS, false, true, true>(v, smc, t, stwc);
+#pragma unroll
+      for (int j = 0; j < EC; ++j) {
+        if (!in_band(j, EC)) {
+          v[j] = make_float2(0.f, 0.f);
+          continue;
+        }
+        const int k = j < EC / 4 ? j : j - EC / 2;
+        const float ky = sky[t + PPC * j];
+        const bool keep = fadd_x(kx2, fmul_x(ky, ky)) < L.b.k2_le;  // sqrt(k^2) <= kmax
+        const float k2 = kx * kx + ky * ky;
+        const float2 nv = keep ? cadd(v[j], cscale(cmul(L.b.fd_c, spec[k]), k2)) : make_float2(0.f, 0.f);
+        spec[k] = nv;
+        v[j] = cscale(nv, L.b.scale);
+        if (!more) L.b.spec[(long long)col * N + t + PPC * j] = nv;
+      }
+      fft::conj_all(v);
+      fft::line_fft<fft::PaddedPlan<PC>, GS, true, false, true>(v, smc, t, stwc);
+      fft::conj_all(v);
+#pragma unroll
+      for (int j = 0; j < EC; ++j) wcol[(long long)j * PPC * N] = v[j];
+    }
+    if (!more) return;
+    const unsigned int seen = loop_arrive<true, false>(L.sync);
+    if (has_row) {
+      const float* Vn = L.planes + (long long)(s + 1) * L.pstride + row0;
+#pragma unroll
+      for (int j = 0; j < E; ++j) V[j] = Vn[lt + P * j];
+    }
+    if (!loop_wait<true, false>(L.sync, ++epoch, seen)) return;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Batched loop: the instances of up to two groups (grid sizes N0 >= N1) share
 // every phase.  A row phase covers every line of every instance, a column
 // phase every column unit of every instance, with grid barriers between them,

@@ -272,8 +272,9 @@ ms_status ms_run_conventional(ms_sim* sim, int* nslices);
  * loops over it (MainWindow.xaml.cs:258-283), equivalent to
  * ms_multislice_step_fd(i) for i = 1..nsteps.  The band-limited potential
  * planes are built once into a device-resident stack (rebuilt when the
- * structure, grid or FD step changes); the fused path then replays one
- * captured CUDA graph of two passes per step.  *nsteps_out (may be NULL)
+ * structure, grid or FD step changes); the fused path then runs all steps in
+ * one persistent cooperative launch (square 256, 512 and 1024 grids,
+ * MS_OPT_SLICE_LOOP) or replays one captured CUDA graph of two passes per step.  *nsteps_out (may be NULL)
  * receives the step count; device time in ms_get_last_device_ms. */
 ms_status ms_run_fd(ms_sim* sim, int nsteps, int* nsteps_out);
 /* Annular detector (no reference counterpart; the HAADF/ADF STEM signal):
