@@ -249,7 +249,9 @@ __global__ void __launch_bounds__(T) k_general_rows(const __grid_constant__ GenA
         float s, c;
         sincos_red(fmul_x(g.sigma, V[m]), &s, &c);
         const float2 v = inv ? cconj(a[i]) : a[i];
-        a[i] = cmul(v, make_float2(c, s));
+        // (contraction written out: one slice per launch pair and a chain of
+        // slices round the same way)
+        a[i] = make_float2(fmaf(v.x, c, -fmul_x(v.y, s)), fmaf(v.x, s, fmul_x(v.y, c)));
       }
     }
     gen_line_fft(g.plan, a, b, tw, 1, t, T);
