@@ -90,16 +90,18 @@ int plan_variants() { return kPlanVariants; }
 // passes of the slice loop; 1, 4, 16, 64 instances):
 //                  chosen                    next best
 //   rows  128      5: 2.5 2.4 3.4, 4: 5.6    1: -, -, 3.5, 5.7
-//         256      5: 3.4, 4: 3.6 5.8, 0: 13.8   4: 3.4, 0: 3.6 6.6, 3: 14.1
+//         256      5: 3.4, 4: 3.3 5.7, 0: 13.1   4: 3.4, 0: 3.4 4.7, 3: 12.1
 //         512      5: 3.4, 0: 5.6 16.7 58.3  2: 3.4, 1: 5.7, 4: 16.8 60.3
 //         1024     0: 5.9 17.5 60.6 246      3: 6.2, 4: 19.0 66.3 258
 //         2048     4: 20.1 71.5 274          1: 20.4 76.0 297
 //         4096     4: 79.7 302               1: 86.8, 0: 325
+//   rows, tc, 512   5: 3.4, 1: 5.6 16.1, 0: 40.3   0: 5.8 12.4, 1: 57.6 (a 512^2
+//                  raster of 16 instances takes the same with either)
 //   rows, tc, 2048 and up  0: 20.7 73.2 270, 1 at 4096: 84.9 324
 //   columns 128    5: 2.5 3.5 2.7 4.4        2
 //         256      5: 2.7 3.5 4.9, 3: 10.0   4: 3.1, 1: 5.2, 0: 10.2
-//         512      5: 3.8, 3: 6.0, 0: 11.6 39.3   2: 3.6, 4: 6.3, 3: 12.1 40.6
-//         1024     3: 7.1, 0: 11.9 40.1 179  1: 8.0, 3: 15.6 53.6 230
+//         512      5: 3.8, 3: 6.0, 0: 9.8 35.3   2: 3.6, 4: 6.3, 3: 12.1 40.6
+//         1024     3: 7.1, 0: 11.2 38.3 172  1: 8.0, 3: 15.6 53.6 230
 //         2048     3: 18.7, 0: 53.7 231      1: 20.0 58.9 251
 //         4096     3: 60.5, 0: 254           0: 67.9, 3: 304
 // Timing them on each handle's first use instead took 2-5 ms, and at one

@@ -247,6 +247,29 @@ MS_D void row_mid(float2 (&v)[PL::E], const PassAArgs& a, const RowOperands<PL, 
   }
 }
 
+// Where the transforms of a slice pass skip the butterflies of the band's zeros
+// (fft::line_fft's BIN, BOUT): this takes two copies of the transform's code
+// instead of one, more registers in flight and more instructions to fetch.
+// Taken where that measured faster (us per launch, one copy -> two; B200):
+//   rows of up to 256       256: 64 instances 13.8 -> 13.1, stored transmission
+//                           12.8 -> 11.8; 16 instances 6.6 -> 4.7; one instance,
+//                           both passes: 128 4.15 -> 3.9, 256 4.98 -> 4.5
+//   rows of 512, stored transmission, the unpacked 32-point plan
+//                           16 instances 16.3 -> 12.4, 64: 52.5 -> 40.3
+//   columns of 512 and 1024, that plan   512, 64: 39.4 -> 35.3; 1024, 4:
+//                           11.8 -> 11.2, 16: 40.2 -> 38.3, 64: 179 -> 172
+// and not where it lost: rows of 512 with the exponential 58.5 -> 59.6 (64),
+// of 1024 246 -> 264, stored 221 -> 225, of 4096 at one instance 80 -> 92;
+// columns of 128 at 64 instances 4.4 -> 4.7, the packed plan at 1024 7.1 -> 8.7,
+// 4096 254 -> 267.
+template <class PL>
+__host__ __device__ constexpr bool wide_plan() { return PL::E >= 32 && !PL::PK; }
+template <class PL, int FLAGS>
+__host__ __device__ constexpr bool row_skips() {
+  return (FLAGS & A_INV) != 0 && (FLAGS & A_FWD) != 0 && (FLAGS & A_BI) != 0 && (FLAGS & A_BO) != 0 &&
+         (((FLAGS & (A_MULT_T | A_MULT_TC)) != 0 && PL::N <= 256) ||
+          ((FLAGS & A_MULT_TC) != 0 && PL::N == 512 && wide_plan<PL>()));
+}
 template <class PL, int FLAGS>
 MS_D void pass_a_body(PassAArgs a) {
   constexpr int NX = PL::N, E = PL::E, P = PL::P, LS = PL::SLOT;
@@ -269,7 +292,13 @@ MS_D void pass_a_body(PassAArgs a) {
   op.load(a, inst, line, row0, t);
 
   if constexpr (!INVF) row_mid<PL, FLAGS>(v, a, op, inst, line, row0, t);
-  if constexpr (INVF || FWDF) {
+  if constexpr (row_skips<PL, FLAGS>()) {
+    fft::conj_all(v);
+    fft::line_fft<PL, 0, true>(v, sm, t, a.tw);
+    fft::conj_all(v);
+    row_mid<PL, FLAGS>(v, a, op, inst, line, row0, t);
+    fft::line_fft<PL, 0, false, true>(v, sm, t, a.tw);
+  } else if constexpr (INVF || FWDF) {
     // one copy of the transform code: iteration 0 is the inverse
     // conj(FFT(conj(.))) followed by the pointwise work, iteration 1 the forward
 #pragma unroll 1
@@ -328,6 +357,11 @@ __host__ __device__ constexpr bool col_stages_py() { return col_uses_py<MODE>() 
 template <int MODE>
 __host__ __device__ constexpr bool col_band_limited() {
   return MODE == B_PROPAGATE || MODE == B_PROPAGATE_ADJ || MODE == B_BANDLIMIT || MODE == B_FD;
+}
+// (see row_skips)
+template <class PL, int MODE>
+__host__ __device__ constexpr bool col_skips() {
+  return MODE == B_PROPAGATE && (PL::N == 512 || PL::N == 1024) && wide_plan<PL>();
 }
 // The column's own factors.  The persistent loop loads them with the column's
 // points (its barriers empty L1); the pass kernels at use: their registers are
@@ -465,21 +499,29 @@ __global__ void __launch_bounds__(cols_per_cta<PL>() * PL::P, col_min_ctas<PL>()
   for (int j = 0; j < E; ++j) v[j] = src[j * step];
   if constexpr (SKY || SPY) __syncthreads();  // tables of every group
 
-  // iteration 0: forward (or, for B_INV_ONLY, the conjugated inverse) and the
-  // pointwise work; iteration 1: the inverse as conj(FFT(conj(.)))
+  if constexpr (col_skips<PL, MODE>()) {
+    fft::line_fft<fft::PaddedPlan<PL>, GS, false, true>(v, sm, t, a.tw);
+    col_mid<PL, MODE>(v, a, ColFactors::load<MODE>(a, col), sky, spy, col, t, base);
+    fft::conj_all(v);
+    fft::line_fft<fft::PaddedPlan<PL>, GS, true>(v, sm, t, a.tw);
+    fft::conj_all(v);
+  } else {
+    // iteration 0: forward (or, for B_INV_ONLY, the conjugated inverse) and the
+    // pointwise work; iteration 1: the inverse as conj(FFT(conj(.)))
 #pragma unroll 1
-  for (int it = 0; it < (TWO ? 2 : 1); ++it) {
-    if (MODE == B_INV_ONLY) fft::conj_all(v);
-    fft::line_fft<fft::PaddedPlan<PL>, GS>(v, sm, t, a.tw);
-    if (it == 0) {
-      if constexpr (MODE == B_INV_ONLY) {
-        fft::conj_all(v);
-      } else if constexpr (TWO) {
-        col_mid<PL, MODE>(v, a, ColFactors::load<MODE>(a, col), sky, spy, col, t, base);
+    for (int it = 0; it < (TWO ? 2 : 1); ++it) {
+      if (MODE == B_INV_ONLY) fft::conj_all(v);
+      fft::line_fft<fft::PaddedPlan<PL>, GS>(v, sm, t, a.tw);
+      if (it == 0) {
+        if constexpr (MODE == B_INV_ONLY) {
+          fft::conj_all(v);
+        } else if constexpr (TWO) {
+          col_mid<PL, MODE>(v, a, ColFactors::load<MODE>(a, col), sky, spy, col, t, base);
+          fft::conj_all(v);
+        }
+      } else {
         fft::conj_all(v);
       }
-    } else {
-      fft::conj_all(v);
     }
   }
 
