@@ -921,11 +921,13 @@ __device__ __noinline__ float clamp_value(const float* __restrict__ tab, const f
 // range map to a zero segment, positions of two pixels share packed FP32x2
 // instructions, and the rare rest (clamp region, bins with many thresholds) is
 // one branch per atom.  Per slice of the 50k-atom carbon slab (0.1 atoms/A^3,
-// 2 A slices) in a stack build, tables included: 1024^2 at 0.049 A 49 -> 28.6 us,
-// 4096^2 at 0.012 A 547 -> 276 us (against the sum over 12 Gaussians at every
+// 2 A slices) in a stack build, tables included: 1024^2 at 0.049 A 49 -> 27.9 us,
+// 4096^2 at 0.012 A 547 -> 272 us (against the sum over 12 Gaussians at every
 // pixel).  CTAs of four warps: eight warps waited longer at the staging
 // barriers (30.2 us); tables staged in shared memory cost occupancy and more
-// L2 traffic (34.8 us).
+// L2 traffic (34.8 us).  Every second patch of an atom inside the slice meets
+// the cut-off's rim, up to ten thresholds in a bin: counted four loads at a time
+// (one by one 28.3 us; two at a time for all of a thread's pixels at once 29.3).
 constexpr int kSepChunk = 128;  // candidates staged at a time
 
 constexpr int kSepThreads = 128;
@@ -1135,8 +1137,14 @@ __global__ void __launch_bounds__(kSepThreads, sep_ctas<RY>()) k_potential_sep(c
                                         __float_as_int(hd.w), dxy[r], fmaf(dxv, dxv, dyv * dyv), hd.y);
                 } else {
                   // more than three thresholds in the bin (the cut-off's rim)
-                  int c = sg[r] - (rad_bin(s) - __float_as_int(hd.z));
-                  while (dxy[r] >= __ldg(tab + kTabAsc + c)) ++c, ++sg[r];
+                  int c = sg[r] - (rad_bin(s) - __float_as_int(hd.z)), k;
+                  do {  // (four loads in flight; past the last threshold: 1e30)
+                    const float* t = tab + kTabAsc + c;
+                    k = (dxy[r] >= __ldg(t)) + (dxy[r] >= __ldg(t + 1)) + (dxy[r] >= __ldg(t + 2)) +
+                        (dxy[r] >= __ldg(t + 3));
+                    c += k;
+                    sg[r] += k;
+                  } while (k == 4);
                 }
               }
             }
