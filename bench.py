@@ -50,7 +50,7 @@ def workload(size=SIZE):
     return Z, x, y, z
 
 
-FORCED_PLAN = -1  # profiling: FFT plan variant forced on every leg's engine (-1: autotuned)
+FORCED_PLAN = -1  # profiling: FFT plan variant forced on every leg's engine (-1: the engine's choice)
 
 
 def new_sim(device: int):
@@ -693,7 +693,7 @@ def main():
     ap.add_argument("--profile", action="store_true",
                     help="profiling mode: set-up plus the timed slice loop only (no e2e, plain or CPU legs)")
     ap.add_argument("--fft-plan", type=int, default=-1,
-                    help="profiling mode and --leg runs: force this FFT plan variant (default: the autotuner's choice)")
+                    help="profiling mode and --leg runs: force this FFT plan variant (default: the engine's choice)")
     ap.add_argument("--leg", choices=["stem", "adjoint", "tds", "mixed", "focal_profile", "c1", "fd", "grid4096",
                                        "grid4096_profile", "potential"],
                     help="run one secondary leg alone and print its JSON (exploration)")
@@ -848,7 +848,7 @@ def main():
         "config": config_dict(len(Z)), "clocks": clk, "gpu_launches": launches,
         "fft_plan": ({"slice_loop": "packed 32-point plan (variant 3), one warp per line, both phases"} if loop_on
                      else {"row_variant": fft_plan[0], "col_variant": fft_plan[1],
-                           "selected_by": "on-device autotuner"}),
+                           "selected_by": "measured table by length and batch"}),
         "roofline": roofline,
         "plain_path": {"value": plain_value, "unit": UNIT, "speedup_fused_vs_plain": value / world / plain_value},
         "per_pass_path": per_pass,

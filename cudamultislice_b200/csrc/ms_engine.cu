@@ -281,7 +281,7 @@ class Engine {
       case MS_OPT_POTENTIAL_SUM:
         if (value < 0 || value > 2) return fail(MS_ERR_INVALID, "potential sum must be 0 (auto), 1 or 2");
         pot_sum_ = value;
-        if (!pot_tile_forced_) pot_tile_ = -1;  // (the tile is tuned per kernel)
+        if (!pot_tile_forced_) pot_tile_ = -1;  // (the choice is per kernel)
         stack_valid_ = false;
         fd_stack_valid_ = false;
         invalidate_graph();
@@ -3232,7 +3232,7 @@ class Engine {
   int nrows_fp_ = 0;
   bool have_fp_ = false;
   // separable potential: expansions [103][2][kGaussJ], per-atom tables of the
-  // current slice, the loaded rows (FP64), per-row check (-1 not yet checked)
+  // slices in flight, the loaded rows (FP64), per-row check (-1 not yet checked)
   static constexpr double kGaussTol = 2e-7;
   DevBuf<float> d_gauss_, d_tab_;
   DevBuf<int> d_zstart_;
