@@ -2779,7 +2779,7 @@ class Engine {
     if (dz == prop_dz_ && d_px_.p) return MS_OK;
     std::vector<float2> px(nx_), py(ny_);
     const double invN = 1.0 / ((double)nx_ * ny_);
-    // unit factors nearest modulus 1 (unit_fp32); the 1/N of the fused
+    // unit factors near modulus 1 (unit_fp32); the 1/N of the fused
     // passes is a power of two, so scaling px by it is exact
     const float fN = (float)invN;
     for (int i = 0; i < nx_; ++i) {

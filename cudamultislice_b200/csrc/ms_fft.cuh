@@ -15,7 +15,7 @@
 // pass 1 hit distinct banks.  In-register butterflies are radix-2 DIF networks
 // with compile-time twiddles applied as exact quarter turns plus three-shear
 // rotations (twc); trivial twiddles cost no multiply.  Table twiddles are the
-// FP32 pairs nearest unit modulus (unit_fp32).
+// FP32 pairs near unit modulus (unit_fp32).
 // Forward = exp(-2 pi i jk/N) (cuFFT CUFFT_FORWARD); the inverse is computed as
 // conj(FFT(conj(x))) so that a kernel holds one copy of the transform code
 // (instruction-cache footprint); both directions unnormalised.

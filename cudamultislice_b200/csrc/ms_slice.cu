@@ -66,17 +66,19 @@ void band_limit_thresholds(float kmax, float* k2_lt, float* k2_le) {
 float2 unit_fp32(double c, double s) {
   const float c0 = (float)c, s0 = (float)s;
   float bc = c0, bs = s0;
-  double bn = INFINITY, ba = INFINITY;
+  double best = INFINITY;
   const double ang = std::atan2(s, c);
   for (int dc = -1; dc <= 1; ++dc)
     for (int ds = -1; ds <= 1; ++ds) {
       const float cc = dc == 0 ? c0 : std::nextafter(c0, dc > 0 ? INFINITY : -INFINITY);
       const float ss = ds == 0 ? s0 : std::nextafter(s0, ds > 0 ? INFINITY : -INFINITY);
-      const double n = std::fabs((double)cc * cc + (double)ss * ss - 1.0);
-      const double a = std::fabs(std::atan2((double)ss, (double)cc) - ang);
-      if (n < bn || (n == bn && a < ba)) {
-        bn = n;
-        ba = a;
+      // the modulus first: its error adds up over all transforms of a run, the
+      // angle's partly cancels between a transform and its inverse
+      const double n = (double)cc * cc + (double)ss * ss - 1.0;
+      const double a = std::remainder(std::atan2((double)ss, (double)cc) - ang, 6.283185307179586);
+      const double cost = std::hypot(n, 0.2 * a);
+      if (cost < best) {
+        best = cost;
         bc = cc;
         bs = ss;
       }

@@ -125,11 +125,15 @@ struct PassBArgs {
 // with them takes exactly the decisions of the rounded square root.
 void band_limit_thresholds(float kmax, float* k2_lt, float* k2_le);
 
-// (cos, sin) as the FP32 pair within one ulp of each component whose modulus
-// is nearest 1 (ties: nearest angle).  Unit factors applied once per transform
+// (cos, sin) as the FP32 pair within one ulp of each component with the least
+// hypot(|modulus^2 - 1|, angle error / 5).  Unit factors applied once per transform
 // or per slice (twiddles, propagator) then scale the wave by |(c, s)|^S over a
 // stack of S slices only to that pair's remaining modulus error, far below the
-// plain rounding's, which adds up coherently when the slices repeat (crystals).
+// plain rounding's, which adds up coherently when the slices repeat (crystals).  The
+// modulus alone would let the angle be off by more than an ulp: 52 slices of a
+// 512^2 crystal then end 0.94e-6 to 1.11e-6 from FP64, with the fifth of the angle
+// 0.84e-6 to 0.98e-6, and a focal-series loss 0.94e-6 (rms of 32 inputs) against
+// 0.42e-6; a tenth or a half of the angle 0.69e-6 and 1.0e-6.
 float2 unit_fp32(double c, double s);
 
 // Line lengths 64..4096 (powers of two) in both directions.
