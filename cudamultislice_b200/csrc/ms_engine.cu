@@ -2363,7 +2363,10 @@ class Engine {
           launches += 2;
           if (dLdxy) {
             PotArgs pa = pot_args(POT_CONVENTIONAL, n, nullptr);
-            const int a0 = hzoff_[pa.kt], a1 = hzoff_[pa.kb + 1];
+            // (the last slice can lie wholly below the box: an empty window,
+            // kt past the last z-bin)
+            const bool window = pa.kt <= pa.kb;
+            const int a0 = window ? hzoff_[pa.kt] : 0, a1 = window ? hzoff_[pa.kb + 1] : 0;
             if (sep && n < adj_lo) {
               // (after the adjoints that read the buffer: the same stream)
               adj_lo = std::max(1, n - adj_gs + 1);

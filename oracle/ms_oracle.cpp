@@ -1292,6 +1292,7 @@ extern "C" int or_focal_grad(or_sim* s, const float* defoci, int nd, const doubl
                 z2d[m - 1] = (double)z - m * (double)s->convdz / 20.0;
             }
             const double wsub = (double)s->convdz / 20.0;
+            if (kt > kb) continue;  // (the slice lies below the box)
             const int a0 = s->off[kt * kBins * kBins], a1 = s->off[(kb + 1) * kBins * kBins];
 #pragma omp parallel for schedule(dynamic, 8)
             for (int l = a0; l < a1; ++l) {
