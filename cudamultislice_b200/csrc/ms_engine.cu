@@ -2264,6 +2264,12 @@ class Engine {
     // timed from here: the potential stack (when the atoms changed), the sweeps
     MS_TRY(cudaEventRecord(ev0_, stream_));
     if (int rc = build_stack(&Sall)) return rc;
+    // (the second pixel stream writes the derivative tables where earlier
+    // potentials of the handle, whose launches may still be queued, read theirs)
+    if (grad && dLdxy) {
+      MS_TRY(cudaEventRecord(ev_fork_, stream_));
+      MS_TRY(cudaStreamWaitEvent(pix_[1], ev_fork_, 0));
+    }
     constexpr int kSaveFirst = A_SAVE | A_MULT_T | A_FWD | A_BO;
     constexpr int kSaveNext = A_INV | A_SAVE | A_MULT_T | A_FWD | A_BI | A_BO;
     // forward sweep; checkpoint c (c = 1..nck-1) holds X_{cK}; the waves of
