@@ -23,7 +23,6 @@
 #include <new>
 #include <sstream>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -31,6 +30,7 @@
 #include "ms_atoms.cuh"
 #include "ms_general.cuh"
 #include "ms_philox.h"
+#include "ms_team.h"
 #include "ms_tiff.h"
 #include "ms_pointwise.cuh"
 #include "ms_slice.cuh"
@@ -2613,18 +2613,7 @@ class Engine {
       }
       rc[t] = e;
     };
-    {
-      std::thread th[StagePool::kThreads];
-      size_t started = 1;
-      try {
-        for (; started < nt; ++started) th[started] = std::thread(work, started);
-      } catch (const std::system_error&) {
-        // (no more threads: this one takes the remaining shares)
-      }
-      work(0);
-      for (size_t t = started; t < nt; ++t) work(t);
-      for (size_t t = 1; t < started; ++t) th[t].join();
-    }
+    run_team<StagePool::kThreads>(nt, work);
     bool ok = true;
     for (cudaError_t e : rc) ok = ok && e == cudaSuccess;
     // (after a failure a transfer may still be in flight on a chunk)
@@ -3191,8 +3180,8 @@ class Engine {
     const long long total = (long long)n * nb;
     const int hw = (int)std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
     const int nt = (int)std::max<long long>(1, std::min<long long>(hw, total / 4096));
-    auto work = [&](int t) {
-      const long long q0 = total * t / nt, q1 = total * (t + 1) / nt;
+    auto work = [&](size_t t) {
+      const long long q0 = total * (long long)t / nt, q1 = total * (long long)(t + 1) / nt;
       for (long long q = q0; q < q1;) {
         const int k = (int)(q / n), a0 = (int)(q % n);
         const int a1 = (int)std::min<long long>(n, a0 + (q1 - q));
@@ -3201,15 +3190,7 @@ class Engine {
         q += a1 - a0;
       }
     };
-    if (nt == 1) {
-      work(0);
-      return;
-    }
-    std::vector<std::thread> th;
-    th.reserve(nt - 1);
-    for (int t = 1; t < nt; ++t) th.emplace_back(work, t);
-    work(0);
-    for (auto& h : th) h.join();
+    run_team<32>((size_t)nt, work);
   }
 
   // state
