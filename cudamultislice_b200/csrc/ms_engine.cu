@@ -2320,12 +2320,14 @@ class Engine {
       // position adjoint: the derivative tables of adj_gs slices at a time
       // (one launch per group; a launch per slice was half of its time on
       // small windows), those of slices adj_lo and up in place
-      const bool sep = dLdxy && separable_ok();
+      bool sep = dLdxy && separable_ok();
       const size_t rows = sep ? window_atoms(hzoff_, nzb_, 1) : 1, per = rows * kTabStride;
       const int adj_gs = (int)std::max<size_t>(1, std::min<size_t>(kTabBytes / (per * sizeof(float)), kSepGroup));
       int adj_lo = S + 1;
-      if (sep)
-        if (int rc = ensure_tables(rows * adj_gs)) return rc;
+      if (sep && !have_tables(rows * adj_gs)) {
+        if (int rc = no_tables()) return rc;
+        sep = false;
+      }
       for (int c = clast; c >= 0; c -= K) {
         const int e = std::min(c + K, S);
         // psi_c .. psi_{e-1} (real space) into segment slots 0 .. e-1-c
@@ -2434,8 +2436,16 @@ class Engine {
     }
     return (size_t)std::max(most, 1);
   }
-  int ensure_tables(size_t rows) {
-    if (d_tab_.n < rows * kTabStride) MS_TRY(d_tab_.resize(rows * kTabStride));
+  // Room for `rows` rows of atom tables; false where the device has none left.
+  bool have_tables(size_t rows) {
+    if (d_tab_.n >= rows * kTabStride || d_tab_.resize(rows * kTabStride) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+  }
+  // Without that room potentials and their adjoint are summed per sub-plane,
+  // unless the separable sum is forced.
+  int no_tables() {
+    if (pot_sum_ == 2) return fail(MS_ERR_NOMEM, "no device memory for the separable potential's atom tables");
     return MS_OK;
   }
 
@@ -2916,13 +2926,13 @@ class Engine {
   // batch of nb indices set up as in tds_potential_batch, instance k at
   // out + k * S * N), in groups of consecutive slices: one table launch and
   // one potential launch per group, each over the group's slices and
-  // instances.  Three table buffers: the tables of the next groups are built
+  // instances.  Up to three table buffers: the tables of the next groups are built
   // on the side stream while earlier groups' potentials run; group g's
-  // potentials run on pixel stream g % kPixStreams (stream 0 is the handle's),
+  // potentials run on pixel stream g % buffers (stream 0 is the handle's),
   // so that the last CTAs of one launch overlap the first of the next.  The
   // tables' side stream has the higher priority, so the next group's tables
   // are not queued behind potential CTAs.  Event order: tables(g) after
-  // potentials(g - 3), which read the same buffer; potentials(g) after
+  // potentials(g - buffers), which read the same buffer; potentials(g) after
   // tables(g).  The side stream joins the handle's stream through the last
   // potentials' dependence on their tables.
   //
@@ -2931,57 +2941,111 @@ class Engine {
   // slice passes that follow group by group start early.  A launch per slice
   // left small grids to the launches and the table kernel's latency (256^2, 42
   // slices: 14 us of tables per slice against 4 us in groups of seven).
-  static constexpr size_t kTabBytes = 24u << 20;
+  //
+  // Large tables: one slice of nb instances can exceed kTabBytes by far, most of
+  // all in specimens thinner than the z-window, where every atom has a row in
+  // every slice (100k atoms x 128 instances: 67 GB).  Instances are then taken in
+  // equal parts of at most kTabMost a buffer, a single instance above that in
+  // fewer buffers, and where the device has no room for those either, in fewer
+  // and smaller ones and at last by the per-sub-plane kernel, without tables.
+  static constexpr size_t kTabBytes = 24u << 20, kTabMost = (size_t)4 << 30;
   int separable_stack(int S, float* out, size_t N, int nb, const float4* atoms = nullptr, const int* off = nullptr,
                       long long b_atoms = 0, long long b_off = 0,
                       const std::function<int(int, cudaEvent_t)>& after_slice = nullptr,
                       const std::vector<int>* zoff = nullptr) {
-    const int tile = separable_tile_option();
-    const size_t rows = window_atoms(zoff ? *zoff : hzoff_, nzb_, nb);
-    const size_t per = (size_t)nb * rows * kTabStride;  // one slice's tables
-    const int gs = (int)std::max<size_t>(
-        1, std::min<size_t>({kTabBytes / (per * sizeof(float)), (size_t)kSepGroup, (size_t)(S + 5) / 6}));
-    const int groups = (S + gs - 1) / gs, npix = std::min(groups, kPixStreams);
-    if (int rc = ensure_tables(npix * gs * nb * rows)) return rc;
+    const size_t rows = window_atoms(zoff ? *zoff : hzoff_, nzb_, nb), bytes = rows * kTabStride * sizeof(float);
+    const size_t most = std::max<size_t>(kTabMost / bytes, 1), parts = (nb + most - 1) / most;
+    int nbp = (int)((nb + parts - 1) / parts);  // instances of a part
+    int gs = (int)std::max<size_t>(
+        1, std::min<size_t>({kTabBytes / (nbp * bytes), (size_t)kSepGroup, (size_t)(S + 5) / 6}));
+    int bufs = (int)std::min<size_t>({(size_t)((S + gs - 1) / gs), (size_t)kPixStreams,
+                                      std::max<size_t>(3 * kTabMost / (gs * nbp * bytes), 1)});
+    while (!have_tables((size_t)bufs * gs * nbp * rows)) {
+      if (bufs > 1) {
+        --bufs;
+      } else if (gs > 1) {
+        gs = 1;
+      } else if (nbp > 1) {
+        nbp = (nbp + 1) / 2;
+      } else {
+        if (int rc = no_tables()) return rc;
+        return sub_plane_stack(S, out, N, nb, atoms, off, b_atoms, b_off, after_slice);
+      }
+    }
+    for (int k = 0; k < nb; k += nbp) {
+      const int n = std::min(nbp, nb - k);
+      SepArgs a = sep_args(PotArgs{}, (int)rows);
+      a.nb = n;
+      a.s_tab = (long long)((size_t)nbp * rows * kTabStride);
+      a.s_V = (long long)N;
+      if (int rc = separable_part(a, S, out + (size_t)k * S * N, gs, bufs, atoms ? atoms + k * b_atoms : nullptr,
+                                  atoms ? off + k * b_off : nullptr, b_atoms, b_off, after_slice))
+        return rc;
+    }
+    last_pot_sum_ = 2;
+    return MS_OK;
+  }
+  // The stacks of one part's instances (a.nb of them; strides and rows in a), in
+  // groups of gs slices and `bufs` table buffers.
+  int separable_part(SepArgs a, int S, float* out, int gs, int bufs, const float4* atoms, const int* off,
+                     long long b_atoms, long long b_off, const std::function<int(int, cudaEvent_t)>& after_slice) {
+    const int tile = separable_tile_option(), groups = (S + gs - 1) / gs;
     MS_TRY(cudaEventRecord(ev_fork_, stream_));
     MS_TRY(cudaStreamWaitEvent(side_, ev_fork_, 0));
-    for (int k = 1; k < npix; ++k) MS_TRY(cudaStreamWaitEvent(pix_[k], ev_fork_, 0));
+    for (int k = 1; k < bufs; ++k) MS_TRY(cudaStreamWaitEvent(pix_[k], ev_fork_, 0));
     int rc = MS_OK;
     for (int g = 0; g < groups && rc == MS_OK; ++g) {
-      const int it0 = 1 + g * gs, ns = std::min(gs, S + 1 - it0), buf = g % npix;
-      SepArgs a = sep_args(pot_args(POT_CONVENTIONAL, it0, out + (size_t)(it0 - 1) * N), (int)rows);
-      for (int i = 1; i < ns; ++i) a.set_slice(i, pot_args(POT_CONVENTIONAL, it0 + i, nullptr));
-      a.ns = ns;
-      a.nb = nb;
-      a.s_tab = (long long)per;
-      a.s_V = (long long)N;
-      a.p.tab = d_tab_.p + (size_t)buf * gs * per;
+      const int it0 = 1 + g * gs, buf = g % bufs;
+      a.ns = std::min(gs, S + 1 - it0);
+      a.p = pot_args(POT_CONVENTIONAL, it0, out + (size_t)(it0 - 1) * a.s_V);
+      a.set_slice(0, a.p);
+      for (int i = 1; i < a.ns; ++i) a.set_slice(i, pot_args(POT_CONVENTIONAL, it0 + i, nullptr));
+      a.p.tab = d_tab_.p + (size_t)buf * gs * a.s_tab;
       if (atoms) {
         a.p.atoms = atoms;
         a.p.off = off;
         a.p.b_atoms = b_atoms;
         a.p.b_off = b_off;
-        a.p.b_tab = (long long)(rows * kTabStride);
-        a.p.b_V = (long long)S * N;
+        a.p.b_tab = (long long)a.rows * kTabStride;
+        a.p.b_V = (long long)S * a.s_V;
       }
-      rc = separable_group(a, g, buf, npix, tile);
-      for (int i = 0; i < ns && rc == MS_OK && after_slice; ++i) rc = after_slice(it0 + i, ev_pix_[buf]);
+      rc = separable_group(a, g, buf, bufs, tile);
+      for (int i = 0; i < a.ns && rc == MS_OK && after_slice; ++i) rc = after_slice(it0 + i, ev_pix_[buf]);
     }
     // join the other pixel streams (also on failure, so that the handle's
     // stream orders after everything enqueued)
-    for (int k = 1; k < npix; ++k) {
+    for (int k = 1; k < bufs; ++k) {
       MS_TRY(cudaEventRecord(ev_pjoin_[k], pix_[k]));
       MS_TRY(cudaStreamWaitEvent(stream_, ev_pjoin_[k], 0));
     }
-    if (rc != MS_OK) return rc;
-    last_pot_sum_ = 2;
+    return rc;
+  }
+  // The same stacks by the per-sub-plane kernel, one slice at a time on the
+  // handle's stream.
+  int sub_plane_stack(int S, float* out, size_t N, int nb, const float4* atoms, const int* off, long long b_atoms,
+                      long long b_off, const std::function<int(int, cudaEvent_t)>& after_slice) {
+    for (int k = 0; k < nb; ++k)
+      for (int it = 1; it <= S; ++it) {
+        PotArgs a = pot_args(POT_CONVENTIONAL, it, out + ((size_t)k * S + (it - 1)) * N);
+        if (atoms) {
+          a.atoms = atoms + k * b_atoms;
+          a.off = off + k * b_off;
+        }
+        MS_TRY(launch_potential(a, POT_CONVENTIONAL, stream_, sub_plane_tile()));
+        ++launches;
+        if (after_slice) {
+          MS_TRY(cudaEventRecord(ev_pix_[0], stream_));
+          if (int rc = after_slice(it, ev_pix_[0])) return rc;
+        }
+      }
+    last_pot_sum_ = 1;
     return MS_OK;
   }
   // Group g of separable_stack: its tables on the side stream (into buffer
-  // buf, once the potentials of group g - npix, which read it, are done), then
+  // buf, once the potentials of group g - bufs, which read it, are done), then
   // its potentials on pixel stream buf.
-  int separable_group(const SepArgs& a, int g, int buf, int npix, int tile) {
-    if (g >= npix) MS_TRY(cudaStreamWaitEvent(side_, ev_pix_[buf], 0));
+  int separable_group(const SepArgs& a, int g, int buf, int bufs, int tile) {
+    if (g >= bufs) MS_TRY(cudaStreamWaitEvent(side_, ev_pix_[buf], 0));
     MS_TRY(launch_atom_tables(a, side_));
     MS_TRY(cudaEventRecord(ev_tab_[buf], side_));
     MS_TRY(cudaStreamWaitEvent(pix_[buf], ev_tab_[buf], 0));
@@ -2991,8 +3055,8 @@ class Engine {
     return MS_OK;
   }
   // One slice's tables and potential on the handle's stream.
-  cudaError_t launch_separable(const PotArgs& a, int tile) {
-    const SepArgs sa = sep_args(a, (int)window_atoms(hzoff_, nzb_, 1));
+  cudaError_t launch_separable(const PotArgs& a, int rows, int tile) {
+    const SepArgs sa = sep_args(a, rows);
     if (cudaError_t e = launch_atom_tables(sa, stream_)) return e;
     return launch_potential_from_tables(sa, stream_, tile);
   }
@@ -3034,19 +3098,21 @@ class Engine {
 
   // Potential of one slice into out (ny x nx floats).
   int potential_slice(int kind, int it, float* out) {
-    const bool sep = kind == POT_CONVENTIONAL && separable_ok();
+    bool sep = kind == POT_CONVENTIONAL && separable_ok();
     if (kind == POT_CONVENTIONAL && pot_sum_ == 2 && !sep)
       return fail(MS_ERR_UNSUPPORTED, "an element of the specimen has no valid Gaussian expansion");
+    const size_t rows = sep ? window_atoms(hzoff_, nzb_, 1) : 0;
+    if (sep && !have_tables(rows)) {
+      if (int rc = no_tables()) return rc;
+      sep = false;
+    }
     if (kind == POT_CONVENTIONAL && !sep && pot_tile_ < 0 && !capturing_)
       if (int rc = tune_pot_tile()) return rc;
-    if (sep)
-      if (int rc = ensure_tables(window_atoms(hzoff_, nzb_, 1))) return rc;
     const PotArgs a = pot_args(kind, it, out);
     if (sep)
-      MS_TRY(launch_separable(a, separable_tile_option()));
+      MS_TRY(launch_separable(a, (int)rows, separable_tile_option()));
     else
-      MS_TRY(launch_potential(a, kind, stream_,
-                              kind == POT_CONVENTIONAL ? std::min(std::max(pot_tile_, 0), potential_tiles() - 1) : 0));
+      MS_TRY(launch_potential(a, kind, stream_, kind == POT_CONVENTIONAL ? sub_plane_tile() : 0));
     launches += sep ? 2 : 1;
     last_pot_sum_ = kind == POT_CONVENTIONAL ? (sep ? 2 : 1) : last_pot_sum_;
     return MS_OK;
@@ -3057,6 +3123,7 @@ class Engine {
   int separable_tile_option() const {
     return pot_tile_forced_ ? std::min(pot_tile_, potential_tiles_separable() - 1) : -1;
   }
+  int sub_plane_tile() const { return std::min(std::max(pot_tile_, 0), potential_tiles() - 1); }
   // Tile shape of the per-sub-plane potential kernel for this grid, tuned on
   // the device the first time it is needed: each shape builds the mid-slab
   // slice (one warm-up launch, then three timed) and the fastest is kept.
