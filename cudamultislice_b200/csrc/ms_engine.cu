@@ -586,17 +586,8 @@ class Engine {
     raster_batch_.clear();
     loop_grid_ = 0;
     if (!pot_tile_forced_) pot_tile_ = -1;
-    if (fused_ok_) {
-      std::vector<float2> tw(2 * (size_t)std::max(nx, ny));
-      for (int v = 0; v < plan_variants(); ++v) {
-        const int sx = make_twiddles(nx, v, tw.data());
-        MS_TRY(d_twx_[v].resize(std::max(sx, 1)));
-        MS_TRY(copy_sync(d_twx_[v].p, tw.data(), sizeof(float2) * sx, cudaMemcpyHostToDevice));
-        const int sy = make_twiddles(ny, v, tw.data());
-        MS_TRY(d_twy_[v].resize(std::max(sy, 1)));
-        MS_TRY(copy_sync(d_twy_[v].p, tw.data(), sizeof(float2) * sy, cudaMemcpyHostToDevice));
-      }
-    }
+    if (fused_ok_ || gen_ok_)
+      if (int rc = upload_twiddles()) return rc;
     prop_dz_ = -1.0f;
     have_freq_ = true;
     have_waves_ = false;
@@ -2182,11 +2173,13 @@ class Engine {
     const int v = forced_plan_ >= 0 ? forced_plan_ : 0;
     DevBuf<float2> buf, tw1, tw2;
     MS_TRY(buf.resize(N));
-    std::vector<float2> tw(2 * (size_t)std::max(nx, ny));
-    const int sx = make_twiddles(nx, v, tw.data());
+    std::vector<float2> roots(std::max(nx, ny)), tw(2 * roots.size());
+    unit_roots(nx, roots.data());
+    const int sx = make_twiddles(nx, v, roots.data(), tw.data());
     MS_TRY(tw1.resize(std::max(sx, 1)));
     MS_TRY(copy_sync(tw1.p, tw.data(), sizeof(float2) * sx, cudaMemcpyHostToDevice));
-    const int sy = make_twiddles(ny, v, tw.data());
+    unit_roots(ny, roots.data());
+    const int sy = make_twiddles(ny, v, roots.data(), tw.data());
     MS_TRY(tw2.resize(std::max(sy, 1)));
     MS_TRY(copy_sync(tw2.p, tw.data(), sizeof(float2) * sy, cudaMemcpyHostToDevice));
     MS_TRY(copy_sync(buf.p, in, sizeof(float2) * N, cudaMemcpyHostToDevice));
@@ -2703,7 +2696,7 @@ class Engine {
     return MS_OK;
   }
 
-  // Plans, twiddles and band of the mixed-radix passes, for grids that the
+  // Plans and band of the mixed-radix passes, for grids that the
   // fused passes do not take and whose lengths they provide (general_plan).
   int prepare_general() {
     gen_ok_ = false;
@@ -2725,14 +2718,42 @@ class Engine {
     runs(hkx_, &gen_cpos_, &gen_cneg_);
     runs(hky_, &gen_rpos_, &gen_rneg_);
     if (gen_cpos_ < 1 || gen_rpos_ < 1) return MS_OK;  // (nothing inside the band)
-    std::vector<float2> tw((size_t)std::max(nx_, ny_));
-    general_twiddles(nx_, tw.data());
-    MS_TRY(d_twx_[0].resize(nx_));
-    MS_TRY(copy_sync(d_twx_[0].p, tw.data(), sizeof(float2) * nx_, cudaMemcpyHostToDevice));
-    general_twiddles(ny_, tw.data());
-    MS_TRY(d_twy_[0].resize(ny_));
-    MS_TRY(copy_sync(d_twy_[0].p, tw.data(), sizeof(float2) * ny_, cudaMemcpyHostToDevice));
     gen_ok_ = true;
+    return MS_OK;
+  }
+  // Twiddle tables of both axes in one copy: per plan of the fused passes, or
+  // the roots themselves for the mixed-radix ones.  Every table of a length is
+  // filled from that length's roots, each formed once.
+  int upload_twiddles() {
+    std::vector<float2> rx(nx_), ry, tw;
+    unit_roots(nx_, rx.data());
+    if (ny_ != nx_) {
+      ry.resize(ny_);
+      unit_roots(ny_, ry.data());
+    }
+    size_t at[2][kPlanTables] = {};
+    for (int axis = 0; axis < 2; ++axis) {
+      const int n = axis ? ny_ : nx_;
+      const std::vector<float2>& r = n == nx_ ? rx : ry;
+      for (int v = 0; v < kPlanTables; ++v) {
+        if (axis == 1 && n == nx_) {
+          at[1][v] = at[0][v];
+          continue;
+        }
+        if (gen_ok_ && v > 0) continue;
+        at[axis][v] = (tw.size() + 31) / 32 * 32;
+        tw.resize(at[axis][v] + 2 * (size_t)n);
+        float2* t = tw.data() + at[axis][v];
+        if (gen_ok_) std::copy(r.begin(), r.end(), t);
+        tw.resize(at[axis][v] + (gen_ok_ ? n : make_twiddles(n, v, r.data(), t)));
+      }
+    }
+    MS_TRY(d_tw_.resize(tw.size()));
+    MS_TRY(copy_sync(d_tw_.p, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
+    for (int v = 0; v < plan_variants(); ++v) {
+      twx_[v] = d_tw_.p + at[0][v % kPlanTables];
+      twy_[v] = d_tw_.p + at[1][v % kPlanTables];
+    }
     return MS_OK;
   }
   // Conventional slices on the mixed-radix passes (the plain path when forced).
@@ -2748,7 +2769,7 @@ class Engine {
     g.cneg = gen_cneg_;
     g.rpos = gen_rpos_;
     g.rneg = gen_rneg_;
-    g.tw = rows ? d_twx_[0].p : d_twy_[0].p;
+    g.tw = rows ? twx_[0] : twy_[0];
     g.px = d_px_.p;
     g.py = d_py_.p;
     g.kx = d_kx_.p;
@@ -2826,13 +2847,13 @@ class Engine {
 
   PassAArgs passa_args(const float2* in, float2* out, int variant) {
     PassAArgs a{};
-    a.in = in; a.out = out; a.tw = d_twx_[variant].p; a.nx = nx_; a.ny = ny_;
+    a.in = in; a.out = out; a.tw = twx_[variant]; a.nx = nx_; a.ny = ny_;
     a.sigma = sigma2_; a.scale = 1.0f;
     return a;
   }
   PassBArgs passb_args(const float2* in, float2* out, int variant) {
     PassBArgs b{};
-    b.in = in; b.out = out; b.tw = d_twy_[variant].p; b.px = d_px_.p; b.py = d_py_.p;
+    b.in = in; b.out = out; b.tw = twy_[variant]; b.px = d_px_.p; b.py = d_py_.p;
     b.kx = d_kx_.p; b.ky = d_ky_.p; b.kmax = kmax_; b.nx = nx_; b.ny = ny_; b.scale = 1.0f;
     band_limit_thresholds(kmax_, &b.k2_lt, &b.k2_le);
     b.err = d_pass_err_.p;  // (long propagation columns: tensor-copy staging, see check_pass_err)
@@ -2852,12 +2873,12 @@ class Engine {
   // Row / column pass launchers with the plan for `batch` instances.
   cudaError_t pass_a(PassAArgs a, int flags, int batch = 1, cudaStream_t s = nullptr) {
     const int v = plan_for(batch).row;
-    a.tw = d_twx_[v].p;
+    a.tw = twx_[v];
     return launch_pass_a(a, v, flags, batch, s ? s : stream_);
   }
   cudaError_t pass_b(PassBArgs b, int mode, int batch = 1, cudaStream_t s = nullptr) {
     const int v = plan_for(batch).col;
-    b.tw = d_twy_[v].p;
+    b.tw = twy_[v];
     return launch_pass_b(b, v, mode, batch, s ? s : stream_);
   }
 
@@ -3314,7 +3335,8 @@ class Engine {
   int gen_cpos_ = 0, gen_cneg_ = 0, gen_rpos_ = 0, gen_rneg_ = 0;
   std::vector<float> hkx_, hky_;
   DevBuf<float> d_kx_, d_ky_;
-  DevBuf<float2> d_twx_[6], d_twy_[6], d_px_, d_py_, d_P_;
+  DevBuf<float2> d_tw_, d_px_, d_py_, d_P_;
+  const float2 *twx_[6] = {}, *twy_[6] = {};  // tables by plan variant, in d_tw_
   int forced_plan_ = -1, ckpt_ = 0;
   float last_device_ms_ = 0.0f;
   // detector model of the noisy image chain

@@ -381,14 +381,6 @@ GenPlan general_plan(int n) {
   return p;
 }
 
-void general_twiddles(int n, float2* out) {
-  const long double twopi = 6.283185307179586476925286766559L;
-  for (int m = 0; m < n; ++m) {
-    const long double a = twopi * (long double)m / (long double)n;
-    out[m] = unit_fp32((double)std::cos(a), (double)(-std::sin(a)));
-  }
-}
-
 cudaError_t launch_general_rows(const GenArgs& a, int flags, cudaStream_t s) {
   if (a.plan.n != a.nx || a.plan.npass < 1 || a.ny < 1) return cudaErrorInvalidValue;
   if (flags != G_INV && flags != (G_MULT | G_FWD) && flags != (G_INV | G_MULT | G_FWD)) return cudaErrorInvalidValue;

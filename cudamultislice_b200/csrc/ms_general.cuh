@@ -23,8 +23,6 @@ struct GenPlan {
   float inv[kGenMaxPass] = {};
 };
 GenPlan general_plan(int n);
-// exp(-2 pi i m / n), m < n, as the FP32 pairs nearest unit modulus.
-void general_twiddles(int n, float2* host_out);
 
 struct GenArgs {
   const float2* in;   // wave read (may alias out)
@@ -35,7 +33,7 @@ struct GenArgs {
   // the band: columns [0, cpos) and [nx - cneg, nx), rows of the column
   // spectrum [0, rpos) and [ny - rneg, ny)
   int cpos, cneg, rpos, rneg;
-  const float2* tw;            // twiddles of this pass's length
+  const float2* tw;            // roots of this pass's length (unit_roots)
   const float2 *px, *py;       // propagator factors (unit modulus)
   const float *kx, *ky;
   float k2_lt;                 // band limit on k^2 (see band_limit_thresholds)

@@ -1,6 +1,7 @@
 // ms_slice.cu -- routing of the fused slice passes by line length and plan
 // variant (kernels in ms_slice_impl.cuh, one translation unit per length).
 #include "ms_slice_impl.cuh"
+#include "ms_unit.h"
 
 namespace ms {
 
@@ -64,26 +65,17 @@ void band_limit_thresholds(float kmax, float* k2_lt, float* k2_le) {
 }
 
 float2 unit_fp32(double c, double s) {
-  const float c0 = (float)c, s0 = (float)s;
-  float bc = c0, bs = s0;
-  double best = INFINITY;
-  const double ang = std::atan2(s, c);
-  for (int dc = -1; dc <= 1; ++dc)
-    for (int ds = -1; ds <= 1; ++ds) {
-      const float cc = dc == 0 ? c0 : std::nextafter(c0, dc > 0 ? INFINITY : -INFINITY);
-      const float ss = ds == 0 ? s0 : std::nextafter(s0, ds > 0 ? INFINITY : -INFINITY);
-      // the modulus first: its error adds up over all transforms of a run, the
-      // angle's partly cancels between a transform and its inverse
-      const double n = (double)cc * cc + (double)ss * ss - 1.0;
-      const double a = std::remainder(std::atan2((double)ss, (double)cc) - ang, 6.283185307179586);
-      const double cost = std::hypot(n, 0.2 * a);
-      if (cost < best) {
-        best = cost;
-        bc = cc;
-        bs = ss;
-      }
-    }
-  return make_float2(bc, bs);
+  float2 u;
+  unit_fp32(c, s, &u.x, &u.y);
+  return u;
+}
+
+void unit_roots(int n, float2* out) {
+  const long double twopi = 6.283185307179586476925286766559L;
+  for (int m = 0; m < n; ++m) {
+    const long double a = twopi * (long double)m / (long double)n;
+    out[m] = unit_fp32((double)std::cos(a), (double)(-std::sin(a)));
+  }
 }
 
 int plan_variants() { return kPlanVariants; }
@@ -122,10 +114,10 @@ int pass_plan(int n, long long lines, bool columns, bool tc) {
   return columns ? kCol[i][b] : tc ? kRowTc[i][b] : kRow[i][b];
 }
 
-int make_twiddles(int n, int variant, float2* host_out) {
+int make_twiddles(int n, int variant, const float2* roots, float2* host_out) {
   int size = 0;
   by_length(n, [&](auto c) {
-    size = twiddles_n<decltype(c)::value>(variant, host_out);
+    size = twiddles_n<decltype(c)::value>(variant, roots, host_out);
     return cudaSuccess;
   });
   return size;

@@ -125,16 +125,10 @@ struct PassBArgs {
 // with them takes exactly the decisions of the rounded square root.
 void band_limit_thresholds(float kmax, float* k2_lt, float* k2_le);
 
-// (cos, sin) as the FP32 pair within one ulp of each component with the least
-// hypot(|modulus^2 - 1|, angle error / 5).  Unit factors applied once per transform
-// or per slice (twiddles, propagator) then scale the wave by |(c, s)|^S over a
-// stack of S slices only to that pair's remaining modulus error, far below the
-// plain rounding's, which adds up coherently when the slices repeat (crystals).  The
-// modulus alone would let the angle be off by more than an ulp: 52 slices of a
-// 512^2 crystal then end 0.94e-6 to 1.11e-6 from FP64, with the fifth of the angle
-// 0.84e-6 to 0.98e-6, and a focal-series loss 0.94e-6 (rms of 32 inputs) against
-// 0.42e-6; a tenth or a half of the angle 0.69e-6 and 1.0e-6.
+// (cos, sin) as the FP32 pair of ms_unit.h, and exp(-2 pi i m / n), m < n, as
+// such pairs.
 float2 unit_fp32(double c, double s);
+void unit_roots(int n, float2* host_out);
 
 // Line lengths 64..4096 (powers of two) in both directions.
 bool fused_supported(int nx, int ny);
@@ -145,8 +139,10 @@ bool fused_supported(int nx, int ny);
 int plan_variants();
 int pass_plan(int n, long long lines, bool columns, bool tc);
 // Twiddle table of plan `variant` for lines of n points into host_out
-// (at most 2n entries); returns its length.
-int make_twiddles(int n, int variant, float2* host_out);
+// (at most 2n entries) from the n-th roots (unit_roots); returns its length.
+// The packed variants' tables are those of their unpacked twins.
+constexpr int kPlanTables = 3;
+int make_twiddles(int n, int variant, const float2* roots, float2* host_out);
 cudaError_t launch_pass_a(const PassAArgs& a, int variant, int flags, int batch, cudaStream_t s);
 cudaError_t launch_pass_b(const PassBArgs& a, int variant, int mode, int batch, cudaStream_t s);
 

@@ -858,20 +858,20 @@ cudaError_t dispatch_b_plan(const PassBArgs& a, int mode, int batch, cudaStream_
 }
 
 template <class PL>
-void fill_twiddles(float2* out) {
-  const long double twopi = 6.283185307179586476925286766559L;
+void fill_twiddles(const float2* roots, float2* out) {
   const int R[4] = {PL::R1, PL::R2, PL::R3, PL::R4};
   int ns = R[0], off = 0;
   for (int p = 1; p < PL::NPASS; ++p) {
     const int m = ns * R[p];
     for (int r = 0; r < R[p]; ++r)
-      for (int k = 0; k < ns; ++k) {
-        const long double ang = twopi * (long double)(((long long)r * k) % m) / (long double)m;
-        out[off + r * ns + k] = unit_fp32((double)std::cos(ang), (double)(-std::sin(ang)));
-      }
+      for (int k = 0; k < ns; ++k) out[off + r * ns + k] = roots[r * k % m * (PL::N / m)];
     off += m;
     ns = m;
   }
+}
+template <class A, class B>
+constexpr bool same_radices() {
+  return A::R1 == B::R1 && A::R2 == B::R2 && A::R3 == B::R3 && A::R4 == B::R4;
 }
 
 // Entry points of one line length (defined in ms_slice_n<N>.cu).
@@ -880,7 +880,7 @@ cudaError_t dispatch_a_n(const PassAArgs& a, int variant, int flags, int batch, 
 template <int N>
 cudaError_t dispatch_b_n(const PassBArgs& a, int variant, int mode, int batch, cudaStream_t s);
 template <int N>
-int twiddles_n(int variant, float2* out);
+int twiddles_n(int variant, const float2* roots, float2* out);
 
 #define MS_SLICE_INSTANTIATE(N)                                                                      \
   template <>                                                                                        \
@@ -908,14 +908,15 @@ int twiddles_n(int variant, float2* out);
     }                                                                                                \
   }                                                                                                  \
   template <>                                                                                        \
-  int twiddles_n<N>(int variant, float2* out) {                                                      \
-    switch (variant) {                                                                               \
-      case 0: fill_twiddles<PlanSel<N, 0>::T>(out); return PlanSel<N, 0>::T::TWSIZE;                 \
-      case 1: fill_twiddles<PlanSel<N, 1>::T>(out); return PlanSel<N, 1>::T::TWSIZE;                 \
-      case 2: fill_twiddles<PlanSel<N, 2>::T>(out); return PlanSel<N, 2>::T::TWSIZE;                 \
-      case 3: fill_twiddles<PlanSel<N, 3>::T>(out); return PlanSel<N, 3>::T::TWSIZE;                 \
-      case 4: fill_twiddles<PlanSel<N, 4>::T>(out); return PlanSel<N, 4>::T::TWSIZE;                 \
-      case 5: fill_twiddles<PlanSel<N, 5>::T>(out); return PlanSel<N, 5>::T::TWSIZE;                 \
+  int twiddles_n<N>(int variant, const float2* roots, float2* out) {                                 \
+    static_assert(same_radices<PlanSel<N, 0>::T, PlanSel<N, 3>::T>() &&                              \
+                      same_radices<PlanSel<N, 1>::T, PlanSel<N, 4>::T>() &&                          \
+                      same_radices<PlanSel<N, 2>::T, PlanSel<N, 5>::T>(),                            \
+                  "a packed variant shares its twin's table");                                       \
+    switch (variant % kPlanTables) {                                                                 \
+      case 0: fill_twiddles<PlanSel<N, 0>::T>(roots, out); return PlanSel<N, 0>::T::TWSIZE;          \
+      case 1: fill_twiddles<PlanSel<N, 1>::T>(roots, out); return PlanSel<N, 1>::T::TWSIZE;          \
+      case 2: fill_twiddles<PlanSel<N, 2>::T>(roots, out); return PlanSel<N, 2>::T::TWSIZE;          \
       default: return 0;                                                                             \
     }                                                                                                \
   }
