@@ -81,34 +81,40 @@ void unit_roots(int n, float2* out) {
 int plan_variants() { return kPlanVariants; }
 
 // Measured per line length and batch of square grids, us per launch (B200, the
-// passes of the slice loop; 1, 4, 16, 64 instances):
-//                  chosen                    next best
-//   rows  128      5: 2.5 2.4 3.4, 4: 5.6    1: -, -, 3.5, 5.7
-//         256      5: 3.4, 4: 3.3 5.7, 0: 13.1   4: 3.4, 0: 3.4 4.7, 3: 12.1
-//         512      5: 3.4, 0: 5.6 16.7 58.3  2: 3.4, 1: 5.7, 4: 16.8 60.3
-//         1024     0: 5.9 17.5 60.6 246      3: 6.2, 4: 19.0 66.3 258
-//         2048     4: 20.1 71.5 274          1: 20.4 76.0 297
-//         4096     4: 79.7 302               1: 86.8, 0: 325
-//   rows, tc, 512   5: 3.4, 1: 5.6 16.1, 0: 40.3   0: 5.8 12.4, 1: 57.6 (a 512^2
-//                  raster of 16 instances takes the same with either)
-//   rows, tc, 2048 and up  0: 20.7 73.2 270, 1 at 4096: 84.9 324
-//   columns 128    5: 2.5 3.5 2.7 4.4        2
-//         256      5: 2.7 3.5 4.9, 3: 10.0   4: 3.1, 1: 5.2, 0: 10.2
-//         512      5: 3.8, 3: 6.0, 0: 9.8 35.3   2: 3.6, 4: 6.3, 3: 12.1 40.6
-//         1024     3: 7.1, 0: 11.2 38.3 172  1: 8.0, 3: 15.6 53.6 230
-//         2048     3: 18.7, 0: 53.7 231      1: 20.0 58.9 251
-//         4096     3: 60.5, 0: 254           0: 67.9, 3: 304
+// passes of the slice loop, 300 launches back to back; 4, 12, 16, 32 and 64
+// instances of up to 512 points, 4, 16 and 64 of 1024, 4 and 8 or 16 above):
+//                  chosen                            the next
+//   rows  128      5: 2.2 2.4 3.3 3.4, 0: 4.5        2: 2.2 2.3 3.2 3.4, 5: 5.1
+//         256      5: 3.9, 0: 4.6 4.6, 3: 7.6 11.9   2: 3.9, 5: 5.2, 1: 5.6, 0: 7.6 12.9
+//         512      0: 5.4 13.6 16.5 29.9 58.1        1: 5.6, 5: 13.9, 4: 16.5 31.3 60.4
+//         1024     0: 17.8 61.2 246                  4: 19.3 67.1 258
+//         2048     4: 72.5 141                       1: 77.0 153
+//         4096     4: 302                            0: 326
+//   rows, tc, 128  5: 2.3 2.2 3.3 3.4, 0: 4.1        1: 2.2 3.8 3.9 4.0, 4: 4.9
+//         256      4: 3.0, 0: 4.3 4.3 7.1 11.6       1: 2.9 4.0 4.9 8.0 14.4
+//         512      0: 5.8 9.9 12.2 21.0 40.1         3: 5.3, 1: 13.5 15.8 29.6 57.6
+//         1024     0: 16.7 56.0 221                  3: 18.9 62.5 254
+//         2048     0: 74.1 140                       1: 76.8 149
+//         4096     1: 324                            4: 338
+//   columns 128    5: 2.5 3.6 3.9 4.0 4.4            2: 2.5 3.7 4.0 4.0 4.4
+//         256      5: 4.6 4.8 4.9, 3: 5.3 9.8        3: 4.0, 4: 4.5 5.0, 0: 5.5 10.0
+//         512      3: 6.0, 0: 9.7 9.7 18.7 36.0      5: 6.2, 4: 10.3 12.1 21.2 40.5
+//         1024     0: 11.2 38.4 172                  3: 15.8 54.4 230
+//         2048     0: 54.1 117                       4: 58.5 126
+//         4096     0: 254                            3: 305
+// One instance (at most 512 points: bound by the launches, chosen by whole slices):
+// 1024 rows 0 5.9, columns 3 7.2; 2048 4 20.5, 3 18.6; 4096 4 79.7, 3 60.6.
 // Timing them on each handle's first use instead took 2-5 ms, and at one
 // instance, where a launch takes as long as the kernel, picked at random.
 int pass_plan(int n, long long lines, bool columns, bool tc) {
   const long long eff = lines / n;  // instances of a square grid
-  const int b = eff < 2 ? 0 : eff < 8 ? 1 : eff < 32 ? 2 : 3;
-  static const signed char kRow[7][4] = {{5, 5, 5, 5}, {5, 5, 5, 4}, {5, 4, 4, 0}, {5, 0, 0, 0},
-                                         {0, 0, 0, 0}, {4, 4, 4, 4}, {4, 4, 4, 4}};
-  static const signed char kRowTc[7][4] = {{5, 5, 5, 5}, {5, 5, 1, 0}, {5, 4, 0, 0}, {5, 1, 1, 0},
-                                           {0, 0, 0, 0}, {0, 0, 0, 0}, {1, 1, 1, 1}};
-  static const signed char kCol[7][4] = {{5, 5, 5, 5}, {5, 5, 5, 5}, {5, 5, 5, 3}, {5, 3, 0, 0},
-                                         {3, 0, 0, 0}, {3, 0, 0, 0}, {3, 0, 0, 0}};
+  const int b = eff < 2 ? 0 : eff < 8 ? 1 : eff < 20 ? 2 : eff < 48 ? 3 : 4;
+  static const signed char kRow[7][5] = {{5, 5, 5, 5, 5}, {5, 5, 5, 5, 0}, {5, 5, 0, 3, 3}, {5, 0, 0, 0, 0},
+                                         {0, 0, 0, 0, 0}, {4, 4, 4, 4, 4}, {4, 4, 4, 4, 4}};
+  static const signed char kRowTc[7][5] = {{5, 5, 5, 5, 5}, {5, 5, 5, 5, 0}, {5, 4, 0, 0, 0}, {5, 0, 0, 0, 0},
+                                           {0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}, {1, 1, 1, 1, 1}};
+  static const signed char kCol[7][5] = {{5, 5, 5, 5, 5}, {5, 5, 5, 5, 5}, {5, 5, 5, 3, 3}, {5, 3, 0, 0, 0},
+                                         {3, 0, 0, 0, 0}, {3, 0, 0, 0, 0}, {3, 0, 0, 0, 0}};
   int i = 0;
   while ((64 << i) < n && i < 6) ++i;
   return columns ? kCol[i][b] : tc ? kRowTc[i][b] : kRow[i][b];
