@@ -2205,8 +2205,9 @@ class Engine {
   //   dL/dV_n = -2 sigma Im(conj(h) t_n psi_{n-1}),  g_{n-1} = conj(t_n) h,
   // and through the potential build to the atoms' x, y.  The waves psi_{n-1}
   // are recomputed segment by segment from checkpoints every K slices
-  // (K = ceil(sqrt(S)) unless MS_OPT_CHECKPOINT sets it; K >= S keeps one
-  // segment, K = 1 stores every wave in the forward sweep).
+  // (auto_checkpoint_stride unless MS_OPT_CHECKPOINT sets K); the last segment's
+  // are kept as the forward sweep passes, so that K = 1 and K >= S, one segment
+  // of all slices, recompute nothing.
   // All waves are held in the fused passes' row-frequency form X with
   // IFFT_row(X) = field; the adjoint state g uses the same form.
   int focal(const float* defoci, int nd, const float* targets, int S, double* loss, float* images, float* dLdV,
@@ -2337,13 +2338,9 @@ class Engine {
           launches += 2;
           cur = d_t1_.p;
         }
-        float2* last = d_seg_.p + (size_t)(e - 1 - c) * N;
-        if (c == clast) {
-          // saved by the forward sweep
-        } else if (e - 1 == 0) {
-          MS_TRY(cudaMemcpyAsync(last, d_psi0_.p, sizeof(float2) * N, cudaMemcpyDeviceToDevice, stream_));
-        } else {
-          MS_TRY(pass_a(passa_args(cur, last, 0), A_INV | A_BI, 1));
+        // (segments before the last hold K >= 2 slices: psi_{e-1} is in `cur`)
+        if (c != clast) {
+          MS_TRY(pass_a(passa_args(cur, d_seg_.p + (size_t)(e - 1 - c) * N, 0), A_INV | A_BI, 1));
           ++launches;
         }
         // adjoint steps e .. c+1

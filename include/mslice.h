@@ -71,8 +71,8 @@ enum {
   MS_OPT_CHECKPOINT = 4,    /* focal-series gradient: slices between stored waves;
                                0 = automatic (default): every wave when the S waves
                                fit in an eighth of the free device memory, else
-                               ceil(sqrt(S)); 1 = store every wave; >= S = one
-                               segment recomputed from the initial wave */
+                               ceil(sqrt(S)); 1 or >= S = every wave, kept by the
+                               forward sweep */
   MS_OPT_SLICE_LOOP = 5,    /* fused conventional slice loop (ms_run_conventional,
                                ms_time_slices) on square 256, 512 and 1024 grids:
                                0 = one persistent cooperative launch for all slices,
