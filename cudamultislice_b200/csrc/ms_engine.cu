@@ -81,6 +81,7 @@ struct DevBuf {
     if (count == 0) return cudaSuccess;
     cudaError_t e = cudaMalloc(&p, count * sizeof(T));
     if (e != cudaSuccess) {
+      cudaGetLastError();  // (reported here; not again by the next launch)
       p = nullptr;
       return e;
     }
@@ -2428,9 +2429,7 @@ class Engine {
   }
   // Room for `rows` rows of atom tables; false where the device has none left.
   bool have_tables(size_t rows) {
-    if (d_tab_.n >= rows * kTabStride || d_tab_.resize(rows * kTabStride) == cudaSuccess) return true;
-    cudaGetLastError();
-    return false;
+    return d_tab_.n >= rows * kTabStride || d_tab_.resize(rows * kTabStride) == cudaSuccess;
   }
   // Without that room potentials and their adjoint are summed per sub-plane,
   // unless the separable sum is forced.
