@@ -3104,10 +3104,19 @@ class Engine {
     gauss_row_ok_[r] = ok ? 1 : 0;
     return ok;
   }
+  // Pixels or atoms so far out that a distance squared can overflow.  There the
+  // separable kernel would multiply the zero polynomial of an atom out of reach by
+  // infinity (a bound on every pixel's argument instead costs 1% of the kernel);
+  // the per-sub-plane kernel leaves such atoms out.
+  bool far_grid() const {
+    const double far = 1e18;
+    return std::fabs((double)xoff_) + (double)nx_ * ps_ > far || std::fabs((double)yoff_) + (double)ny_ * ps_ > far ||
+           (double)box_.MaxX - box_.MinX > far || (double)box_.MaxY - box_.MinY > far;
+  }
   // The separable conventional kernel applies when every element of the
   // specimen has a valid expansion (MS_OPT_POTENTIAL_SUM 0 or 2).
   bool separable_ok() {
-    if (pot_sum_ == 1 || !have_fp_) return false;
+    if (pot_sum_ == 1 || !have_fp_ || far_grid()) return false;
     for (int z = 1; z <= 103; ++z)
       if (z < (int)zpresent_.size() && zpresent_[z] && !gauss_row_ok(z - 1)) return false;
     return true;
@@ -3116,7 +3125,7 @@ class Engine {
   // Potential of one slice into out (ny x nx floats).
   int potential_slice(int kind, int it, float* out) {
     bool sep = kind == POT_CONVENTIONAL && separable_ok();
-    if (kind == POT_CONVENTIONAL && pot_sum_ == 2 && !sep)
+    if (kind == POT_CONVENTIONAL && pot_sum_ == 2 && !sep && !far_grid())
       return fail(MS_ERR_UNSUPPORTED, "an element of the specimen has no valid Gaussian expansion");
     const size_t rows = sep ? window_atoms(hzoff_, nzb_, 1) : 0;
     if (sep && !have_tables(rows)) {

@@ -107,7 +107,8 @@ enum {
                                sum is a function of the distance in the plane alone,
                                expanded once per atom and slice into piecewise polynomials
                                (5e-8 of the sum); the same sub-planes pass the reference's
-                               FP32 cut-off test as term by term. */
+                               FP32 cut-off test as term by term.  Pixels or specimens that
+                               extend past 1e18 A: always term by term. */
   MS_OPT_BUILD_OVERLAP = 11 /* ms_run_conventional when the potential stack must be built:
                                1 = run each slice's fused passes on a second stream while the
                                next slices' potentials are built (default; separable
