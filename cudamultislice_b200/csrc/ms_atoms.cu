@@ -921,13 +921,15 @@ __device__ __noinline__ float clamp_value(const float* __restrict__ tab, const f
 // range map to a zero segment, positions of two pixels share packed FP32x2
 // instructions, and the rare rest (clamp region, bins with many thresholds) is
 // one branch per atom.  Per slice of the 50k-atom carbon slab (0.1 atoms/A^3,
-// 2 A slices) in a stack build, tables included: 1024^2 at 0.049 A 49 -> 27.9 us,
-// 4096^2 at 0.012 A 547 -> 272 us (against the sum over 12 Gaussians at every
+// 2 A slices) in a stack build, tables included: 1024^2 at 0.049 A 49 -> 28.2 us,
+// 4096^2 at 0.012 A 547 -> 273 us (against the sum over 12 Gaussians at every
 // pixel).  CTAs of four warps: eight warps waited longer at the staging
 // barriers (30.2 us); tables staged in shared memory cost occupancy and more
 // L2 traffic (34.8 us).  Every second patch of an atom inside the slice meets
 // the cut-off's rim, up to ten thresholds in a bin: counted four loads at a time
-// (one by one 28.3 us; two at a time for all of a thread's pixels at once 29.3).
+// (one by one 0.4 us more; two at a time for all of a thread's pixels at once 1.4).
+// Of the 28.2 us, 0.35 are the separate rounding of dx^2 + dy^2 (mul2_rn): fused,
+// one pixel in a million decided a sub-plane at the cut-off the other way.
 constexpr int kSepChunk = 128;  // candidates staged at a time
 
 constexpr int kSepThreads = 128;
@@ -950,6 +952,7 @@ __global__ void __launch_bounds__(kSepThreads, sep_ctas<RY>()) k_potential_sep(c
   __shared__ int s_warp[33];
 
   constexpr int PX = TX / 8, RP = RY / 2;  // patches across, pixel pairs per thread
+  const f2p zero = pk2(q.zero, q.zero);
   // this slice's window, this instance's index, tables and output
   const PotArgs& a = q.p;
   const int sl = blockIdx.z / q.nb, inst = blockIdx.z - sl * q.nb;
@@ -1102,7 +1105,7 @@ __global__ void __launch_bounds__(kSepThreads, sep_ctas<RY>()) k_potential_sep(c
 #pragma unroll
             for (int h = 0; h < RP; ++h) {
               const f2p dy = add2(py[h], nay);
-              const f2p d2 = add2(dx2p, mul2(dy, dy));
+              const f2p d2 = add2(dx2p, mul2_rn(dy, dy, zero));  // (as the cut-off rounds it)
               const f2p s2 = add2(d2, h0);
               const f2p dyv = add2(dy, py_lo[h]);
               const f2p sv = fma2(dyv, dyv, xvp);
@@ -1469,8 +1472,8 @@ static cudaError_t run_potential_sep(const SepArgs& a, cudaStream_t s) {
 
 // Tile of a launch: four pixels per thread (a warp's per-atom work shared by
 // four rows), eight for pixels of at most 0.02 A (a patch of 0.16 x 0.32 A is
-// still small against the atoms' reach: 4096^2 at 0.012 A 276 us against 290;
-// at 0.049 A 30.6 against 28.5), two where four would leave SMs without a CTA
+// still small against the atoms' reach: 4096^2 at 0.012 A 273 us against 292;
+// at 0.049 A 30.2 against 28.2), two where four would leave SMs without a CTA
 // (64^2, two slices: 7.6 us a slice against 8.0).
 static int separable_tile(const SepArgs& a) {
   const long long ctas = (long long)((a.p.nx + 31) / 32) * ((a.p.ny + 15) / 16) * a.nb * a.ns;

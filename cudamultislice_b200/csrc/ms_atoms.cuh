@@ -117,6 +117,7 @@ struct SepArgs {
   PotArgs p;
   int ns, nb;
   int rows;  // atoms of the fullest window (bounds the table launch)
+  float zero;  // 0, unknown to the compiler (mul2_rn)
   long long s_tab, s_V;
   SlicePlanes pl[kSepGroup];
   void set_slice(int i, const PotArgs& a) {

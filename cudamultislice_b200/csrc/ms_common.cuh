@@ -85,6 +85,14 @@ MS_D f2p fma2(f2p a, f2p b, f2p c) {
   return d;
 }
 
+// a b rounded by itself, to be added with add2 where the sum's rounding decides.
+// The assembler contracts a mul2 that feeds an add2 into one FMA, whatever their
+// rounding qualifiers say (of a million sums dx^2 + dy^2 so written 16% differed
+// from the separate operations, all of them equal to the FMA; scalar __fmul_rn and
+// __fadd_rn are kept apart).  An FMA with a zero that it cannot see (z: a kernel
+// argument) rounds as the product and is not contracted further.
+MS_D f2p mul2_rn(f2p a, f2p b, f2p z) { return fma2(a, b, z); }
+
 // sin and cos of two values at once: sincos_red with its polynomial and
 // reduction steps on the packed FP32x2 pipe.  Each lane rounds exactly as the
 // scalar fmaf/multiply of sincos_red does, so the results are bit-identical.
