@@ -567,7 +567,7 @@ def potential_leg(fparams, device: int, reps: int = 3) -> dict:
     """The workload's potential stack (102 slices, 1024^2, 50k atoms) built by
     the separable kernel (the default) and by the per-sub-plane kernel: device
     time of ms_build_potential_stack, best of `reps` rebuilds after a first
-    build that tunes each kernel's tile shape."""
+    build (in which the per-sub-plane kernel's tile is tuned)."""
     atoms = workload()
     out = {}
     for mode, name in ((2, "separable"), (1, "per_subplane")):

@@ -272,7 +272,7 @@ class Engine {
         return MS_OK;
       case MS_OPT_POTENTIAL_TILE:
         if (value < -1 || value >= std::max(potential_tiles(), potential_tiles_separable()))
-          return fail(MS_ERR_INVALID, "tile must be -1 (tuned) or a tile index of the potential kernels");
+          return fail(MS_ERR_INVALID, "tile must be -1 (default) or a tile index of the potential kernels");
         pot_tile_ = value;
         pot_tile_forced_ = value >= 0;
         stack_valid_ = false;
@@ -1494,7 +1494,7 @@ class Engine {
       if (B > cap) break;
       rs_prefer_loop_ = lp == 1;  // slices in the batched persistent loop, or per pass
       std::vector<int> qx(B, px0), qy(B, py0);
-      for (int rep = 0; rep < 2; ++rep) {  // the first run tunes the plans and loads the kernels
+      for (int rep = 0; rep < 2; ++rep) {  // (the first run loads the kernels and allocates)
         if (int rc = raster_prepare(qx.data(), qy.data(), B, inner, outer, B)) return rc;
         MS_TRY(cudaEventRecord(ev0_, stream_));
         if (int rc = raster_enqueue(stream_, true)) return rc;
@@ -2778,9 +2778,9 @@ class Engine {
     g.plan = rows ? gen_row_ : gen_col_;
     return g;
   }
-  // One slice: rows (from the initial wave, from real space, or continuing
-  // from the last slice's band: `chain`), then columns, leaving the band in
-  // d_t1_; finish_general returns it to real space in d_psi_.
+  // One slice: rows (from `real_in`, the initial wave or another in real space;
+  // null: from the last slice's band), then columns, leaving the band in d_t1_;
+  // finish_general returns it to real space in d_psi_.
   int enqueue_general_step(const float* V, const float2* real_in, cudaStream_t s) {
     GenArgs r = gen_args(real_in ? real_in : d_t1_.p, d_t1_.p, true);
     r.V = V;
@@ -3351,7 +3351,7 @@ class Engine {
   uint64_t det_seed_ = 0;
   uint32_t det_serial_ = 0;
   bool image_noisy_ = false;
-  int pot_tile_ = -1;                    // tuned tile shape of the conventional potential (-1: not yet)
+  int pot_tile_ = -1;                    // conventional potential's tile: forced, or per sub-plane tuned (-1: neither)
   bool pot_tile_forced_ = false;
   int rs_n_ = 0, rs_B_ = 1, rs_S_ = 0;  // prepared probe raster
   bool rs_loop_ = false;                 // its slices ran in the batched persistent loop
